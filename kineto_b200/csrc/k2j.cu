@@ -151,20 +151,43 @@ uint32_t pow2_at_least(uint64_t n) {
   return p;
 }
 
-struct Scan {
-  static uint32_t blocks(uint64_t n) { return (uint32_t)((n + kScanTile - 1) / kScanTile); }
-};
-
 // Exclusive scan of `cols` columns of n u32 each (column stride n) into u64; totals land in
-// totals[0..cols).  Three launches.
-k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches) {
-  const uint32_t nb = std::max<uint32_t>(1, Scan::blocks(n));
+// totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length: up to
+// kScanSmallMax elements one block per column is done sooner than a second launch would begin; up to
+// kScanDirectBlocks tiles adding up the sums in front of a block costs it less than the launch that scans them.
+constexpr uint64_t kScanSmallMax = 2 * kScanSmallTile;
+constexpr uint32_t kScanDirectBlocks = 4096;
+k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches,
+                    const ScanReport& rep = ScanReport{}) {
+  if (n <= kScanSmallMax) {
+    k_scan_small<<<cols, kScanSmallThreads, 0, c->stream>>>(in, n, totals, out, rep);
+    *launches += 1;
+    K2J_CUDA(c, cudaGetLastError());
+    return K2J_OK;
+  }
+  const uint32_t nb = (uint32_t)((n + kScanTile - 1) / kScanTile);
   K2J_CUDA(c, c->scan_sums.reserve((size_t)nb * cols * 8));
   uint64_t* sums = c->scan_sums.as<uint64_t>();
   k_scan_reduce<<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb);
-  k_scan_sums<<<cols, kScanThreads, 0, c->stream>>>(sums, nb, totals);
-  k_scan_apply<<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb, out);
-  *launches += 3;
+  if (nb <= kScanDirectBlocks) k_scan_apply<true><<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb, out, totals, rep);
+  else {
+    k_scan_sums<<<cols, kScanThreads, 0, c->stream>>>(sums, nb, totals);
+    k_scan_apply<false><<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb, out, nullptr, rep);
+    *launches += 1;
+  }
+  *launches += 2;
+  K2J_CUDA(c, cudaGetLastError());
+  return K2J_OK;
+}
+
+// One launch that gives every region of the list its initial value.
+k2j_status run_clear(k2j_ctx* c, const ClearList& l) {
+  uint64_t words = 0;
+  for (uint32_t k = 0; k < l.n; k++) words = std::max(words, l.r[k].words);
+  if (words == 0) return K2J_OK;
+  const uint64_t blocks = (words / 2 + kClearThreads) / kClearThreads;
+  k_clear<<<(uint32_t)std::min<uint64_t>(blocks, 148 * 8), kClearThreads, 0, c->stream>>>(l);
+  c->launches++;
   K2J_CUDA(c, cudaGetLastError());
   return K2J_OK;
 }
@@ -305,9 +328,8 @@ k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint3
       d, c->span_out.as<SpanRec>(), n, c->ann_size.as<uint32_t>(), nullptr, 0);
   c->launches++;
   K2J_CUDA(c, cudaGetLastError());
-  k2j_status st = run_scan(c, c->ann_size.as<uint32_t>(), n, 1, c->ann_off.as<uint64_t>(), c->scan_totals.as<uint64_t>() + 22, &c->launches);
+  k2j_status st = run_scan(c, c->ann_size.as<uint32_t>(), n, 1, c->ann_off.as<uint64_t>(), c->h_totals + 22, &c->launches);
   if (st) return st;
-  K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 22, c->scan_totals.as<uint64_t>() + 22, 8, cudaMemcpyDeviceToHost, s));
   K2J_CUDA(c, cudaStreamSynchronize(s));  // also covers `ordered`, which goes out of scope
   *bytes_out = c->h_totals[22];
   return K2J_OK;
@@ -552,7 +574,6 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
   d.guest_front = (uint32_t)(c->guest_front_bytes / 8);
   d.guest_back = c->guest_back_bytes == ~0ull ? 0xFFFFFFFFu : (uint32_t)(c->guest_back_bytes / 8);
 
-  K2J_CUDA(c, cudaMemsetAsync(c->counters.p, 0, sizeof(Counters), s));
   K2J_CUDA(c, cudaEventRecord(c->ev[0], s));
 
   // ---- string pool: sanitised copies (once per pool) ----
@@ -582,9 +603,8 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     k_seg_compose<<<c->n_buf, 256, 0, s>>>(d);
     c->launches += 2;
     K2J_CUDA(c, cudaGetLastError());
-    k2j_status st = run_scan(c, d.chunk_cnt, nch, C_NCOL, d.chunk_base, c->scan_totals.as<uint64_t>(), &c->launches);
+    k2j_status st = run_scan(c, d.chunk_cnt, nch, C_NCOL, d.chunk_base, c->h_totals, &c->launches);
     if (st) return st;
-    K2J_CUDA(c, cudaMemcpyAsync(c->h_totals, c->scan_totals.p, C_NCOL * 8, cudaMemcpyDeviceToHost, s));
     K2J_CUDA(c, cudaStreamSynchronize(s));
     for (int i = 0; i < C_NCOL; i++) totals[i] = c->h_totals[i];
   }
@@ -935,7 +955,12 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   K2J_CUDA(c, cudaEventRecord(c->ev[6], s));
   // every counter belongs to the emit step (segmentation counts through its scan columns): a second k2j_emit after
   // one k2j_segment starts from zero, and an earlier failed check does not fail this run
-  K2J_CUDA(c, cudaMemsetAsync(d.counters, 0, sizeof(Counters), s));
+  ClearList clear;
+  auto clear_later = [&](void* p, uint64_t bytes, bool ones = false) {  // whole 8-byte words
+    clear.ones |= (ones ? 1u : 0u) << clear.n;
+    clear.r[clear.n].p = static_cast<uint64_t*>(p); clear.r[clear.n].words = bytes / 8; clear.n++;
+  };
+  clear_later(d.counters, sizeof(Counters));
 
   // ---- join tables ----
   uint64_t own_begin = 0, own_end = totals[C_EXT];
@@ -970,22 +995,21 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   d.corr_tab = c->corr_tab.as<unsigned long long>(); d.corr_mask = corr_cap - 1;
   d.user_tab = c->user_tab.as<unsigned long long>(); d.user_mask = corr_cap - 1;
   d.op_tab = c->op_tab.as<unsigned long long>(); d.op_mask = op_cap - 1;
-  K2J_CUDA(c, cudaMemsetAsync(d.corr_tab, 0, (size_t)corr_cap * 8, s));
+  clear_later(d.corr_tab, (size_t)corr_cap * 8);
   K2J_CUDA(c, c->corr0.reserve(16));
   d.corr0 = c->corr0.as<unsigned long long>();
-  K2J_CUDA(c, cudaMemsetAsync(d.corr0, 0, 16, s));
+  clear_later(d.corr0, 16);
   // the user-annotation table is only written and read when CUSTOM1 correlation records exist
   // (several shards: another shard's CUSTOM1 records may name this shard's events, so the local count says nothing,
   // unless the caller has said that no shard holds any)
   const bool user_records = c->have_global_join ? c->join_user_hint != 0 : totals[C_USER] > 0;
-  if (user_records) K2J_CUDA(c, cudaMemsetAsync(d.user_tab, 0, (size_t)corr_cap * 8, s));
+  if (user_records) clear_later(d.user_tab, (size_t)corr_cap * 8);
   else d.user_tab = nullptr;
-  K2J_CUDA(c, cudaMemsetAsync(d.op_tab, 0, (size_t)op_cap * 8, s));
+  clear_later(d.op_tab, (size_t)op_cap * 8);
   const uint32_t tid_cap = std::max<uint32_t>(16384, pow2_at_least(4ull * c->n_tid));
   K2J_CUDA(c, c->tid_tab.reserve((size_t)tid_cap * 8));
   d.tid_tab = c->tid_tab.as<unsigned long long>(); d.tid_mask = tid_cap - 1;
-  K2J_CUDA(c, cudaMemsetAsync(d.tid_tab, 0, (size_t)tid_cap * 8, s));
-  if (c->n_tid + c->n_ops) { k_build_tids<<<(uint32_t)((c->n_tid + c->n_ops + 255) / 256), 256, 0, s>>>(d); c->launches++; }
+  clear_later(d.tid_tab, (size_t)tid_cap * 8);
   // user-annotation span tables (single-shard runs only)
   const bool spans_on = (c->params.flags & K2J_FLAG_USER_ANNOTATIONS) && user_records;
   d.span_key = nullptr;
@@ -1003,26 +1027,27 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     d.span_key = c->span_key.as<unsigned long long>(); d.span_nstart = c->span_nstart.as<unsigned long long>();
     d.span_end = c->span_end.as<unsigned long long>(); d.span_nfirst = c->span_nfirst.as<unsigned long long>();
     d.span_row = c->span_row.as<uint32_t>(); d.span_mask = span_cap - 1;
-    K2J_CUDA(c, cudaMemsetAsync(d.ds_tab, 0, (size_t)ds_cap * 8, s));
-    K2J_CUDA(c, cudaMemsetAsync(d.span_key, 0, (size_t)span_cap * 8, s));
-    K2J_CUDA(c, cudaMemsetAsync(d.span_nstart, 0, (size_t)span_cap * 8, s));
-    K2J_CUDA(c, cudaMemsetAsync(d.span_end, 0, (size_t)span_cap * 8, s));
-    K2J_CUDA(c, cudaMemsetAsync(d.span_nfirst, 0, (size_t)span_cap * 8, s));
+    clear_later(d.ds_tab, (size_t)ds_cap * 8);
+    clear_later(d.span_key, (size_t)span_cap * 8);
+    clear_later(d.span_nstart, (size_t)span_cap * 8);
+    clear_later(d.span_end, (size_t)span_cap * 8);
+    clear_later(d.span_nfirst, (size_t)span_cap * 8);
   }
   d.need_corr = nullptr; d.need_op = nullptr;
+  bool mark_corr = false;
   if (filter) {
     const uint32_t corr_bits = std::max<uint32_t>(1u << 20, pow2_at_least(8 * std::max<uint64_t>(1, n_gpu_events)));
     const uint32_t op_bits = corr_bits;
     K2J_CUDA(c, c->need_op.reserve(op_bits / 8));
     d.need_op = c->need_op.as<uint32_t>(); d.need_op_mask = op_bits - 1;
-    K2J_CUDA(c, cudaMemsetAsync(d.need_op, 0, op_bits / 8, s));
+    clear_later(d.need_op, op_bits / 8);
     if (c->need_bits) {  // the filter the caller had filled for the exchange (k2j_join_need_bits): the same marks
       d.need_corr = c->need_bits; d.need_corr_mask = (uint32_t)(c->need_n_bits - 1);
     } else {
       K2J_CUDA(c, c->need_corr.reserve(corr_bits / 8));
       d.need_corr = c->need_corr.as<uint32_t>(); d.need_corr_mask = corr_bits - 1;
-      K2J_CUDA(c, cudaMemsetAsync(d.need_corr, 0, corr_bits / 8, s));
-      if (d.ops_begin) { k_mark_corr<<<(uint32_t)((d.ops_begin + 255) / 256), 256, 0, s>>>(d); c->launches++; }
+      clear_later(d.need_corr, corr_bits / 8);
+      mark_corr = d.ops_begin != 0;
     }
   }
   // collective enrichment: kernels look at their linked op's name only if some op is a record_param_comms call;
@@ -1030,9 +1055,7 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   d.has_comms = nullptr;
   if (c->n_ops && c->n_strings) {
     K2J_CUDA(c, c->comms_flag.reserve(16));
-    K2J_CUDA(c, cudaMemsetAsync(c->comms_flag.p, 0, 4, s));
-    k_find_comms<<<(uint32_t)((c->n_ops + 255) / 256), 256, 0, s>>>(d, c->comms_flag.as<uint32_t>(), 1);
-    c->launches++;
+    clear_later(c->comms_flag.p, 8);
     d.has_comms = c->comms_flag.as<uint32_t>();
     if (c->have_global_join) {
       // several shards: the join's table holds positions in the gathered keys, so the record_param_comms ops that carry
@@ -1040,9 +1063,7 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
       const uint32_t coll_cap = pow2_at_least(2 * c->n_ops + 16);
       K2J_CUDA(c, c->coll_tab.reserve((size_t)coll_cap * 8));
       d.coll_tab = c->coll_tab.as<unsigned long long>(); d.coll_mask = coll_cap - 1;
-      K2J_CUDA(c, cudaMemsetAsync(d.coll_tab, 0, (size_t)coll_cap * 8, s));
-      k_build_coll<<<(uint32_t)((c->n_ops + 255) / 256), 256, 0, s>>>(d);
-      c->launches++;
+      clear_later(d.coll_tab, (size_t)coll_cap * 8);
     }
   }
   d.work_indirect = nullptr; d.n_indirect = 0; d.coll_list = nullptr;
@@ -1054,39 +1075,56 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   d.ctx_tab = nullptr; d.evt = nullptr; d.n_evt = 0; d.seen_tab = nullptr; d.row_key = nullptr; d.row_first = nullptr; d.corr_zero = nullptr;
   d.work_origin = 0; d.wait_pass = 0;
   if (n_sync + n_cuda_events > 0) {
-    K2J_CUDA(c, c->corr_zero.reserve(corr_cap / 8 + 8));
+    const uint64_t zero_bytes = (corr_cap / 8 + 15) & ~7ull;  // one bit per table slot, whole words
+    K2J_CUDA(c, c->corr_zero.reserve(zero_bytes));
     d.corr_zero = c->corr_zero.as<uint32_t>();
-    K2J_CUDA(c, cudaMemsetAsync(d.corr_zero, 0, corr_cap / 8 + 8, s));
+    clear_later(d.corr_zero, zero_bytes);
     const uint32_t ctx_cap = 1u << 14;   // distinct CUDA contexts of one trace: a few per device
     K2J_CUDA(c, c->ctx_tab.reserve((size_t)ctx_cap * 8));
     d.ctx_tab = c->ctx_tab.as<unsigned long long>(); d.ctx_mask = ctx_cap - 1;
-    K2J_CUDA(c, cudaMemsetAsync(d.ctx_tab, 0, (size_t)ctx_cap * 8, s));
-    const uint64_t n_named = d.cls_begin[C_OVERHEAD] - d.cls_begin[C_KERNEL];
-    if (n_named) { k_build_ctx<<<(uint32_t)((n_named + 255) / 256), 256, 0, s>>>(d); c->launches++; }
-    if (n_sync && n_cuda_events) {
-      k2j_status st = sort_cuda_events(c, n_cuda_events);
-      if (st) return st;
-    }
+    clear_later(d.ctx_tab, (size_t)ctx_cap * 8);
     if (totals[C_WAIT]) {
       const uint32_t seen_cap = 1u << 16;  // (device, stream) pairs
       K2J_CUDA(c, c->seen_tab.reserve((size_t)seen_cap * 8));
       d.seen_tab = c->seen_tab.as<unsigned long long>(); d.seen_mask = seen_cap - 1;
-      K2J_CUDA(c, cudaMemsetAsync(d.seen_tab, 0, (size_t)seen_cap * 8, s));
+      clear_later(d.seen_tab, (size_t)seen_cap * 8);
     }
     if (totals[C_SYNC]) {
       const uint32_t row_cap = pow2_at_least(2 * totals[C_SYNC] + 16);
       K2J_CUDA(c, c->row_key.reserve((size_t)row_cap * 8));
       K2J_CUDA(c, c->row_first.reserve((size_t)row_cap * 4));
       d.row_key = c->row_key.as<unsigned long long>(); d.row_first = c->row_first.as<uint32_t>(); d.row_mask = row_cap - 1;
-      K2J_CUDA(c, cudaMemsetAsync(d.row_key, 0, (size_t)row_cap * 8, s));
-      K2J_CUDA(c, cudaMemsetAsync(d.row_first, 0xFF, (size_t)row_cap * 4, s));
+      clear_later(d.row_key, (size_t)row_cap * 8);
+      clear_later(d.row_first, (size_t)row_cap * 4, true);
     }
   }
-  if (d.n_ext_all) { k_build_corr<<<(uint32_t)((d.n_ext_all + 255) / 256), 256, 0, s>>>(d, own_begin, own_end); c->launches++; }
-  if (d.op_bits != nullptr) {  // the other shards' ids came as bitmaps: the table holds this shard's own ids only
-    const uint64_t first = (uint64_t)c->g_ops_stride * c->g_rank, last = first + d.own_n_ops;
-    if (last > first) { k_build_ops<<<(uint32_t)((last - first + 255) / 256), 256, 0, s>>>(d, first, last); c->launches++; }
-  } else if (d.n_join_ops) { k_build_ops<<<(uint32_t)((d.n_join_ops + 255) / 256), 256, 0, s>>>(d, 0, d.n_join_ops); c->launches++; }
+  k2j_status st_clear = run_clear(c, clear);
+  if (st_clear) return st_clear;
+  if (mark_corr) { k_mark_corr<<<(uint32_t)((d.ops_begin + 255) / 256), 256, 0, s>>>(d); c->launches++; }
+  if (d.coll_tab != nullptr) { k_build_coll<<<(uint32_t)((c->n_ops + 255) / 256), 256, 0, s>>>(d); c->launches++; }
+  if (n_sync + n_cuda_events > 0) {
+    const uint64_t n_named = d.cls_begin[C_OVERHEAD] - d.cls_begin[C_KERNEL];
+    if (n_named) { k_build_ctx<<<(uint32_t)((n_named + 255) / 256), 256, 0, s>>>(d); c->launches++; }
+    if (n_sync && n_cuda_events) {
+      k2j_status st = sort_cuda_events(c, n_cuda_events);
+      if (st) return st;
+    }
+  }
+  // (several shards whose other ids came as bitmaps: the table holds this shard's own ids only)
+  JoinJobs jobs{};
+  jobs.ops_first = d.op_bits != nullptr ? (uint64_t)c->g_ops_stride * c->g_rank : 0;
+  jobs.ops_last = d.op_bits != nullptr ? jobs.ops_first + d.own_n_ops : d.n_join_ops;
+  jobs.own_begin = own_begin; jobs.own_end = own_end; jobs.comms_flag = c->comms_flag.as<uint32_t>();
+  auto launch_join = [&](bool ops, bool others) {
+    const uint64_t items[J_COUNT] = {others ? c->n_tid + c->n_ops : 0, others && d.has_comms ? c->n_ops : 0,
+                                     ops ? jobs.ops_last - jobs.ops_first : 0, others ? d.n_ext_all : 0};
+    uint32_t blocks = 0;
+    for (int k = 0; k < J_COUNT; k++) jobs.end[k] = blocks += (uint32_t)((items[k] + kJoinThreads - 1) / kJoinThreads);
+    if (blocks) { k_build_join<<<blocks, kJoinThreads, 0, s>>>(d, jobs); c->launches++; }
+  };
+  // with a filter the ops job asks which ids the correlation records name, so it waits for them
+  launch_join(!filter, true);
+  if (filter) launch_join(true, false);
   if (d.n_ext_all) { k_resolve_corr<<<(corr_cap + 255) / 256, 256, 0, s>>>(d); c->launches++; }
   K2J_CUDA(c, cudaGetLastError());
   K2J_CUDA(c, cudaEventRecord(c->ev[2], s));
@@ -1115,15 +1153,13 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     }
     K2J_CUDA(c, cudaGetLastError());
     K2J_CUDA(c, cudaEventRecord(c->ev[3], s));
-    k2j_status st = run_scan(c, d.ev_size, d.n_events, 1, c->ev_off.as<uint64_t>(), c->scan_totals.as<uint64_t>() + 20, &c->launches);
+    c->h_totals[25] = 0; c->h_totals[26] = 0;
+    ScanReport rep;
+    if (n_gpu_events) { rep.at = c->n_ops; rep.at_dst = c->h_totals + 21; }
+    if (d.has_comms) { rep.flag = d.has_comms; rep.flag_dst = c->h_totals + 25; }
+    if (d.coll_list) { rep.count = &d.counters->n_coll; rep.count_dst = c->h_totals + 26; }
+    k2j_status st = run_scan(c, d.ev_size, d.n_events, 1, c->ev_off.as<uint64_t>(), c->h_totals + 20, &c->launches, rep);
     if (st) return st;
-    K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 20, c->scan_totals.as<uint64_t>() + 20, 8, cudaMemcpyDeviceToHost, s));
-    if (n_gpu_events)
-      K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 21, c->ev_off.as<uint64_t>() + c->n_ops, 8, cudaMemcpyDeviceToHost, s));
-    c->h_totals[25] = 0;
-    if (d.has_comms) K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 25, d.has_comms, 4, cudaMemcpyDeviceToHost, s));
-    c->h_totals[26] = 0;
-    if (d.coll_list) K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 26, &d.counters->n_coll, 8, cudaMemcpyDeviceToHost, s));
     K2J_CUDA(c, cudaEventRecord(c->ev[4], s));
     K2J_CUDA(c, cudaStreamSynchronize(s));
     total_bytes = c->h_totals[20];
@@ -1310,9 +1346,8 @@ k2j_status k2j_exclusive_scan_u32(k2j_ctx* c, const uint32_t* sizes, uint64_t n,
   *total = 0;
   if (n == 0) return K2J_OK;
   uint32_t launches = 0;
-  k2j_status st = run_scan(c, sizes, n, 1, offsets, c->scan_totals.as<uint64_t>() + 24, &launches);
+  k2j_status st = run_scan(c, sizes, n, 1, offsets, c->h_totals + 24, &launches);
   if (st) return st;
-  K2J_CUDA(c, cudaMemcpyAsync(c->h_totals + 24, c->scan_totals.as<uint64_t>() + 24, 8, cudaMemcpyDeviceToHost, c->stream));
   K2J_CUDA(c, cudaStreamSynchronize(c->stream));
   *total = c->h_totals[24];
   return K2J_OK;

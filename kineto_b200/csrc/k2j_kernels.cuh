@@ -589,8 +589,7 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_write(Dev d) {
 // CUPTI thread id -> system thread id.  Priority order: the explicit pairs, then every CPU-side activity
 // of this process in order (processCpuTrace -> recordThreadInfo(resourceId, getThreadId, deviceId),
 // libkineto/src/GenericActivityProfiler.cpp:272); the first writer of a thread id wins.
-__global__ void k_build_tids(Dev d) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_tids(const Dev& d, uint64_t i) {
   if (i >= (uint64_t)d.n_tid_pairs + d.n_ops) return;
   uint32_t key;
   if (i < d.n_tid_pairs) key = (uint32_t)d.tid_pairs[2 * i];
@@ -651,11 +650,10 @@ __global__ void k_take_wanted(Dev d, const uint32_t* flags, const uint64_t* at, 
 }
 // Is any CPU-side activity of this run named record_param_comms (bit 0: kernel events look at their linked op's
 // name only if so), is any an instant event (bit 1)?
-__global__ void k_find_comms(Dev d, uint32_t* flag, int comms_on) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void find_comms(const Dev& d, uint64_t i, uint32_t* flag) {
   if (i >= d.n_ops) return;
   const uint32_t name = d.op_name[i];
-  if (comms_on && name < d.n_strings && d.str_class[name] == 1u) atomicOr(flag, 1u);
+  if (name < d.n_strings && d.str_class[name] == 1u) atomicOr(flag, 1u);
   const int type = d.op_type[i];
   if (type == 9 || type == 17 || type == 26 || type == 28) atomicOr(flag, 2u);  // instant and counter events: written by the same extra launch
 }
@@ -668,8 +666,7 @@ __global__ void k_build_coll(Dev d) {
   if (!tab_insert(d.coll_tab, d.coll_mask, (uint32_t)d.op_id[i], (uint32_t)i)) atomicAdd(&d.counters->device_check, 1ull);
 }
 // CPU-op id -> position (last writer wins): activityMap_[id] = op, GenericActivityProfiler.cpp:262.
-__global__ void k_build_ops(Dev d, uint64_t first, uint64_t last) {
-  const uint64_t i = first + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_ops(const Dev& d, uint64_t i, uint64_t last) {
   uint32_t id = 0u;
   const bool in = i < last && op_id_at(d, i, &id);
   const bool valid = in && (d.need_op == nullptr || bit_test(d.need_op, d.need_op_mask, id));
@@ -681,8 +678,7 @@ __global__ void k_build_ops(Dev d, uint64_t first, uint64_t last) {
 }
 // correlation id -> index of the winning EXTERNAL_CORRELATION record (handleCorrelationActivity,
 // CuptiActivityProfiler.cpp:290-302).  `count_invalid`: only the shard that owns a record counts it.
-__global__ void k_build_corr(Dev d, uint64_t own_begin, uint64_t own_end) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void build_corr(const Dev& d, uint64_t i, uint64_t own_begin, uint64_t own_end) {
   ExtRec e;
   if (i >= d.n_ext_all || !ext_at(d, i, &e)) return;
   bool ok = true;
@@ -706,13 +702,67 @@ __global__ void k_build_corr(Dev d, uint64_t own_begin, uint64_t own_end) {
   if (!ok) atomicAdd(&d.counters->device_check, 1ull);
 }
 
+// The join tables in one launch: four independent jobs, each with a range of blocks of its own (a job that is not
+// wanted has no blocks).  A launch costs a short trace more than any of these jobs: one trace of 150 launches spent
+// four launches and eight memory sets here.
+constexpr int kJoinThreads = 256;
+enum : int { J_TIDS = 0, J_COMMS, J_OPS, J_CORR, J_COUNT };
+struct JoinJobs {
+  uint32_t end[J_COUNT];            // first block past each job
+  uint64_t ops_first, ops_last;     // range of positions of the op ids
+  uint64_t own_begin, own_end;      // this shard's EXTERNAL_CORRELATION records
+  uint32_t* comms_flag;
+};
+__global__ void __launch_bounds__(kJoinThreads) k_build_join(Dev d, JoinJobs j) {
+  const uint32_t b = blockIdx.x;
+  auto at = [&](uint32_t first) { return (uint64_t)(b - first) * kJoinThreads + threadIdx.x; };
+  if (b < j.end[J_TIDS]) build_tids(d, at(0u));
+  else if (b < j.end[J_COMMS]) find_comms(d, at(j.end[J_TIDS]), j.comms_flag);
+  else if (b < j.end[J_OPS]) build_ops(d, j.ops_first + at(j.end[J_COMMS]), j.ops_last);
+  else build_corr(d, at(j.end[J_OPS]), j.own_begin, j.own_end);
+}
+
+// ---- initial values of a run's tables, all in one launch ----
+constexpr int kClearThreads = 256, kClearMax = 24;
+struct ClearList {
+  struct { uint64_t* p; uint64_t words; } r[kClearMax];  // 16-byte aligned, a count of 8-byte words
+  uint32_t n = 0, ones = 0;                              // bit k of ones: region k is set to all ones, not zeros
+};
+__global__ void __launch_bounds__(kClearThreads) k_clear(const __grid_constant__ ClearList l) {
+  const uint64_t first = (uint64_t)blockIdx.x * kClearThreads + threadIdx.x, step = (uint64_t)gridDim.x * kClearThreads;
+  for (uint32_t k = 0; k < l.n; k++) {
+    const uint32_t x = (l.ones >> k) & 1u ? 0xFFFFFFFFu : 0u;
+    const uint64_t pairs = l.r[k].words >> 1;
+    uint4* p = reinterpret_cast<uint4*>(l.r[k].p);
+    for (uint64_t i = first; i < pairs; i += step) p[i] = make_uint4(x, x, x, x);
+    if ((l.r[k].words & 1ull) && first == 0) l.r[k].p[l.r[k].words - 1] = ((uint64_t)x << 32) | x;
+  }
+}
+
 // ---- exclusive scan: u32 in -> u64 out, `gridDim.y` independent columns -----------------------------
+// Three shapes by length (run_scan): one launch of a block per column, two launches whose second adds up the sums in
+// front of its block itself, three launches with the sums scanned in between.  No block ever waits for another one.
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanSmallThreads = 1024;
+constexpr int kScanSmallTile = kScanSmallThreads * kScanItems;
 
+// What the host wants to know once a scan is done, written straight to its pinned memory by the scan's last kernel: a
+// copy of eight bytes on the stream costs as much as a small kernel.  `at`: element of the (single) column whose offset goes to at_dst.
+struct ScanReport {
+  uint64_t* at_dst = nullptr; uint64_t at = ~0ull;
+  uint64_t* flag_dst = nullptr; const uint32_t* flag = nullptr;
+  uint64_t* count_dst = nullptr; const unsigned long long* count = nullptr;
+};
+__device__ __forceinline__ void scan_report(const ScanReport& r) {
+  if (r.flag != nullptr) *r.flag_dst = *r.flag;
+  if (r.count != nullptr) *r.count_dst = *r.count;
+}
+
+template <int THREADS = kScanThreads>
 __device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* total) {
-  __shared__ uint64_t s_warp[kScanThreads / 32];
+  __shared__ uint64_t s_warp[THREADS / 32];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint64_t x = v;
 #pragma unroll
@@ -722,11 +772,43 @@ __device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t v, uint64_t* t
   __syncthreads();
   uint64_t base = 0, tot = 0;
 #pragma unroll
-  for (int i = 0; i < kScanThreads / 32; i++) { if ((uint32_t)i < w) base += s_warp[i]; tot += s_warp[i]; }
+  for (int i = 0; i < THREADS / 32; i++) { if ((uint32_t)i < w) base += s_warp[i]; tot += s_warp[i]; }
   *total = tot;
   return base + x - v;
 }
+// A thread's kScanItems elements from `base` on: loads, and the stores of their exclusive offsets.
+__device__ __forceinline__ uint64_t scan_load(const uint32_t* src, uint64_t base, uint64_t n, uint32_t (&v)[kScanItems]) {
+  uint64_t s = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) { const uint64_t i = base + k; v[k] = i < n ? src[i] : 0; s += v[k]; }
+  return s;
+}
+__device__ __forceinline__ void scan_store(uint64_t* dst, uint64_t base, uint64_t n, const uint32_t (&v)[kScanItems], uint64_t ex, const ScanReport& rep) {
+#pragma unroll
+  for (int k = 0; k < kScanItems; k++) {
+    const uint64_t i = base + k;
+    if (i < n) dst[i] = ex;
+    if (i == rep.at) *rep.at_dst = ex;
+    ex += v[k];
+  }
+}
 
+__global__ void __launch_bounds__(kScanSmallThreads) k_scan_small(const uint32_t* in, uint64_t n, uint64_t* totals, uint64_t* out, ScanReport rep) {
+  const uint32_t* src = in + (uint64_t)blockIdx.x * n;
+  uint64_t* dst = out + (uint64_t)blockIdx.x * n;
+  uint64_t carry = 0;
+  for (uint64_t t0 = 0; t0 < n; t0 += kScanSmallTile) {
+    const uint64_t base = t0 + (uint64_t)threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    const uint64_t s = scan_load(src, base, n, v);
+    uint64_t tot;
+    const uint64_t ex = carry + block_exclusive_scan<kScanSmallThreads>(s, &tot);
+    scan_store(dst, base, n, v, ex, rep);
+    carry += tot;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) { totals[blockIdx.x] = carry; scan_report(rep); }
+}
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* in, uint64_t n, uint64_t col_stride, uint64_t* block_sums, uint32_t n_blocks) {
   const uint32_t* src = in + (uint64_t)blockIdx.y * col_stride;
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
@@ -755,18 +837,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint64_t* block_sums
   }
   if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint64_t n, uint64_t col_stride, const uint64_t* block_sums, uint32_t n_blocks, uint64_t* out) {
+// totals != nullptr: block_sums holds the blocks' sums as k_scan_reduce left them; every block adds up those in front
+// of it (at most kScanDirectBlocks eight-byte reads from the L2), and the last one stores the column total.
+template <bool DIRECT>
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint64_t n, uint64_t col_stride, const uint64_t* block_sums, uint32_t n_blocks,
+                                                             uint64_t* out, uint64_t* totals, ScanReport rep) {
   const uint32_t* src = in + (uint64_t)blockIdx.y * col_stride;
   uint64_t* dst = out + (uint64_t)blockIdx.y * col_stride;
+  const uint64_t* sums = block_sums + (uint64_t)blockIdx.y * n_blocks;
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
-  uint64_t s = 0;
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++) { const uint64_t i = base + k; v[k] = i < n ? src[i] : 0; s += v[k]; }
-  uint64_t tot;
-  uint64_t ex = block_exclusive_scan(s, &tot) + block_sums[(uint64_t)blockIdx.y * n_blocks + blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++) { const uint64_t i = base + k; if (i < n) dst[i] = ex; ex += v[k]; }
+  const uint64_t s = scan_load(src, base, n, v);
+  uint64_t front, tot;
+  if (DIRECT) {
+    uint64_t f = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanThreads) f += sums[b];
+    block_exclusive_scan(f, &front);
+    __syncthreads();
+  } else front = sums[blockIdx.x];
+  const uint64_t ex = block_exclusive_scan(s, &tot) + front;
+  scan_store(dst, base, n, v, ex, rep);
+  if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {
+    if (DIRECT) totals[blockIdx.y] = front + tot;
+    if (blockIdx.y == 0) scan_report(rep);
+  }
 }
 
 struct CountSink2 : CountSink {

@@ -1,0 +1,27 @@
+"""Paths that are chosen by size or by record class, at the sizes where the choice changes (results against numpy or the
+CPU restatement)."""
+import numpy as np
+import pytest
+
+import helpers
+from kineto_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+# one launch up to 2 tiles of 8192; two launches up to 4096 tiles of 2048; three above
+@pytest.mark.parametrize("n", [1, 8192, 16384, 16385, 2048 * 9 + 1, 4096 * 2048, 4096 * 2048 + 1])
+def test_exclusive_scan_at_the_edges_of_its_shapes(n):
+    import torch
+    from kineto_b200 import api
+    sizes = np.random.default_rng(n).integers(0, 1 << 20, n, dtype=np.uint32)
+    d_sizes = torch.from_numpy(sizes.view(np.int32)).to("cuda:0")
+    d_off = torch.full((n + 1,), -1, dtype=torch.int64, device="cuda:0")
+    torch.cuda.synchronize()
+    ctx = api.K2J(0)
+    total = ctx.exclusive_scan(d_sizes, d_off[:n])
+    ctx.close()
+    sums = np.cumsum(sizes, dtype=np.uint64)
+    off = d_off.cpu().numpy()
+    assert total == int(sums[-1]) and off[0] == 0 and off[n] == -1
+    assert np.array_equal(off[1:n].astype(np.uint64), sums[:-1])
