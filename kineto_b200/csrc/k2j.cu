@@ -10,7 +10,7 @@
 #include <string.h>
 
 #include <algorithm>
-#include <map>
+#include <memory_resource>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -80,8 +80,9 @@ struct k2j_ctx {
   DevBuf ds_tab, span_key, span_nstart, span_end, span_nfirst, span_row, span_out, span_cnt, ann_size, ann_off;
   DevBuf sort_keys[2], sort_vals[2], sort_hist, sort_base, sort_rank;
   DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, out, counters;
-  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 23 sort, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata
+  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 23 sort, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans
   Counters* h_counters = nullptr; // pinned
+  SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans: allocated by the first run with user-annotation spans
   void* h_stage[2] = {nullptr, nullptr};            // pinned staging buffers of k2j_write_output
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   cudaEvent_t ev[8]{};
@@ -277,30 +278,18 @@ k2j_status sort_gpu_events(k2j_ctx* c, uint64_t n) {
 // std::map over (device, stream), and inside it a std::unordered_map<int64_t, ...> over the op id,
 // filled in order of first use (libkineto/src/GenericActivityProfiler.h:341-346, .cpp:320-327) — and
 // sizes their events.  Host work is O(distinct annotations).
-// The span table as a list on the host (no order).
-k2j_status collect_spans(k2j_ctx* c, uint32_t span_cap, std::vector<SpanRec>* spans) {
-  cudaStream_t s = c->stream;
-  Dev& d = c->d;
-  K2J_CUDA(c, c->span_out.reserve((size_t)span_cap * sizeof(SpanRec)));
-  K2J_CUDA(c, c->span_cnt.reserve(16));
-  K2J_CUDA(c, cudaMemsetAsync(c->span_cnt.p, 0, 4, s));
-  k_span_collect<<<(span_cap + 255) / 256, 256, 0, s>>>(d, c->span_out.as<SpanRec>(), c->span_cnt.as<unsigned int>());
-  c->launches++;
-  unsigned int n = 0;
-  K2J_CUDA(c, cudaMemcpyAsync(&n, c->span_cnt.p, 4, cudaMemcpyDeviceToHost, s));
-  K2J_CUDA(c, cudaStreamSynchronize(s));
-  spans->resize(n);
-  if (n == 0) return K2J_OK;
-  K2J_CUDA(c, cudaMemcpyAsync(spans->data(), c->span_out.p, (size_t)n * sizeof(SpanRec), cudaMemcpyDeviceToHost, s));
-  K2J_CUDA(c, cudaStreamSynchronize(s));
+// The span table as a list on the host (no order), after a stream synchronisation that followed k_span_collect: the
+// kernel puts the first kPinnedSpans of them into pinned memory, so that a trace with few spans pays no copy for them.
+constexpr uint32_t kPinnedSpans = 4096;
+k2j_status take_spans(k2j_ctx* c, std::vector<SpanRec>* spans) {
+  const uint32_t n = (uint32_t)c->h_totals[28];
+  spans->assign(c->h_spans, c->h_spans + std::min(n, kPinnedSpans));
+  if (n > kPinnedSpans) {
+    spans->resize(n);
+    K2J_CUDA(c, cudaMemcpyAsync(spans->data(), c->span_out.p, (size_t)n * sizeof(SpanRec), cudaMemcpyDeviceToHost, c->stream));
+    K2J_CUDA(c, cudaStreamSynchronize(c->stream));
+  }
   return K2J_OK;
-}
-k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint32_t* n_out, uint64_t* bytes_out);
-k2j_status order_annotations(k2j_ctx* c, uint32_t span_cap, uint32_t* n_out, uint64_t* bytes_out) {
-  std::vector<SpanRec> spans;
-  k2j_status st = collect_spans(c, span_cap, &spans);
-  if (st) return st;
-  return size_annotations(c, spans, n_out, bytes_out);
 }
 // Puts spans in logging order (see above), leaves them in span_out and sizes their events (ann_size, ann_off).
 k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint32_t* n_out, uint64_t* bytes_out) {
@@ -310,18 +299,28 @@ k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint3
   *n_out = n; *bytes_out = 0;
   if (n == 0) return K2J_OK;
   K2J_CUDA(c, c->span_out.reserve((size_t)n * sizeof(SpanRec)));
-  std::map<std::pair<int64_t, int64_t>, std::vector<const SpanRec*>> by_stream;
-  for (const SpanRec& r : spans) by_stream[{(int64_t)r.device, (int64_t)r.stream}].push_back(&r);
-  std::vector<SpanRec> ordered;
-  ordered.reserve(n);
-  for (auto& kv : by_stream) {
-    auto& v = kv.second;
-    std::sort(v.begin(), v.end(), [](const SpanRec* a, const SpanRec* b) { return a->first_event < b->first_event; });
-    std::unordered_map<int64_t, const SpanRec*> m;
-    for (const SpanRec* r : v) m.insert({(int64_t)r->op_id, r});
-    for (auto& e : m) ordered.push_back(*e.second);
+  // by (device, stream), inside one by first use; the order of one (device, stream)'s spans is then the iteration order
+  // of a hash map filled in that order (a map of one element needs none).  The maps' nodes come from one buffer: a
+  // trace of 10 annotations over 256 streams holds 2 560 of them.
+  std::vector<const SpanRec*> by_use(n);
+  for (unsigned int i = 0; i < n; i++) by_use[i] = &spans[i];
+  std::sort(by_use.begin(), by_use.end(), [](const SpanRec* a, const SpanRec* b) {
+    return a->device != b->device ? a->device < b->device : a->stream != b->stream ? a->stream < b->stream : a->first_event < b->first_event;
+  });
+  std::vector<SpanRec> room;
+  SpanRec* ordered = c->h_spans;  // (the spans were copied out of it)
+  if (!ordered || n > kPinnedSpans) { room.resize(n); ordered = room.data(); }
+  SpanRec* next = ordered;
+  std::vector<char> node_space(64 * 1024);
+  for (unsigned int i = 0, e; i < n; i = e) {
+    for (e = i + 1; e < n && by_use[e]->device == by_use[i]->device && by_use[e]->stream == by_use[i]->stream;) e++;
+    if (e == i + 1) { *next++ = *by_use[i]; continue; }
+    std::pmr::monotonic_buffer_resource nodes(node_space.data(), node_space.size());
+    std::pmr::unordered_map<int64_t, const SpanRec*> m(&nodes);
+    for (unsigned int k = i; k < e; k++) m.insert({(int64_t)by_use[k]->op_id, by_use[k]});
+    for (auto& kv : m) *next++ = *kv.second;
   }
-  K2J_CUDA(c, cudaMemcpyAsync(c->span_out.p, ordered.data(), (size_t)n * sizeof(SpanRec), cudaMemcpyHostToDevice, s));
+  K2J_CUDA(c, cudaMemcpyAsync(c->span_out.p, ordered, (size_t)n * sizeof(SpanRec), cudaMemcpyHostToDevice, s));
   K2J_CUDA(c, c->ann_size.reserve((size_t)n * 4));
   K2J_CUDA(c, c->ann_off.reserve((size_t)n * 8));
   k_annotations<false><<<(n + kEventThreads - 1) / kEventThreads, kEventThreads, 0, s>>>(
@@ -386,6 +385,7 @@ void k2j_destroy(k2j_ctx* c) {
     b->release();
   if (c->h_totals) cudaFreeHost(c->h_totals);
   if (c->h_counters) cudaFreeHost(c->h_counters);
+  if (c->h_spans) cudaFreeHost(c->h_spans);
   for (int i = 0; i < 2; i++) {
     if (c->h_stage[i]) cudaFreeHost(c->h_stage[i]);
     if (c->stage_ev[i]) cudaEventDestroy(c->stage_ev[i]);
@@ -1023,6 +1023,10 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     K2J_CUDA(c, c->span_end.reserve((size_t)span_cap * 8));
     K2J_CUDA(c, c->span_nfirst.reserve((size_t)span_cap * 8));
     K2J_CUDA(c, c->span_row.reserve((size_t)span_cap * 4));
+    K2J_CUDA(c, c->span_out.reserve((size_t)span_cap * sizeof(SpanRec)));
+    K2J_CUDA(c, c->span_cnt.reserve(16));
+    if (!c->h_spans) K2J_CUDA(c, cudaMallocHost((void**)&c->h_spans, kPinnedSpans * sizeof(SpanRec)));
+    clear_later(c->span_cnt.p, 8);
     d.ds_tab = c->ds_tab.as<unsigned long long>(); d.ds_mask = ds_cap - 1;
     d.span_key = c->span_key.as<unsigned long long>(); d.span_nstart = c->span_nstart.as<unsigned long long>();
     d.span_end = c->span_end.as<unsigned long long>(); d.span_nfirst = c->span_nfirst.as<unsigned long long>();
@@ -1158,6 +1162,11 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     if (n_gpu_events) { rep.at = c->n_ops; rep.at_dst = c->h_totals + 21; }
     if (d.has_comms) { rep.flag = d.has_comms; rep.flag_dst = c->h_totals + 25; }
     if (d.coll_list) { rep.count = &d.counters->n_coll; rep.count_dst = c->h_totals + 26; }
+    if (spans_on) {  // the span table is complete: the host has the list when it learns the text's size
+      k_span_collect<<<(span_cap + 255) / 256, 256, 0, s>>>(d, c->span_out.as<SpanRec>(), c->span_cnt.as<unsigned long long>(), c->h_spans, kPinnedSpans);
+      c->launches++;
+      rep.spans = c->span_cnt.as<unsigned long long>(); rep.spans_dst = c->h_totals + 28;
+    }
     k2j_status st = run_scan(c, d.ev_size, d.n_events, 1, c->ev_off.as<uint64_t>(), c->h_totals + 20, &c->launches, rep);
     if (st) return st;
     K2J_CUDA(c, cudaEventRecord(c->ev[4], s));
@@ -1167,10 +1176,12 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     if (spans_on && c->have_global_join) {
       // several shards: this shard's part of every span waits for the caller to merge it with the other shards' parts
       // (k2j_partial_spans, k2j_append_spans); nothing is written here
-      k2j_status st2 = collect_spans(c, span_cap, &c->partial_spans);
+      k2j_status st2 = take_spans(c, &c->partial_spans);
       if (st2) return st2;
     } else if (spans_on) {
-      k2j_status st2 = order_annotations(c, span_cap, &n_spans, &ann_bytes);
+      std::vector<SpanRec> spans;
+      k2j_status st2 = take_spans(c, &spans);
+      if (!st2) st2 = size_annotations(c, spans, &n_spans, &ann_bytes);
       if (st2) return st2;
     }
     (void)ev_blocks;

@@ -754,10 +754,12 @@ struct ScanReport {
   uint64_t* at_dst = nullptr; uint64_t at = ~0ull;
   uint64_t* flag_dst = nullptr; const uint32_t* flag = nullptr;
   uint64_t* count_dst = nullptr; const unsigned long long* count = nullptr;
+  uint64_t* spans_dst = nullptr; const unsigned long long* spans = nullptr;
 };
 __device__ __forceinline__ void scan_report(const ScanReport& r) {
   if (r.flag != nullptr) *r.flag_dst = *r.flag;
   if (r.count != nullptr) *r.count_dst = *r.count;
+  if (r.spans != nullptr) *r.spans_dst = *r.spans;
 }
 
 template <int THREADS = kScanThreads>
@@ -2512,7 +2514,8 @@ __global__ void k_sort_remap(Dev d, const uint32_t* rank) {
 }
 
 // ---- user-annotation spans: collect, then format in the order the host determined ----
-__global__ void k_span_collect(Dev d, SpanRec* out, unsigned int* n_out) {
+// The list goes to `out`, its first n_front records to `front` (pinned host memory) as well.
+__global__ void k_span_collect(Dev d, SpanRec* out, unsigned long long* n_out, SpanRec* front, uint32_t n_front) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j > d.span_mask) return;
   const unsigned long long key = d.span_key[j];
@@ -2524,7 +2527,9 @@ __global__ void k_span_collect(Dev d, SpanRec* out, unsigned int* n_out) {
   r.first_event = ~d.span_nfirst[j];
   r.device = (uint32_t)(ds >> 32); r.stream = (uint32_t)ds;
   r.op_id = (int32_t)(uint32_t)key; r.op_row = d.span_row[j];
-  out[atomicAdd(n_out, 1u)] = r;
+  const uint32_t at = (uint32_t)atomicAdd(n_out, 1ull);
+  out[at] = r;
+  if (at < n_front) front[at] = r;
 }
 
 // One thread per span, in emission order: the gpu_user_annotation event that
