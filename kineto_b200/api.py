@@ -39,6 +39,9 @@ class DeviceProps(C.Structure):
                 ("reserved_smem_per_block", C.c_uint64)]
 
 
+DEVICE_PROPS = np.dtype(DeviceProps)
+
+
 class Ops(C.Structure):
     _fields_ = [("n_ops", C.c_uint64), ("start_ns", C.c_void_p), ("end_ns", C.c_void_p), ("id", C.c_void_p),
                 ("device", C.c_void_p), ("resource", C.c_void_p), ("thread", C.c_void_p), ("type", C.c_void_p),
@@ -188,12 +191,12 @@ class K2J:
                     int(p["conv_t0_approx"]), int(p["conv_scale_mant"]), int(p["conv_scale_exp"]),
                     activity_type_mask(int(p["mode"]), int(p["flags"])))
         n = int(p["n_devices"])
-        props = (DeviceProps * max(n, 1))()
-        for i in range(n):
-            d = trace.devprops[i]
-            for name, _ in DeviceProps._fields_:
-                setattr(props[i], name, int(d[name]))
-        self._check(self.lib.k2j_set_params(self.h, C.byref(cp), props))
+        if n > len(trace.devprops):
+            raise IndexError("fewer device rows than n_devices")
+        props = np.zeros(max(n, 1), DEVICE_PROPS)  # column by column: field by field cost 40 us for eight devices
+        for name in DEVICE_PROPS.names if n > 0 else ():
+            props[name][:n] = trace.devprops[name][:n]
+        self._check(self.lib.k2j_set_params(self.h, C.byref(cp), props.ctypes.data_as(C.POINTER(DeviceProps))))
 
     def set_arrays(self, a: dict, buftab: np.ndarray, tidmap: np.ndarray):
         """`a` maps Trace attribute names to numpy arrays (host) or torch tensors (host or device)."""

@@ -274,10 +274,6 @@ k2j_status sort_gpu_events(k2j_ctx* c, uint64_t n) {
   return K2J_OK;
 }
 
-// Collects the span table, puts the spans in the order GpuUserEventMap::logEvents walks them — a
-// std::map over (device, stream), and inside it a std::unordered_map<int64_t, ...> over the op id,
-// filled in order of first use (libkineto/src/GenericActivityProfiler.h:341-346, .cpp:320-327) — and
-// sizes their events.  Host work is O(distinct annotations).
 // The span table as a list on the host (no order), after a stream synchronisation that followed k_span_collect: the
 // kernel puts the first kPinnedSpans of them into pinned memory, so that a trace with few spans pays no copy for them.
 constexpr uint32_t kPinnedSpans = 4096;
@@ -291,7 +287,10 @@ k2j_status take_spans(k2j_ctx* c, std::vector<SpanRec>* spans) {
   }
   return K2J_OK;
 }
-// Puts spans in logging order (see above), leaves them in span_out and sizes their events (ann_size, ann_off).
+// Puts the spans in the order GpuUserEventMap::logEvents walks them — a
+// std::map over (device, stream), and inside it a std::unordered_map<int64_t, ...> over the op id,
+// filled in order of first use (libkineto/src/GenericActivityProfiler.h:341-346, .cpp:320-327); leaves them in
+// span_out and sizes their events (ann_size, ann_off).  Host work is O(distinct annotations).
 k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint32_t* n_out, uint64_t* bytes_out) {
   cudaStream_t s = c->stream;
   Dev& d = c->d;
@@ -413,9 +412,9 @@ k2j_status k2j_set_params(k2j_ctx* c, const k2j_params* p, const k2j_device_prop
     return fail(c, K2J_ERR_INVALID_ARGUMENT, "converter scale must be a normalised 64-bit significand");
   K2J_CUDA(c, cudaSetDevice(c->device));
   c->params = *p;
-  c->props.resize(p->n_devices);
+  std::vector<DevProps> fresh(p->n_devices);
   for (int i = 0; i < p->n_devices; i++) {
-    DevProps& d = c->props[i];
+    DevProps& d = fresh[i];
     d.major = props[i].major; d.minor = props[i].minor;
     d.max_threads_per_block = props[i].max_threads_per_block; d.max_threads_per_sm = props[i].max_threads_per_sm;
     d.regs_per_block = props[i].regs_per_block; d.regs_per_sm = props[i].regs_per_sm;
@@ -423,10 +422,18 @@ k2j_status k2j_set_params(k2j_ctx* c, const k2j_params* p, const k2j_device_prop
     d.smem_per_block = props[i].smem_per_block; d.smem_per_block_optin = props[i].smem_per_block_optin;
     d.smem_per_sm = props[i].smem_per_sm; d.reserved_smem_per_block = props[i].reserved_smem_per_block;
   }
-  K2J_CUDA(c, c->d_props.reserve(std::max<size_t>(1, c->props.size()) * sizeof(DevProps)));
-  if (!c->props.empty())
-    K2J_CUDA(c, cudaMemcpyAsync(c->d_props.p, c->props.data(), c->props.size() * sizeof(DevProps), cudaMemcpyHostToDevice, c->stream));
-  K2J_CUDA(c, cudaStreamSynchronize(c->stream));  // c->props may be resized by the next call
+  static_assert(sizeof(DevProps) == 8 * sizeof(int32_t) + 4 * sizeof(uint64_t), "no padding: compared as bytes");
+  // rows equal to the last call's are on the GPU already
+  if (c->d_props.p && fresh.size() == c->props.size() && (fresh.empty() || memcmp(fresh.data(), c->props.data(), fresh.size() * sizeof(DevProps)) == 0)) {
+    c->have_params = true;
+    return K2J_OK;
+  }
+  c->have_params = false;  // until the upload is known to have worked
+  c->props.clear();
+  K2J_CUDA(c, c->d_props.reserve(std::max<size_t>(1, fresh.size()) * sizeof(DevProps)));
+  if (!fresh.empty()) K2J_CUDA(c, cudaMemcpyAsync(c->d_props.p, fresh.data(), fresh.size() * sizeof(DevProps), cudaMemcpyHostToDevice, c->stream));
+  K2J_CUDA(c, cudaStreamSynchronize(c->stream));  // `fresh` goes out of use
+  c->props = fresh;
   c->have_params = true;
   return K2J_OK;
 }

@@ -11,7 +11,7 @@
 //   k_scan_*         exclusive scans (chunk counts, later event sizes)
 //   k_seg_write      per chunk: walk again, fill the per-class work lists, insert
 //                    EXTERNAL_CORRELATION records into the correlation tables (last writer wins)
-//   k_build_ops      CPU-op id -> row table (last writer wins)
+//   k_build_join     the join tables: correlation ids, CPU-op ids (last writer wins), thread ids
 //   k_events<Count>  one thread per event, class-sorted: exact JSON byte length of the event
 //   k_events<Write>  same traversal, bytes go straight to their final offset
 #pragma once

@@ -25,3 +25,21 @@ def test_exclusive_scan_at_the_edges_of_its_shapes(n):
     off = d_off.cpu().numpy()
     assert total == int(sums[-1]) and off[0] == 0 and off[n] == -1
     assert np.array_equal(off[1:n].astype(np.uint64), sums[:-1])
+
+
+def test_device_rows_that_change_between_calls_of_one_context():
+    """Equal device rows are not uploaded again; changed ones are, and so is the way back."""
+    from kineto_b200 import api
+    a = synth.gen_kernel_launches(300, seed=41, pool_size=20)
+    b = synth.gen_kernel_launches(300, seed=41, pool_size=20)
+    b.devprops = b.devprops.copy()
+    b.devprops["num_sms"] = 7
+    b.devprops["max_threads_per_sm"] = 1024
+    want = {id(t): helpers.run_port(t)[0] for t in (a, b)}
+    assert want[id(a)] != want[id(b)]
+    ctx = api.K2J(0)
+    for t in (a, a, b, b, a):
+        ctx.load(t)
+        ctx.run()
+        assert ctx.copy_output().tobytes() == want[id(t)]
+    ctx.close()
