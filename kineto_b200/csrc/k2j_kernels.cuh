@@ -373,8 +373,17 @@ __device__ __forceinline__ uint32_t code_class(uint32_t code) {
 // (twelve 8-bit counts packed in three words: a 4 KiB chunk holds at most 170 records).  Kind -> code and
 // class -> count increments come from two small tables in shared memory, so neither the decode nor
 // the walk branches on the record kind.
+// Walks of a chunk meet soon: a walk that starts inside a record reads payload as kinds, ends, or lands on a record and
+// from there on is the walk of that record.  So each lane walks only until it has passed slot kMergeSlots; of the lanes
+// that stand on one slot then, one goes on for all, and the block packs these few of all its chunks into its first
+// warps for the long rest.  The kernel is bound by the issue of its walks' instructions (83 % of the slots when all 26
+// walks of a chunk ran to its end).  Segmentation stage, 11.5 M mixed records: 557 -> 532 us; 1 M launches: 256 -> 249.
+constexpr uint32_t kMergeSlots = 96;
 __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
-  __shared__ uint8_t s_code[kSegWarps][kChunkSlots];
+  __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots];
+  __shared__ uint32_t s_lead[kSegWarps * 32], s_rest[kSegWarps * 32][4], s_n_lead;  // walks that go on: chunk << 16 | slot; where they end, counts
+  __shared__ uint16_t s_nvalid[kSegWarps];
+  __shared__ bool s_last[kSegWarps];
   __shared__ uint8_t s_kind[64];     // slot code of record kinds 0..63 (CUSTOM1 correlation records add one class)
   __shared__ uint32_t s_inc[256][3]; // per slot code: increments of the three packed count words
   static_assert(kSegWarps * 32 == 256, "one thread per slot code");
@@ -388,11 +397,13 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
     } else if ((threadIdx.x & 31u) != 0u) inc[C_UNEXPECTED >> 2] = 1u << (8 * (C_UNEXPECTED & 3));  // a record that is stepped over
     s_inc[threadIdx.x][0] = inc[0]; s_inc[threadIdx.x][1] = inc[1]; s_inc[threadIdx.x][2] = inc[2];
   }
+  if (threadIdx.x == 0) s_n_lead = 0;
   __syncthreads();
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunk = blockIdx.x * kSegWarps + w;
-  if (chunk >= d.n_chunks) return;
-  const ChunkGeom g = chunk_geom(d, chunk);
+  const bool live = chunk < d.n_chunks;
+  ChunkGeom g{0, 0, false};
+  if (live) g = chunk_geom(d, chunk);
   const uint2* words = reinterpret_cast<const uint2*>(d.cupti);
 #pragma unroll
   for (int j = 0; j < kChunkSlots / 128; j++) {
@@ -419,19 +430,56 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
   __syncwarp();
   uint8_t code = kEntryNone;
   uint32_t c0 = 0, c1 = 0, c2 = 0;  // 8-bit counts of columns 0-3, 4-7, 8-11
-  if (lane < kMaxEntry) {
-    uint32_t pos = lane;
-    code = 0;
-    // Bounded: every step advances by at least 3 slots.
-    for (int it = 0; it < kChunkSlots; it++) {
-      if (pos >= g.nvalid) { code = g.last ? 0 : (uint8_t)(pos - g.nvalid); break; }
-      const uint32_t sc = s_code[w][pos];
+  // One walk from `pos` to the first record start at or past `end`; false when it ends inside the chunk.  Bounded:
+  // every step advances by at least 3 slots.
+  auto walk = [&](const uint8_t* codes, uint32_t nvalid, bool last, uint32_t end, uint32_t& pos) -> bool {
+    for (int it = 0; it < kChunkSlots && pos < end; it++) {
+      const uint32_t sc = codes[pos];
       const uint32_t n = sc & 31u;
-      if (n == 0 || (g.last && pos + n > g.nvalid)) { code = kExitTerminate; c2 += 1u << (8 * (C_UNEXPECTED - 8)); break; }
+      if (n == 0 || (last && pos + n > nvalid)) { c2 += 1u << (8 * (C_UNEXPECTED - 8)); return false; }
       const uint32_t* inc = s_inc[sc];
       c0 += inc[0]; c1 += inc[1]; c2 += inc[2];
       pos += n;
     }
+    return true;
+  };
+  uint32_t pos = lane, mine = 0xFFFFFFFFu;  // this lane's entry of s_rest
+  bool on = false;                          // the walk goes on behind kMergeSlots
+  if (lane < kMaxEntry) {
+    if (!walk(s_code[w], g.nvalid, g.last, min(kMergeSlots, g.nvalid), pos)) code = kExitTerminate;
+    else if (pos >= g.nvalid) code = g.last ? 0 : (uint8_t)(pos - g.nvalid);
+    else on = true;
+  }
+  const uint32_t peers = __match_any_sync(0xffffffffu, on ? pos : 0x80000000u), leader = (uint32_t)__ffs((int)peers) - 1u;
+  const uint32_t leads = __ballot_sync(0xffffffffu, on && leader == lane);
+  uint32_t base = 0;
+  if (lane == 0) {
+    if (leads) base = atomicAdd(&s_n_lead, (uint32_t)__popc(leads));
+    s_nvalid[w] = (uint16_t)g.nvalid; s_last[w] = g.last;
+  }
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (on) {
+    mine = base + (uint32_t)__popc(leads & ((1u << leader) - 1u));
+    if (leader == lane) s_lead[mine] = (w << 16) | pos;
+  }
+  __syncthreads();
+  const uint32_t p0 = c0, p1 = c1, p2 = c2;
+  if (threadIdx.x < s_n_lead) {  // at most one per thread
+    const uint32_t lw = s_lead[threadIdx.x] >> 16, nvalid = s_nvalid[lw];
+    uint32_t at = s_lead[threadIdx.x] & 0xFFFFu;
+    const bool last = s_last[lw];
+    c0 = 0; c1 = 0; c2 = 0;
+    const bool out = walk(s_code[lw], nvalid, last, nvalid, at);
+    uint32_t* r = s_rest[threadIdx.x];
+    r[0] = out ? (last ? 0u : at - nvalid) : (uint32_t)kExitTerminate;
+    r[1] = c0; r[2] = c1; r[3] = c2;
+  }
+  __syncthreads();
+  if (!live) return;
+  c0 = p0; c1 = p1; c2 = p2;
+  if (mine != 0xFFFFFFFFu) {
+    const uint32_t* r = s_rest[mine];
+    code = (uint8_t)r[0]; c0 += r[1]; c1 += r[2]; c2 += r[3];
   }
   d.exit_map[(uint64_t)chunk * 32 + lane] = code;
   uint32_t* cw = d.walk_cnt + ((uint64_t)chunk * 32 + lane) * 3;
@@ -523,37 +571,49 @@ __device__ __forceinline__ uint32_t load_codes(const Dev& d, const ChunkGeom& g,
   return off;
 }
 
-// One warp per chunk.  Lane 0 walks the chunk from its true entry and notes where records start; the
-// warp then ranks the records within their class (32 at a time, by ballot) and writes the per-class
-// work lists and the compacted EXTERNAL_CORRELATION records.
+// One warp per chunk; the block's first warp walks the chunks of the whole block from their true entries, a chunk to
+// a lane, and notes where records start; every warp then ranks the records of its chunk within their class (32 at a
+// time, by ballot) and writes the per-class work lists and the compacted EXTERNAL_CORRELATION records.  With a walking
+// lane in every warp that walk was most of the kernel's instructions (10.8 lanes active on average): segmentation
+// stage, 11.5 M mixed records 557 -> 529 us, with k_seg_chunks' shared walks 506; 1 M launches 256 -> 248 and 243.
+// (32 chunks to a block, four a warp, together with a byte-wise decode in k_seg_chunks: 292 on 1 M launches.)
+constexpr int kPosStride = kChunkSlots / 3 + 4;  // positions of a chunk's records; an odd number of 32-bit words
+static_assert(kPosStride % 4 == 2, "lanes at the same place in different chunks meet in different banks");
 __global__ void __launch_bounds__(kSegWarps * 32) k_seg_write(Dev d) {
   __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots + 4];
-  __shared__ uint16_t s_pos[kSegWarps][kChunkSlots / 3 + 2];
-  __shared__ uint32_t s_n[kSegWarps];
+  __shared__ uint16_t s_pos[kSegWarps][kPosStride];
+  __shared__ uint32_t s_n[kSegWarps], s_walk[kSegWarps];  // s_walk: where a chunk's walk begins (entry, code offset), its slots, "last chunk"
   __shared__ uint64_t s_base[kSegWarps][C_NCLASS];
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunk = blockIdx.x * kSegWarps + w;
-  if (chunk >= d.n_chunks) return;
-  const uint32_t entry = d.chunk_entry[chunk];
-  if (entry == kEntryNone) return;
-  const ChunkGeom g = chunk_geom(d, chunk);
-  const uint8_t* codes = s_code[w] + load_codes(d, g, s_code[w], lane);
-  if (lane == 0) {
-    uint32_t n = 0, pos = entry;
-    for (int it = 0; it < kChunkSlots && pos < g.nvalid; it++) {  // bounded: every step advances by at least 3 slots
-      const uint32_t len = codes[pos] & 31u;
-      if (len == 0 || (g.last && pos + len > g.nvalid)) break;    // unknown kind or overrun: the walk ends
-      s_pos[w][n++] = (uint16_t)pos;
-      pos += len;
-    }
-    s_n[w] = n;
+  const uint32_t entry = chunk < d.n_chunks ? (uint32_t)d.chunk_entry[chunk] : (uint32_t)kEntryNone;
+  ChunkGeom g{0, 0, false};
+  uint32_t off = 0;
+  if (entry != kEntryNone) { g = chunk_geom(d, chunk); off = load_codes(d, g, s_code[w], lane); }
+  if (lane == 0) s_walk[w] = entry | (off << 8) | (g.last ? 1u << 10 : 0u) | (g.nvalid << 16);
+  // next free position of every class (work list, or the compacted EXTERNAL_CORRELATION array): on its way during the walk
+  if (lane < (uint32_t)C_NCLASS && entry != kEntryNone)
+    s_base[w][lane] = d.chunk_base[(uint64_t)lane * d.n_chunks + chunk] + (lane == (uint32_t)C_EXT ? 0 : d.cls_begin[lane]);
+  const uint64_t ev_first = entry != kEntryNone ? d.chunk_base[(uint64_t)C_EVENTS * d.n_chunks + chunk] : 0;
+  __syncthreads();
+  if (threadIdx.x < (uint32_t)kSegWarps) {
+    const uint32_t q = threadIdx.x, x = s_walk[q], nvalid = x >> 16;
+    const uint8_t* codes = s_code[q] + ((x >> 8) & 3u);
+    const bool last = (x >> 10) & 1u;
+    uint32_t n = 0, pos = x & 0xffu;
+    if (pos != kEntryNone)
+      for (int it = 0; it < kChunkSlots && pos < nvalid; it++) {  // bounded: every step advances by at least 3 slots
+        const uint32_t len = codes[pos] & 31u;
+        if (len == 0 || (last && pos + len > nvalid)) break;      // unknown kind or overrun: the walk ends
+        s_pos[q][n++] = (uint16_t)pos;
+        pos += len;
+      }
+    s_n[q] = n;
   }
-  __syncwarp();
+  __syncthreads();
+  const uint8_t* codes = s_code[w] + off;
   const uint32_t n = s_n[w];
-  // next free position of every class (work list, or the compacted EXTERNAL_CORRELATION array)
-  if (lane < (uint32_t)C_NCLASS) s_base[w][lane] = d.chunk_base[(uint64_t)lane * d.n_chunks + chunk] + (lane == (uint32_t)C_EXT ? 0 : d.cls_begin[lane]);
-  __syncwarp();
-  uint64_t ev_base = d.n_ops + d.chunk_base[(uint64_t)C_EVENTS * d.n_chunks + chunk];
+  uint64_t ev_base = d.n_ops + ev_first;
   const uint32_t lt = (1u << lane) - 1u;
   for (uint32_t i0 = 0; i0 < n; i0 += 32) {
     const uint32_t i = i0 + lane;
