@@ -195,7 +195,7 @@ k2j_status run_clear(k2j_ctx* c, const ClearList& l) {
 
 // Workspaces of the radix sort for n pairs.
 k2j_status sort_reserve(k2j_ctx* c, uint64_t n) {
-  const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
+  const uint32_t tiles = sort_tiles(n);
   for (int i = 0; i < 2; i++) {
     K2J_CUDA(c, c->sort_keys[i].reserve(n * 8));
     K2J_CUDA(c, c->sort_vals[i].reserve(n * 4));
@@ -208,15 +208,15 @@ k2j_status sort_reserve(k2j_ctx* c, uint64_t n) {
 // the buffers that hold the result.
 k2j_status sort_passes(k2j_ctx* c, uint64_t n, int passes, int* cur_io) {
   cudaStream_t s = c->stream;
-  const uint32_t tiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
+  const uint32_t tiles = sort_tiles(n);
   int cur = *cur_io;
   for (int pass = 0; pass < passes; pass++) {
-    k_rs_hist<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), n, 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
+    k_rs_hist<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), n, sort_rounds(n), 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
     c->launches++;
     k2j_status st = run_scan(c, c->sort_hist.as<uint32_t>(), (uint64_t)tiles * 256, 1, c->sort_base.as<uint64_t>(),
                              c->scan_totals.as<uint64_t>() + 23, &c->launches);
     if (st) return st;
-    k_rs_scatter<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, 8 * pass,
+    k_rs_scatter<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, sort_rounds(n), 8 * pass,
                                                 c->sort_base.as<uint64_t>(), tiles, c->sort_keys[cur ^ 1].as<uint64_t>(),
                                                 c->sort_vals[cur ^ 1].as<uint32_t>());
     c->launches++;

@@ -9,17 +9,27 @@
 namespace k2j {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortRounds = 8;
-constexpr int kSortTile = kSortThreads * kSortRounds;  // keys per block
+// Rounds of kSortThreads keys a block (a tile) takes.  The scatter's rounds are a serial chain of barriers, so a sort too
+// short to fill the chip with tiles of eight rounds takes fewer, up to one tile for every block that can be resident
+// (148 SMs x 8): 500 k keys fill 245 blocks at eight rounds and 977 at two.  Size pass and sort of 500 k events: 263 -> 252 us.
+constexpr uint64_t kSortResident = 148 * 8;
+constexpr uint32_t kSortMaxRounds = 8;
+inline uint32_t sort_rounds(uint64_t n) {
+  const uint64_t r = (n + kSortResident * kSortThreads - 1) / (kSortResident * kSortThreads);
+  return r < 1 ? 1u : r > kSortMaxRounds ? kSortMaxRounds : (uint32_t)r;
+}
+inline uint32_t sort_tiles(uint64_t n) {
+  const uint64_t tile = (uint64_t)sort_rounds(n) * kSortThreads;
+  return (uint32_t)((n + tile - 1) / tile);
+}
 
 // hist[digit * n_tiles + tile] = number of keys of the tile with that digit
-__global__ void __launch_bounds__(kSortThreads) k_rs_hist(const uint64_t* keys, uint64_t n, int shift, uint32_t* hist, uint32_t n_tiles) {
+__global__ void __launch_bounds__(kSortThreads) k_rs_hist(const uint64_t* keys, uint64_t n, uint32_t rounds, int shift, uint32_t* hist, uint32_t n_tiles) {
   __shared__ uint32_t s_h[256];
   s_h[threadIdx.x] = 0;
   __syncthreads();
-  const uint64_t base = (uint64_t)blockIdx.x * kSortTile;
-#pragma unroll
-  for (int r = 0; r < kSortRounds; r++) {
+  const uint64_t base = (uint64_t)blockIdx.x * rounds * kSortThreads;
+  for (uint32_t r = 0; r < rounds; r++) {
     const uint64_t i = base + (uint64_t)r * kSortThreads + threadIdx.x;
     if (i < n) atomicAdd(&s_h[(uint32_t)(keys[i] >> shift) & 255u], 1u);
   }
@@ -28,15 +38,15 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_hist(const uint64_t* keys, 
 }
 
 // base[digit * n_tiles + tile] = global position of the tile's first key with that digit
-__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const uint64_t* keys, const uint32_t* vals, uint64_t n, int shift,
+__global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const uint64_t* keys, const uint32_t* vals, uint64_t n, uint32_t rounds, int shift,
                                                              const uint64_t* base, uint32_t n_tiles, uint64_t* keys_out,
                                                              uint32_t* vals_out) {
   __shared__ uint32_t s_cnt[kSortThreads / 32][256];  // per warp and digit: count, then offset within the round
   __shared__ uint32_t s_run[256];                      // keys of each digit placed by earlier rounds
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   s_run[threadIdx.x] = 0;
-  const uint64_t tile0 = (uint64_t)blockIdx.x * kSortTile;
-  for (int r = 0; r < kSortRounds; r++) {
+  const uint64_t tile0 = (uint64_t)blockIdx.x * rounds * kSortThreads;
+  for (uint32_t r = 0; r < rounds; r++) {
     for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
     const uint64_t i = tile0 + (uint64_t)r * kSortThreads + threadIdx.x;

@@ -3,8 +3,10 @@ CPU restatement)."""
 import numpy as np
 import pytest
 
+import cases
 import helpers
 from kineto_b200 import synth
+from kineto_b200 import tracefile as tf
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +45,13 @@ def test_device_rows_that_change_between_calls_of_one_context():
         ctx.run()
         assert ctx.copy_output().tobytes() == want[id(t)]
     ctx.close()
+
+
+# a tile of the sort is one round of 256 keys up to 148 * 8 of them (303 104 keys, two a launch), two rounds above
+@pytest.mark.parametrize("n", [151_552, 151_553])
+def test_sorted_trace_at_the_edge_of_the_sort_s_tiles(n):
+    from kineto_b200 import api
+    trace = cases.with_flags(synth.gen_kernel_launches(n, seed=43, pool_size=50), tf.FLAG_SORT_BY_START)
+    got, res = api.process(trace, device=0)
+    want, _ = helpers.run_port(trace)
+    assert got == want, helpers.first_diff(want, got)
