@@ -82,7 +82,7 @@ struct k2j_ctx {
   DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, out, counters;
   uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 23 sort, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans
   Counters* h_counters = nullptr; // pinned
-  SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans: allocated by the first run with user-annotation spans
+  SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans, behind h_totals in one allocation (one of its own cost the first run with spans 10 ms)
   void* h_stage[2] = {nullptr, nullptr};            // pinned staging buffers of k2j_write_output
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   cudaEvent_t ev[8]{};
@@ -353,7 +353,7 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return K2J_ERR_CUDA; }
     c->own_stream = true;
   }
-  bool ok = cudaMallocHost((void**)&c->h_totals, 32 * sizeof(uint64_t)) == cudaSuccess &&
+  bool ok = cudaMallocHost((void**)&c->h_totals, 32 * sizeof(uint64_t) + kPinnedSpans * sizeof(SpanRec)) == cudaSuccess &&
             cudaMallocHost((void**)&c->h_counters, sizeof(Counters)) == cudaSuccess &&
             c->counters.reserve(sizeof(Counters)) == cudaSuccess && c->scan_totals.reserve(32 * 8) == cudaSuccess;
   for (auto& e : c->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
@@ -361,6 +361,7 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
   ok = ok && cudaFuncSetAttribute(k_events<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)events_smem_bytes(true)) == cudaSuccess &&
        cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)events_smem_bytes(true)) == cudaSuccess;
   if (!ok) { k2j_destroy(c); return K2J_ERR_CUDA; }
+  c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
   *out = c;
   return K2J_OK;
 }
@@ -384,7 +385,6 @@ void k2j_destroy(k2j_ctx* c) {
     b->release();
   if (c->h_totals) cudaFreeHost(c->h_totals);
   if (c->h_counters) cudaFreeHost(c->h_counters);
-  if (c->h_spans) cudaFreeHost(c->h_spans);
   for (int i = 0; i < 2; i++) {
     if (c->h_stage[i]) cudaFreeHost(c->h_stage[i]);
     if (c->stage_ev[i]) cudaEventDestroy(c->stage_ev[i]);
@@ -1032,7 +1032,6 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     K2J_CUDA(c, c->span_row.reserve((size_t)span_cap * 4));
     K2J_CUDA(c, c->span_out.reserve((size_t)span_cap * sizeof(SpanRec)));
     K2J_CUDA(c, c->span_cnt.reserve(16));
-    if (!c->h_spans) K2J_CUDA(c, cudaMallocHost((void**)&c->h_spans, kPinnedSpans * sizeof(SpanRec)));
     clear_later(c->span_cnt.p, 8);
     d.ds_tab = c->ds_tab.as<unsigned long long>(); d.ds_mask = ds_cap - 1;
     d.span_key = c->span_key.as<unsigned long long>(); d.span_nstart = c->span_nstart.as<unsigned long long>();
