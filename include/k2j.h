@@ -293,7 +293,8 @@ k2j_status k2j_set_guest_ops(k2j_ctx* ctx, uint64_t n_guest_ops);
  * first_event ordered by (shard, event number) - names for each span the row of its op among the LAST shard's
  * CPU-side activities (its own or guest rows, k2j_set_guest_ops; 0xFFFFFFFF: no name), and hands the list to
  * k2j_append_spans on the last shard's context, which appends their events, in the reference's order
- * (libkineto/src/GenericActivityProfiler.h:341-346), to the text k2j_emit left there. */
+ * (libkineto/src/GenericActivityProfiler.h:341-346), to the text k2j_emit left there.  Of several entries with one
+ * device, stream and op_id only the one with the smallest first_event is written. */
 typedef struct {
   int64_t start_ns, end_ns;
   uint64_t first_event;

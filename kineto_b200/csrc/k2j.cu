@@ -294,31 +294,36 @@ k2j_status take_spans(k2j_ctx* c, std::vector<SpanRec>* spans) {
 k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint32_t* n_out, uint64_t* bytes_out) {
   cudaStream_t s = c->stream;
   Dev& d = c->d;
-  const unsigned int n = (unsigned int)spans.size();
-  *n_out = n; *bytes_out = 0;
-  if (n == 0) return K2J_OK;
-  K2J_CUDA(c, c->span_out.reserve((size_t)n * sizeof(SpanRec)));
+  const unsigned int listed = (unsigned int)spans.size();
+  *n_out = 0; *bytes_out = 0;
+  if (listed == 0) return K2J_OK;
+  K2J_CUDA(c, c->span_out.reserve((size_t)listed * sizeof(SpanRec)));
   // by (device, stream), inside one by first use; the order of one (device, stream)'s spans is then the iteration order
   // of a hash map filled in that order (a map of one element needs none).  The maps' nodes come from one buffer: a
   // trace of 10 annotations over 256 streams holds 2 560 of them.
-  std::vector<const SpanRec*> by_use(n);
-  for (unsigned int i = 0; i < n; i++) by_use[i] = &spans[i];
+  std::vector<const SpanRec*> by_use(listed);
+  for (unsigned int i = 0; i < listed; i++) by_use[i] = &spans[i];
   std::sort(by_use.begin(), by_use.end(), [](const SpanRec* a, const SpanRec* b) {
-    return a->device != b->device ? a->device < b->device : a->stream != b->stream ? a->stream < b->stream : a->first_event < b->first_event;
+    if (a->device != b->device) return a->device < b->device;
+    if (a->stream != b->stream) return a->stream < b->stream;
+    return a->first_event != b->first_event ? a->first_event < b->first_event : a < b;
   });
   std::vector<SpanRec> room;
   SpanRec* ordered = c->h_spans;  // (the spans were copied out of it)
-  if (!ordered || n > kPinnedSpans) { room.resize(n); ordered = room.data(); }
+  if (listed > kPinnedSpans) { room.resize(listed); ordered = room.data(); }
   SpanRec* next = ordered;
   std::vector<char> node_space(64 * 1024);
-  for (unsigned int i = 0, e; i < n; i = e) {
-    for (e = i + 1; e < n && by_use[e]->device == by_use[i]->device && by_use[e]->stream == by_use[i]->stream;) e++;
+  for (unsigned int i = 0, e; i < listed; i = e) {
+    for (e = i + 1; e < listed && by_use[e]->device == by_use[i]->device && by_use[e]->stream == by_use[i]->stream;) e++;
     if (e == i + 1) { *next++ = *by_use[i]; continue; }
     std::pmr::monotonic_buffer_resource nodes(node_space.data(), node_space.size());
     std::pmr::unordered_map<int64_t, const SpanRec*> m(&nodes);
     for (unsigned int k = i; k < e; k++) m.insert({(int64_t)by_use[k]->op_id, by_use[k]});
     for (auto& kv : m) *next++ = *kv.second;
   }
+  // a caller's list may name a (device, stream, op) more than once: the map kept the entry used first
+  const unsigned int n = (unsigned int)(next - ordered);
+  *n_out = n;
   K2J_CUDA(c, cudaMemcpyAsync(c->span_out.p, ordered, (size_t)n * sizeof(SpanRec), cudaMemcpyHostToDevice, s));
   K2J_CUDA(c, c->ann_size.reserve((size_t)n * 4));
   K2J_CUDA(c, c->ann_off.reserve((size_t)n * 8));

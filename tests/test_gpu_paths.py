@@ -55,3 +55,32 @@ def test_sorted_trace_at_the_edge_of_the_sort_s_tiles(n):
     got, res = api.process(trace, device=0)
     want, _ = helpers.run_port(trace)
     assert got == want, helpers.first_diff(want, got)
+
+
+# up to 4096 spans are ordered in pinned memory that earlier runs have filled, more of them in a list of their own
+@pytest.mark.parametrize("n", [3, 4095, 4096, 5000])
+def test_appended_spans_that_name_an_annotation_twice(n):
+    """Parts of two shards handed over without merging: of the entries of one (device, stream, op) the one used first is
+    written, once, and nothing that an earlier run left behind."""
+    from kineto_b200 import api
+    trace = cases.annotation_trace()
+    once = np.zeros(n - 1, api.SPAN)
+    once["start_ns"] = int(trace.params["window_start_ns"][0]) + 10 * np.arange(n - 1)
+    once["end_ns"] = once["start_ns"] + 7
+    once["first_event"] = np.arange(n - 1)
+    once["device"], once["stream"], once["op_id"] = 1, np.arange(n - 1) // 2, np.arange(n - 1) % 2
+    again = once[:1].copy()
+    again["first_event"], again["start_ns"] = n, again["start_ns"] + 3
+    texts = []
+    for spans in (once, np.concatenate([once, again]), np.concatenate([again, once])):
+        ctx = api.K2J(0)
+        ctx.load(trace)
+        before = ctx.run()["out_bytes"]
+        assert ctx.result["annotation_bytes"] > 0
+        added = ctx.append_spans(spans)
+        text = ctx.copy_output().tobytes()
+        ctx.close()
+        assert len(text) == before + added
+        texts.append(text[before:])
+    assert texts[0].count(b'"ph": "X"') == n - 1
+    assert texts[1] == texts[0] and texts[2] == texts[0]
