@@ -956,6 +956,7 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   K2J_CUDA(c, cudaSetDevice(c->device));
   memset(res, 0, sizeof *res);
   c->ran = false; c->streamed = false;
+  c->partial_spans.clear();
   cudaStream_t s = c->stream;
   Dev& d = c->d;
   const uint64_t* totals = c->totals;
@@ -1183,7 +1184,6 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     K2J_CUDA(c, cudaEventRecord(c->ev[4], s));
     K2J_CUDA(c, cudaStreamSynchronize(s));
     total_bytes = c->h_totals[20];
-    c->partial_spans.clear();
     if (spans_on && c->have_global_join) {
       // several shards: this shard's part of every span waits for the caller to merge it with the other shards' parts
       // (k2j_partial_spans, k2j_append_spans); nothing is written here

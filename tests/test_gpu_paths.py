@@ -84,3 +84,24 @@ def test_appended_spans_that_name_an_annotation_twice(n):
         texts.append(text[before:])
     assert texts[0].count(b'"ph": "X"') == n - 1
     assert texts[1] == texts[0] and texts[2] == texts[0]
+
+
+def test_a_shard_without_events_has_no_parts_of_spans():
+    """The parts of an earlier run of the same context are not reported for a shard that holds nothing to write."""
+    import torch
+    from kineto_b200 import api
+    full = cases.annotation_trace()
+    b = synth.TraceBuilder(n_devices=2, flags=tf.FLAG_USER_ANNOTATIONS)
+    b.extcorr(1, 20, ext_kind=tf.EXTERNAL_KIND_CUSTOM1)   # a record that no event comes from
+    ctx = api.K2J(0)
+    for trace in (full, b.build()):
+        ctx.load(trace)
+        info = ctx.segment()
+        ext = api.device_view(info.external_records, int(info.n_external) * 2, "<i8").clone()
+        ops = torch.from_numpy(trace.op_id.astype(np.int32)).to("cuda:0")
+        torch.cuda.synchronize()
+        ctx.set_global_join(ext, int(info.n_external), 0, ops, trace.n_ops)
+        out = ctx.emit()["out_bytes"]
+        parts = ctx.partial_spans()
+        assert (len(parts) > 0) == (out > 0) == (trace is full)
+    ctx.close()
