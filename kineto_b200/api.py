@@ -143,6 +143,24 @@ def activity_type_mask(mode: int, flags: int) -> int:
     return m if flags & 1 else m & ~(1 << 2)
 
 
+def device_rows(rows, n: int) -> np.ndarray:
+    """The first `n` of a trace's device rows in the layout of k2j_device_props."""
+    props = np.zeros(max(n, 1), DEVICE_PROPS)
+    if n <= 0:
+        return props
+    if n > len(rows):
+        raise IndexError("fewer device rows than n_devices")
+    if isinstance(rows, np.ndarray) and rows.dtype.names and all(rows.dtype[name].kind in "iu" for name in DEVICE_PROPS.names):
+        for name in DEVICE_PROPS.names:  # column by column: field by field costs 40 us for eight devices
+            props[name] = rows[name][:n]
+        return props
+    filled = (DeviceProps * n).from_buffer(props)
+    for i in range(n):  # any other sequence of rows with these fields: a list of dicts, columns of other types
+        for name in DEVICE_PROPS.names:
+            setattr(filled[i], name, int(rows[i][name]))
+    return props
+
+
 def _ptr(a):
     """Address of a numpy array or a torch tensor (host or device)."""
     if a is None:
@@ -190,12 +208,7 @@ class K2J:
                     int(p["ts_mode"]), int(p["flags"]) | (12 if int(p["mode"]) == 1 else 0), int(p["n_devices"]), int(p["conv_t0"]),
                     int(p["conv_t0_approx"]), int(p["conv_scale_mant"]), int(p["conv_scale_exp"]),
                     activity_type_mask(int(p["mode"]), int(p["flags"])))
-        n = int(p["n_devices"])
-        if n > len(trace.devprops):
-            raise IndexError("fewer device rows than n_devices")
-        props = np.zeros(max(n, 1), DEVICE_PROPS)  # column by column: field by field cost 40 us for eight devices
-        for name in DEVICE_PROPS.names if n > 0 else ():
-            props[name][:n] = trace.devprops[name][:n]
+        props = device_rows(trace.devprops, int(p["n_devices"]))
         self._check(self.lib.k2j_set_params(self.h, C.byref(cp), props.ctypes.data_as(C.POINTER(DeviceProps))))
 
     def set_arrays(self, a: dict, buftab: np.ndarray, tidmap: np.ndarray):

@@ -261,3 +261,31 @@ def test_intern_kernel_names_round_trip_gives_the_generated_buffers():
     assert np.array_equal(raw, trace.cupti)
     off, data = names.pool()
     assert np.array_equal(off, trace.pool_off) and np.array_equal(data, trace.pool_data)
+
+
+def _as_columns(rows, kind):
+    from kineto_b200 import api
+    names = api.DEVICE_PROPS.names
+    wide = np.zeros(len(rows), [(name, kind) for name in names])
+    for name in names:
+        wide[name] = rows[name]
+    return wide
+
+
+@pytest.mark.parametrize("form", [lambda r: r, list, lambda r: [{k: x[k] for k in r.dtype.names} for x in r], lambda r: r[::-1].copy()[::-1],
+                                  lambda r: _as_columns(r, np.int64), lambda r: _as_columns(r, object), lambda r: _as_columns(r, np.float64)],
+                         ids=["array", "rows", "dicts", "strided", "int64", "object", "float64"])
+def test_device_rows_in_every_form(form):
+    """A trace's device rows may be any sequence of rows with the fields of k2j_device_props, longer than n_devices too."""
+    from kineto_b200 import api
+    rows = tf.b200_device_props(3)
+    rows["num_sms"] = [148, 7, -1]
+    rows["smem_per_sm"][1] = 1 << 40
+    for n in (1, 2, 3):
+        got = api.device_rows(form(rows), n)
+        assert got.dtype.itemsize == ctypes.sizeof(api.DeviceProps) and len(got) == n
+        for name in got.dtype.names:
+            assert got[name].tolist() == rows[name][:n].tolist(), name
+    with pytest.raises(IndexError):
+        api.device_rows(form(rows), 4)
+    assert len(api.device_rows(None, 0)) == 1   # no devices: the rows are not looked at
