@@ -1,7 +1,7 @@
 """Benchmark of the trace post-processing hot path.
 
     python bench.py --gpus N --steps K --warmup W [--workload W --size N]   # this library (CUDA, sm_100a)
-    python bench.py --impl reference --gpus N --steps K ...               # the reference's CPU path on host cores
+    python bench.py --impl reference --gpus N --steps K ...               # the reference's CPU path on host cores, where its driver is built
 
 Workloads (seeded synthetic traces that stand in for real captures; `--size` is the generator's size argument
 per GPU):
@@ -53,6 +53,7 @@ FALLBACK_HBM_GBS = 6650.0
 # launch it timed; workloads without a capture report null.
 EMIT_TRAFFIC_PER_OUT_BYTE = {"mixed": 2254.8 / 1510.1, "kernel_launches": 2637.2 / 1858.1}
 SLAB_BYTES = 256 << 20
+REF_DRIVER = os.path.join(ROOT, "oracle", "_ref", "ref_driver")
 
 DEFAULT_N = {"mixed": 10_000_000, "kernel_launches": 1_000_000, "op_tree": 2_000_000, "distributed_rank": 2_000_000,
              "memory_events": 1_000_000, "generic": 2_000_000}
@@ -178,9 +179,9 @@ def activities_span(doc: bytes) -> bytes:
 # the reference's own CPU code (oracle/_ref/ref_driver), or our CPU restatement where it is absent
 # ------------------------------------------------------------------------------------------------
 def run_reference_once(trace, procs, keep_output=False):
-    """`procs` concurrent single-threaded reference processes, each over its own copy of `trace`.  Returns
-    (aggregate records/s, seconds, records per process, kind, sha256 of the activities text or None)."""
-    ref = os.path.join(ROOT, "oracle", "_ref", "ref_driver")
+    """`procs` concurrent single-threaded reference processes, each over its own copy of `trace`; without the reference's
+    driver one run of the CPU restatement.  Returns (seconds, kind, processes, (sha256, length) of the activities text or None)."""
+    ref = REF_DRIVER
     with tempfile.TemporaryDirectory(dir="/dev/shm" if os.path.isdir("/dev/shm") else None) as d:
         path = os.path.join(d, "sample.k2jt")
         trace.write(path)
@@ -225,17 +226,19 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    if not os.path.exists(REF_DRIVER):  # this arm is the reference's own code or nothing: the CPU restatement is not the reference
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/ref_driver is not built (make -C oracle ref, from the reference's sources)"}))
+        return
     cores = os.cpu_count() or 1
     procs = max(1, min(cores, 32))
     sample_n = min(args.n, max(1000, args.cpu_sample))   # per process: the size the cpu_baseline sample has
     trace = generate(args.workload, sample_n)
     n_rec = cupti_record_count(trace) + len(trace.op_start)
     vals, secs_all = [], []
-    kind = "reference"
     for i in range(args.warmup + args.steps):
-        secs, kind, used, _ = run_reference_once(trace, procs)
+        secs, kind, _, _ = run_reference_once(trace, procs)
         if i >= args.warmup:
-            vals.append(n_rec * used / secs)
+            vals.append(n_rec * procs / secs)
             secs_all.append(secs)
     value = statistics.mean(vals)
     cfg = config(args, args.gpus, args.n)
@@ -247,7 +250,7 @@ def run_reference(args):
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * statistics.mean(secs_all),
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u8", "data": "synthetic",
             "config": cfg,
-            "cpu_baseline": {"value": value, "unit": UNIT, "cores": procs if kind == "reference" else 1, "kind": kind,
+            "cpu_baseline": {"value": value, "unit": UNIT, "cores": procs, "kind": kind,
                              "sample": cfg["reference_sample"]},
             "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     print(json.dumps(line))
@@ -527,9 +530,11 @@ def cpu_baseline_and_parity(args, api, device):
     text, r = api.process(sample, device=device)
     n_rec = r["n_records"] + len(sample.op_start)
     out = {"cpu_baseline": {"value": n_rec / secs, "unit": UNIT, "cores": 1, "kind": kind,
-                            "sample": "%s trace of size argument %d (%d records, %d bytes of text), one single-threaded process "
-                                      "(the reference path is single-threaded), %.1f s, output on tmpfs"
-                                      % (args.workload, sample_n, n_rec, len(text), secs)}}
+                            "sample": "%s trace of size argument %d (%d records, %d bytes of text), one single-threaded process of "
+                                      "%s, %.1f s"
+                                      % (args.workload, sample_n, n_rec, len(text),
+                                         "the reference (its path is single-threaded), output on tmpfs" if kind == "reference"
+                                         else "this repository's CPU restatement of the reference, output in memory", secs)}}
     out["cpu_baseline"]["save_e2e"] = save_through_the_reference(args)
     if digest is not None:
         out["parity"] = {"sha256_match": digest[0] == hashlib.sha256(text).hexdigest(), "bytes": len(text),

@@ -289,3 +289,16 @@ def test_device_rows_in_every_form(form):
     with pytest.raises(IndexError):
         api.device_rows(form(rows), 4)
     assert len(api.device_rows(None, 0)) == 1   # no devices: the rows are not looked at
+
+
+def test_the_reference_arm_runs_the_reference_or_nothing():
+    """bench.py --impl reference without the reference's driver: one line that says so, and no figure of other code."""
+    import json
+    import sys
+    if helpers.have_ref():
+        pytest.skip("the reference's driver is built")
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--size", "1000", "--cpu-sample", "1000",
+                        "--steps", "1", "--warmup", "0"], capture_output=True, text=True, cwd=ROOT)
+    assert r.returncode == 0, r.stderr[-1000:]
+    line = json.loads(r.stdout.strip().splitlines()[-1])
+    assert line["impl"] == "reference" and "ref_driver" in line["unavailable"] and "value" not in line
