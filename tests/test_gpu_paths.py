@@ -105,3 +105,105 @@ def test_a_shard_without_events_has_no_parts_of_spans():
         parts = ctx.partial_spans()
         assert (len(parts) > 0) == (out > 0) == (trace is full)
     ctx.close()
+
+
+def _whole_text(ctx, trace):
+    """The text of a run, left on the GPU."""
+    from kineto_b200 import api
+    ctx.load(trace)
+    ctx.run()
+    ptr, size = ctx.output_ptr()
+    return api.device_view(ptr, size, "|u1")
+
+
+# Sort tiles take one to eight rounds of 256 keys, one more for every 303 104 of them (148 * 8 tiles): the first size of
+# three rounds and of eight, the last one of seven, and sizes at and past the last full eight (more tiles than can be
+# resident from there on), all but two with a partial last tile.
+@pytest.mark.parametrize("n", [606_209, 909_500, 1_400_000, 1_600_001, 2_121_728, 2_121_729, 2_424_832, 2_424_833, 3_000_001])
+def test_sort_order_at_every_number_of_rounds(n):
+    """Events of one length, so that the sorted text is the unsorted one's rows in numpy's stable order of the starts."""
+    import torch
+    from kineto_b200 import api
+    b = synth.TraceBuilder(n_devices=1, flags=0)
+    rec = np.repeat(b.runtime(b.t0, b.t0, 1), n)
+    rng = np.random.default_rng(n)
+    starts = b.t0 + rng.integers(0, 8_000_000, n) * 1000 + rng.integers(0, 2, n)  # seven digits of microseconds; ties
+    rec["start"], rec["end"], rec["correlationId"] = starts, starts + 100, 1_000_000 + np.arange(n)
+    trace = b.build()
+    trace.cupti, trace.buftab = rec.view(np.uint8), tf.make_buftab(np.arange(n + 1) * rec.itemsize)
+    ctx = api.K2J(0)
+    rows = _whole_text(ctx, trace)
+    length = len(rows) // n
+    assert len(rows) == n * length
+    rows = rows.view(n, length).clone()
+    order = torch.from_numpy(np.argsort(starts, kind="stable")).to("cuda:0")
+    got = _whole_text(ctx, cases.with_flags(trace, tf.FLAG_SORT_BY_START))
+    assert torch.equal(got.view(n, length), rows[order])
+    ctx.close()
+
+
+# the scan of the event sizes takes two launches up to 4096 * 2048 events, three above; the smallest takes one
+@pytest.mark.parametrize("n_events", [200, 4096 * 2048, 4096 * 2048 + 1])
+def test_what_the_scan_reports_at_the_edges_of_its_shapes(n_events):
+    """Bytes of CPU-op text, the flag of instant events, kernels with collective metadata and the annotations' spans reach
+    the host with the scan's totals: a trace whose first op recurs is that op's text as often, then the small trace's."""
+    from kineto_b200 import api
+    b = synth.TraceBuilder(n_devices=1)
+    b.op(b.t0 + 10, b.t0 + 20, 7, "recurs")
+    b.op(b.t0 + 10, b.t0 + 900, 8, "record_param_comms", md=[
+        ("Collective name", tf.MD_STRING, "allreduce"), ("In msg nelems", tf.MD_INT64, 64), ("Out msg nelems", tf.MD_INT64, 64),
+        ("Group size", tf.MD_INT64, 8), ("dtype", tf.MD_STRING, "Float")])
+    b.op(b.t0 + 30, b.t0 + 30, 0, "[memory]", type=synth.CPU_INSTANT_EVENT, md=[("Bytes", tf.MD_INT64, 512)])
+    b.op(b.t0 + 5, b.t0 + 990, 9, "step", type=synth.USER_ANNOTATION)
+    for i in range(40):
+        b.extcorr(100 + i, 8)
+        b.extcorr(100 + i, 9, ext_kind=tf.EXTERNAL_KIND_CUSTOM1)
+        b.runtime(b.t0 + 100 + i, b.t0 + 110 + i, 100 + i)
+        b.kernel(b.t0 + 200 + i, b.t0 + 300 + i, 100 + i, "k%d" % i, stream=7 + i % 3)
+    small = b.build()
+    want = helpers.run_port(small)[0]
+    ctx = api.K2J(0)
+    assert _whole_text(ctx, small).cpu().numpy().tobytes() == want and ctx.result["annotation_bytes"] > 0
+    res0 = dict(ctx.result)
+    assert b'"Collective name"' in want[res0["ops_bytes"]:] and b'"ph": "i"' in want
+    more = n_events - (small.n_ops + 80)
+    for col in ("op_start", "op_end", "op_id", "op_device", "op_resource", "op_thread", "op_type", "op_name", "op_flow", "op_flowt", "op_mdoff"):
+        a = getattr(small, col)
+        setattr(small, col, np.concatenate([np.repeat(a[:1], more), a]))
+    got = _whole_text(ctx, small)
+    length = want.index(b"\n  {", 1)
+    front = got[:more * length].view(more, length)
+    assert bool((front == front[0]).all()) and front[0].cpu().numpy().tobytes() == want[:length]
+    assert got[more * length:].cpu().numpy().tobytes() == want
+    assert ctx.result["ops_bytes"] == res0["ops_bytes"] + more * length and ctx.result["annotation_bytes"] == res0["annotation_bytes"]
+    assert ctx.result["x_events"] == res0["x_events"] + more
+    ctx.close()
+
+
+# the scan of the chunks' class counts (13 columns) takes one launch up to 16 384 chunks of 4 KiB, two above
+@pytest.mark.parametrize("n_chunks", [16_384, 16_385])
+def test_class_counts_at_the_edge_of_one_launch(n_chunks):
+    """A small trace's records over and over: its text as often, and then that of the buffers which make up the number."""
+    from kineto_b200 import api
+    t = synth.gen_mixed(200, seed=47, pool_size=50, buffer_bytes=4096)
+    each, size = t.n_buffers, len(t.cupti)
+    times, rest = divmod(n_chunks, each)
+
+    def repeated(k):
+        r = tf.Trace(**{attr: getattr(t, attr) for _, attr, _ in tf._SECTIONS})
+        tab = np.concatenate([t.buftab.reshape(-1, 2) + np.array([i * size, 0], np.uint64) for i in range(k + 1)])
+        r.cupti, r.buftab = np.tile(t.cupti, k + 1), tab[:k * each + rest].reshape(-1)
+        return r
+
+    ctx = api.K2J(0)
+    alone = repeated(1)
+    want = helpers.run_port(alone)[0]
+    assert _whole_text(ctx, alone).cpu().numpy().tobytes() == want
+    n_ops_text = ctx.result["ops_bytes"]
+    first = len(helpers.run_port(t)[0]) - n_ops_text            # text of the records once
+    got = _whole_text(ctx, repeated(times))
+    body = got[n_ops_text:n_ops_text + times * first].view(times, first)
+    assert bool((body == body[0]).all()) and body[0].cpu().numpy().tobytes() == want[n_ops_text:n_ops_text + first]
+    assert got[:n_ops_text].cpu().numpy().tobytes() == want[:n_ops_text]
+    assert got[n_ops_text + times * first:].cpu().numpy().tobytes() == want[n_ops_text + first:]
+    ctx.close()
