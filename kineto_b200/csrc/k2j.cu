@@ -80,9 +80,9 @@ struct k2j_ctx {
   DevBuf ds_tab, span_key, span_nstart, span_end, span_nfirst, span_row, span_out, span_cnt, ann_size, ann_off;
   DevBuf sort_keys[2], sort_vals[2], sort_hist, sort_base, sort_rank;
   DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, out, counters;
-  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 23 sort, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans
+  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans (23 and 27 are words of scan_totals, device memory: sort, filtered join keys)
   Counters* h_counters = nullptr; // pinned
-  SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans, behind h_totals in one allocation (one of its own cost the first run with spans 10 ms)
+  SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans, behind h_totals in one allocation
   void* h_stage[2] = {nullptr, nullptr};            // pinned staging buffers of k2j_write_output
   cudaEvent_t stage_ev[2] = {nullptr, nullptr};
   cudaEvent_t ev[8]{};
@@ -153,9 +153,16 @@ uint32_t pow2_at_least(uint64_t n) {
 }
 
 // Exclusive scan of `cols` columns of n u32 each (column stride n) into u64; totals land in
-// totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length: up to
-// kScanSmallMax elements one block per column is done sooner than a second launch would begin; up to
-// kScanDirectBlocks tiles adding up the sums in front of a block costs it less than the launch that scans them.
+// totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length.  Each line lies
+// where its shape still beats what stood for every length before, three launches and a copy of the total.  One column,
+// us per call of k2j_exclusive_scan_u32 with its wait:
+//   elements                   200   4096   8192   12 288   16 384  |  tiles of 2048   4096   4097   6144   8192   16 384
+//   one launch                  16     19     21       25       27  |
+//   two launches                17     18     18       18       18  |                    66     69     93    121      244
+//   three launches                                                  |                    72     72     99    127      237
+//   three launches and a copy   27     27     27       28       31  |                    82     81
+// Among themselves the first two meet near 4096 elements (a block's serial rounds of 8192 against a launch), the last two
+// between 8192 and 16 384 tiles (sums that every block adds up again against a launch).
 constexpr uint64_t kScanSmallMax = 2 * kScanSmallTile;
 constexpr uint32_t kScanDirectBlocks = 4096;
 k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches,
@@ -183,6 +190,7 @@ k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, u
 
 // One launch that gives every region of the list its initial value.
 k2j_status run_clear(k2j_ctx* c, const ClearList& l) {
+  if (l.n > (uint32_t)kClearMax) return fail(c, K2J_ERR_UNSUPPORTED, "more than %d tables to clear", kClearMax);
   uint64_t words = 0;
   for (uint32_t k = 0; k < l.n; k++) words = std::max(words, l.r[k].words);
   if (words == 0) return K2J_OK;
@@ -969,11 +977,7 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   // every counter belongs to the emit step (segmentation counts through its scan columns): a second k2j_emit after
   // one k2j_segment starts from zero, and an earlier failed check does not fail this run
   ClearList clear;
-  auto clear_later = [&](void* p, uint64_t bytes, bool ones = false) {  // whole 8-byte words
-    clear.ones |= (ones ? 1u : 0u) << clear.n;
-    clear.r[clear.n].p = static_cast<uint64_t*>(p); clear.r[clear.n].words = bytes / 8; clear.n++;
-  };
-  clear_later(d.counters, sizeof(Counters));
+  clear.add(d.counters, sizeof(Counters));
 
   // ---- join tables ----
   uint64_t own_begin = 0, own_end = totals[C_EXT];
@@ -1008,21 +1012,21 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   d.corr_tab = c->corr_tab.as<unsigned long long>(); d.corr_mask = corr_cap - 1;
   d.user_tab = c->user_tab.as<unsigned long long>(); d.user_mask = corr_cap - 1;
   d.op_tab = c->op_tab.as<unsigned long long>(); d.op_mask = op_cap - 1;
-  clear_later(d.corr_tab, (size_t)corr_cap * 8);
+  clear.add(d.corr_tab, (size_t)corr_cap * 8);
   K2J_CUDA(c, c->corr0.reserve(16));
   d.corr0 = c->corr0.as<unsigned long long>();
-  clear_later(d.corr0, 16);
+  clear.add(d.corr0, 16);
   // the user-annotation table is only written and read when CUSTOM1 correlation records exist
   // (several shards: another shard's CUSTOM1 records may name this shard's events, so the local count says nothing,
   // unless the caller has said that no shard holds any)
   const bool user_records = c->have_global_join ? c->join_user_hint != 0 : totals[C_USER] > 0;
-  if (user_records) clear_later(d.user_tab, (size_t)corr_cap * 8);
+  if (user_records) clear.add(d.user_tab, (size_t)corr_cap * 8);
   else d.user_tab = nullptr;
-  clear_later(d.op_tab, (size_t)op_cap * 8);
+  clear.add(d.op_tab, (size_t)op_cap * 8);
   const uint32_t tid_cap = std::max<uint32_t>(16384, pow2_at_least(4ull * c->n_tid));
   K2J_CUDA(c, c->tid_tab.reserve((size_t)tid_cap * 8));
   d.tid_tab = c->tid_tab.as<unsigned long long>(); d.tid_mask = tid_cap - 1;
-  clear_later(d.tid_tab, (size_t)tid_cap * 8);
+  clear.add(d.tid_tab, (size_t)tid_cap * 8);
   // user-annotation span tables (single-shard runs only)
   const bool spans_on = (c->params.flags & K2J_FLAG_USER_ANNOTATIONS) && user_records;
   d.span_key = nullptr;
@@ -1038,16 +1042,16 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     K2J_CUDA(c, c->span_row.reserve((size_t)span_cap * 4));
     K2J_CUDA(c, c->span_out.reserve((size_t)span_cap * sizeof(SpanRec)));
     K2J_CUDA(c, c->span_cnt.reserve(16));
-    clear_later(c->span_cnt.p, 8);
+    clear.add(c->span_cnt.p, 8);
     d.ds_tab = c->ds_tab.as<unsigned long long>(); d.ds_mask = ds_cap - 1;
     d.span_key = c->span_key.as<unsigned long long>(); d.span_nstart = c->span_nstart.as<unsigned long long>();
     d.span_end = c->span_end.as<unsigned long long>(); d.span_nfirst = c->span_nfirst.as<unsigned long long>();
     d.span_row = c->span_row.as<uint32_t>(); d.span_mask = span_cap - 1;
-    clear_later(d.ds_tab, (size_t)ds_cap * 8);
-    clear_later(d.span_key, (size_t)span_cap * 8);
-    clear_later(d.span_nstart, (size_t)span_cap * 8);
-    clear_later(d.span_end, (size_t)span_cap * 8);
-    clear_later(d.span_nfirst, (size_t)span_cap * 8);
+    clear.add(d.ds_tab, (size_t)ds_cap * 8);
+    clear.add(d.span_key, (size_t)span_cap * 8);
+    clear.add(d.span_nstart, (size_t)span_cap * 8);
+    clear.add(d.span_end, (size_t)span_cap * 8);
+    clear.add(d.span_nfirst, (size_t)span_cap * 8);
   }
   d.need_corr = nullptr; d.need_op = nullptr;
   bool mark_corr = false;
@@ -1056,22 +1060,22 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     const uint32_t op_bits = corr_bits;
     K2J_CUDA(c, c->need_op.reserve(op_bits / 8));
     d.need_op = c->need_op.as<uint32_t>(); d.need_op_mask = op_bits - 1;
-    clear_later(d.need_op, op_bits / 8);
+    clear.add(d.need_op, op_bits / 8);
     if (c->need_bits) {  // the filter the caller had filled for the exchange (k2j_join_need_bits): the same marks
       d.need_corr = c->need_bits; d.need_corr_mask = (uint32_t)(c->need_n_bits - 1);
     } else {
       K2J_CUDA(c, c->need_corr.reserve(corr_bits / 8));
       d.need_corr = c->need_corr.as<uint32_t>(); d.need_corr_mask = corr_bits - 1;
-      clear_later(d.need_corr, corr_bits / 8);
+      clear.add(d.need_corr, corr_bits / 8);
       mark_corr = d.ops_begin != 0;
     }
   }
   // collective enrichment: kernels look at their linked op's name only if some op is a record_param_comms call;
   // ops of other shards carry no metadata here, so sharded runs do not enrich
-  d.has_comms = nullptr;
+  d.has_comms = nullptr; d.coll_tab = nullptr;
   if (c->n_ops && c->n_strings) {
     K2J_CUDA(c, c->comms_flag.reserve(16));
-    clear_later(c->comms_flag.p, 8);
+    clear.add(c->comms_flag.p, 8);
     d.has_comms = c->comms_flag.as<uint32_t>();
     if (c->have_global_join) {
       // several shards: the join's table holds positions in the gathered keys, so the record_param_comms ops that carry
@@ -1079,7 +1083,7 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
       const uint32_t coll_cap = pow2_at_least(2 * c->n_ops + 16);
       K2J_CUDA(c, c->coll_tab.reserve((size_t)coll_cap * 8));
       d.coll_tab = c->coll_tab.as<unsigned long long>(); d.coll_mask = coll_cap - 1;
-      clear_later(d.coll_tab, (size_t)coll_cap * 8);
+      clear.add(d.coll_tab, (size_t)coll_cap * 8);
     }
   }
   d.work_indirect = nullptr; d.n_indirect = 0; d.coll_list = nullptr;
@@ -1094,24 +1098,24 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     const uint64_t zero_bytes = (corr_cap / 8 + 15) & ~7ull;  // one bit per table slot, whole words
     K2J_CUDA(c, c->corr_zero.reserve(zero_bytes));
     d.corr_zero = c->corr_zero.as<uint32_t>();
-    clear_later(d.corr_zero, zero_bytes);
+    clear.add(d.corr_zero, zero_bytes);
     const uint32_t ctx_cap = 1u << 14;   // distinct CUDA contexts of one trace: a few per device
     K2J_CUDA(c, c->ctx_tab.reserve((size_t)ctx_cap * 8));
     d.ctx_tab = c->ctx_tab.as<unsigned long long>(); d.ctx_mask = ctx_cap - 1;
-    clear_later(d.ctx_tab, (size_t)ctx_cap * 8);
+    clear.add(d.ctx_tab, (size_t)ctx_cap * 8);
     if (totals[C_WAIT]) {
       const uint32_t seen_cap = 1u << 16;  // (device, stream) pairs
       K2J_CUDA(c, c->seen_tab.reserve((size_t)seen_cap * 8));
       d.seen_tab = c->seen_tab.as<unsigned long long>(); d.seen_mask = seen_cap - 1;
-      clear_later(d.seen_tab, (size_t)seen_cap * 8);
+      clear.add(d.seen_tab, (size_t)seen_cap * 8);
     }
     if (totals[C_SYNC]) {
       const uint32_t row_cap = pow2_at_least(2 * totals[C_SYNC] + 16);
       K2J_CUDA(c, c->row_key.reserve((size_t)row_cap * 8));
       K2J_CUDA(c, c->row_first.reserve((size_t)row_cap * 4));
       d.row_key = c->row_key.as<unsigned long long>(); d.row_first = c->row_first.as<uint32_t>(); d.row_mask = row_cap - 1;
-      clear_later(d.row_key, (size_t)row_cap * 8);
-      clear_later(d.row_first, (size_t)row_cap * 4, true);
+      clear.add(d.row_key, (size_t)row_cap * 8);
+      clear.add(d.row_first, (size_t)row_cap * 4, true);
     }
   }
   k2j_status st_clear = run_clear(c, clear);

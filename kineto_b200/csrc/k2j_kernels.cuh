@@ -376,8 +376,11 @@ __device__ __forceinline__ uint32_t code_class(uint32_t code) {
 // Walks of a chunk meet soon: a walk that starts inside a record reads payload as kinds, ends, or lands on a record and
 // from there on is the walk of that record.  So each lane walks only until it has passed slot kMergeSlots; of the lanes
 // that stand on one slot then, one goes on for all, and the block packs these few of all its chunks into its first
-// warps for the long rest.  The kernel is bound by the issue of its walks' instructions (83 % of the slots when all 26
-// walks of a chunk ran to its end).  Segmentation stage, 11.5 M mixed records: 557 -> 532 us; 1 M launches: 256 -> 249.
+// warps for the long rest.  With all 26 walks of a chunk running to its end the kernel was bound by the issue of their
+// instructions (83 % of the slots).  Segmentation stage, 11.5 M mixed records: 557 -> 532 us; 1 M launches: 256 -> 249.
+// By kMergeSlots (with k_seg_write's shared walk, below): 32 504 and 241, 64 506 and 241, 96 508 and 243, 128 511 and
+// 244, 192 517 and 247, 512 (never) 561 and 260; at 32 long records keep walks apart (120 k nested operators 120-126 us,
+// else 118).
 constexpr uint32_t kMergeSlots = 96;
 __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
   __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots];
@@ -783,10 +786,14 @@ __global__ void __launch_bounds__(kJoinThreads) k_build_join(Dev d, JoinJobs j) 
 }
 
 // ---- initial values of a run's tables, all in one launch ----
-constexpr int kClearThreads = 256, kClearMax = 24;
+constexpr int kClearThreads = 256, kClearMax = 24;  // a run with every table has 21
 struct ClearList {
   struct { uint64_t* p; uint64_t words; } r[kClearMax];  // 16-byte aligned, a count of 8-byte words
   uint32_t n = 0, ones = 0;                              // bit k of ones: region k is set to all ones, not zeros
+  void add(void* p, uint64_t bytes, bool all_ones = false) {  // past kClearMax it only counts: run_clear refuses the list
+    if (n < (uint32_t)kClearMax) { r[n].p = static_cast<uint64_t*>(p); r[n].words = bytes / 8; ones |= (all_ones ? 1u : 0u) << n; }
+    n++;
+  }
 };
 __global__ void __launch_bounds__(kClearThreads) k_clear(const __grid_constant__ ClearList l) {
   const uint64_t first = (uint64_t)blockIdx.x * kClearThreads + threadIdx.x, step = (uint64_t)gridDim.x * kClearThreads;
@@ -899,8 +906,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint64_t* block_sums
   }
   if (threadIdx.x == 0) totals[blockIdx.x] = carry;
 }
-// totals != nullptr: block_sums holds the blocks' sums as k_scan_reduce left them; every block adds up those in front
-// of it (at most kScanDirectBlocks eight-byte reads from the L2), and the last one stores the column total.
+// DIRECT: block_sums holds the blocks' sums as k_scan_reduce left them; every block adds up those in front of it (at
+// most kScanDirectBlocks eight-byte reads from the L2), and the last one stores the column total.  Otherwise k_scan_sums
+// has turned them into the blocks' offsets and stored the totals.
 template <bool DIRECT>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint64_t n, uint64_t col_stride, const uint64_t* block_sums, uint32_t n_blocks,
                                                              uint64_t* out, uint64_t* totals, ScanReport rep) {
