@@ -150,7 +150,8 @@ def device_rows(rows, n: int) -> np.ndarray:
         return props
     if n > len(rows):
         raise IndexError("fewer device rows than n_devices")
-    if isinstance(rows, np.ndarray) and rows.dtype.names and all(rows.dtype[name].kind in "iu" for name in DEVICE_PROPS.names):
+    if isinstance(rows, np.ndarray) and (rows.dtype == tf.DEVICE_PROPS or (
+            rows.dtype.names and all(rows.dtype[name].kind in "iu" for name in DEVICE_PROPS.names))):
         for name in DEVICE_PROPS.names:  # column by column: field by field costs 40 us for eight devices
             props[name] = rows[name][:n]
         return props

@@ -312,9 +312,7 @@ k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint3
   std::vector<const SpanRec*> by_use(listed);
   for (unsigned int i = 0; i < listed; i++) by_use[i] = &spans[i];
   std::sort(by_use.begin(), by_use.end(), [](const SpanRec* a, const SpanRec* b) {
-    if (a->device != b->device) return a->device < b->device;
-    if (a->stream != b->stream) return a->stream < b->stream;
-    return a->first_event != b->first_event ? a->first_event < b->first_event : a < b;
+    return a->device != b->device ? a->device < b->device : a->stream != b->stream ? a->stream < b->stream : a->first_event < b->first_event;
   });
   std::vector<SpanRec> room;
   SpanRec* ordered = c->h_spans;  // (the spans were copied out of it)
