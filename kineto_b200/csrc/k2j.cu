@@ -369,8 +369,8 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
             c->counters.reserve(sizeof(Counters)) == cudaSuccess && c->scan_totals.reserve(32 * 8) == cudaSuccess;
   for (auto& e : c->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
   // the emit kernels' shared memory (record areas + output windows) is above the 48 KiB that needs no opt-in
-  ok = ok && cudaFuncSetAttribute(k_events<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)events_smem_bytes(true)) == cudaSuccess &&
-       cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)events_smem_bytes(true)) == cudaSuccess;
+  ok = ok && cudaFuncSetAttribute(k_events<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess &&
+       cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
   if (!ok) { k2j_destroy(c); return K2J_ERR_CUDA; }
   c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
   *out = c;
@@ -921,6 +921,11 @@ constexpr uint64_t kSlabPad = 64;              // bytes in front of a slab's tex
 
 k2j_status stream_bytes(k2j_ctx* c, const uint8_t* src, int fd, bool positioned, uint64_t file_offset, uint64_t total, cudaStream_t stream);
 
+// Threads of a block of the emit pass: a trace that one wave of the chip holds spreads over all SMs.
+int emit_threads(uint64_t items) {
+  const uint64_t each = (items + 148 * kEmitBlocks - 1) / (148 * kEmitBlocks);
+  return (int)std::min<uint64_t>(kEmitThreads, std::max<uint64_t>(64, (each + 31) & ~31ull));
+}
 // The emit launches for the events whose text starts in [d.tile_begin, d.tile_end).  `ranges`: per class the work
 // items to look at ([begin, end) pairs, C_API .. C_WAIT, then the CPU-side activities); nullptr: everything.
 k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool instant, uint64_t n_coll, cudaStream_t s) {
@@ -928,7 +933,8 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     if (end <= begin) return;
     Dev dr = d;
     dr.work_origin = begin; dr.n_work = end;
-    k_events<true><<<(uint32_t)((end - begin + kEventThreads - 1) / kEventThreads), kEventThreads, events_smem_bytes(true), s>>>(dr);
+    const int threads = emit_threads(end - begin);
+    k_events<true><<<(uint32_t)((end - begin + threads - 1) / threads), threads, emit_smem_bytes(threads), s>>>(dr);
     c->launches++;
   };
   if (!ranges) launch(0, d.n_work);
@@ -939,7 +945,7 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     di.work_origin = ranges ? ranges[2 * C_EXT] : d.ops_begin;
     di.n_work = ranges ? ranges[2 * C_EXT + 1] : d.n_work;
     if (di.n_work > di.work_origin) {
-      k_events<true, true><<<(uint32_t)((di.n_work - di.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, events_smem_bytes(true), s>>>(di);
+      k_events<true, true><<<(uint32_t)((di.n_work - di.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(di);
       c->launches++;
     }
   }
@@ -948,7 +954,7 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     // listed, so that the launch above holds no code for them
     Dev dk = d;
     dk.work_indirect = d.coll_list; dk.n_indirect = n_coll;
-    k_events<true, true><<<(uint32_t)((dk.n_indirect + kEventThreads - 1) / kEventThreads), kEventThreads, events_smem_bytes(true), s>>>(dk);
+    k_events<true, true><<<(uint32_t)((dk.n_indirect + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(dk);
     c->launches++;
   }
   K2J_CUDA(c, cudaGetLastError());
@@ -1160,13 +1166,13 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   uint32_t n_spans = 0;
   if (d.n_work) {
     const uint32_t ev_blocks = (uint32_t)((d.n_work + kEventThreads - 1) / kEventThreads);
-    k_events<false><<<ev_blocks, kEventThreads, events_smem_bytes(false), s>>>(d);
+    k_events<false><<<ev_blocks, kEventThreads, size_smem_bytes(), s>>>(d);
     c->launches++;
     if (totals[C_WAIT]) {  // deferred synchronisation records: sized once every stream with GPU work is known
       Dev dw = d;
       dw.wait_pass = 1; dw.work_origin = d.cls_begin[C_WAIT];
       dw.n_work = d.cls_begin[C_WAIT] + ((totals[C_WAIT] + 31) & ~31ull);
-      k_events<false><<<(uint32_t)((dw.n_work - dw.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, events_smem_bytes(false), s>>>(dw);
+      k_events<false><<<(uint32_t)((dw.n_work - dw.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, size_smem_bytes(), s>>>(dw);
       c->launches++;
     }
     K2J_CUDA(c, cudaGetLastError());

@@ -2160,190 +2160,269 @@ __device__ __forceinline__ void count_fields(S& s, const Dev& d, const uint32_t*
     count_fields<BASE, F + 1, NF>(s, d, a, present, name_bytes);
   }
 }
-// Emit pass, hot record classes: the sink is asked for room once per group of fields whose longest possible text
-// fits the group size, not once per field; the groups are fixed at compile time.
-constexpr uint32_t kGroupBytes = 88;
-static_assert(kGroupBytes + 32 + kWinSlack <= (uint32_t)kWinBytes, "a group must fit a window that has just been flushed");
-// First field of a group?  (Walks the class's fields from its first one, as the field loop does.)
-constexpr bool group_starts_at(int base, int first, int f) {
-  uint32_t acc = 0xffffu;  // the first field always starts a group
-  bool starts = true;
-  for (int g = first; g <= f; g++) {
-    const uint32_t v = value_max_bytes(kAllFields[base + g].type, kAllFields[base + g].vk);
-    const uint32_t need = (uint32_t)c_strlen(kAllFields[base + g].lit) + (v == 0xffffu ? 0u : v);
-    starts = acc == 0xffffu || acc + need > kGroupBytes;
-    if (starts) acc = need; else acc += need;
-    if (v == 0xffffu) acc = 0xffffu;  // after a value of any length the next field asks again
-  }
-  return starts;
-}
-// Bytes the group starting at field f can take (f starts a group).
-constexpr uint32_t group_bytes_from(int base, int f, int nf) {
-  uint32_t acc = 0;
-  for (int g = f; g < nf; g++) {
-    const uint32_t v = value_max_bytes(kAllFields[base + g].type, kAllFields[base + g].vk);
-    const uint32_t need = (uint32_t)c_strlen(kAllFields[base + g].lit) + (v == 0xffffu ? 0u : v);
-    if (g > f && acc + need > kGroupBytes) break;
-    acc += need;
-    if (v == 0xffffu) break;
-  }
-  return acc;
-}
-// Number formatting of the hot classes' field loop: one out-of-line copy of each formatter per kernel, so that a
-// field costs a call instead of a copy of the formatter (with the formatters inlined the kernel is bound by
-// instruction fetch).  The sink travels in registers: window, position and open word in, position
+// Number formatting of the hot classes: one out-of-line copy of each formatter per kernel, so that a field costs a call
+// instead of a copy of the formatter (with the formatters inlined the kernel is bound by instruction fetch).  The sink travels in registers: window, position and open word in, position
 // and open word out; nothing here flushes, the caller has asked for the room.
-__device__ __forceinline__ WindowSink sink_at(uint32_t* win, uint32_t pos, uint32_t carry) {
+__device__ __forceinline__ WindowSink sink_at(Win win, uint32_t pos, uint32_t carry) {
   WindowSink s;
-  s.win = win; s.pos = pos; s.carry = carry; s.w0 = 0; s.head = 0; s.gbase = nullptr;
+  s.win = win; s.pos = pos; s.carry = carry; s.open = 0; s.gbase = nullptr;
   return s;
 }
 __device__ __forceinline__ uint64_t sink_state(const WindowSink& s) { return (uint64_t)s.pos | ((uint64_t)s.carry << 32); }
-__device__ __noinline__ uint64_t app_u64(uint32_t* win, uint32_t pos, uint32_t carry, uint64_t v) {
-  WindowSink s = sink_at(win, pos, carry);
-  put_dec(s, v);
-  return sink_state(s);
+// Three decimal digits per look-up: the zero-padded characters in the low three bytes, most significant first, and eight
+// times the number of leading zeros (of at most two) in the top byte.  The table is in front of the emit kernel's dynamic
+// shared memory.  A number below 1000 costs some 25 instructions with its append, by arithmetic on four digits some 40.
+struct alignas(16) Digits3 { uint32_t w[1024]; };  // 1000 used; copied by 16-byte words
+constexpr Digits3 make_digits3() {
+  Digits3 t{};
+  for (uint32_t v = 0; v < 1000; v++)
+    t.w[v] = (0x30u + v / 100) | ((0x30u + v / 10 % 10) << 8) | ((0x30u + v % 10) << 16) | ((v < 10 ? 16u : v < 100 ? 8u : 0u) << 24);
+  return t;
 }
-__device__ __noinline__ uint64_t app_u32(uint32_t* win, uint32_t pos, uint32_t carry, uint32_t v) {
+__device__ const Digits3 g_digits3 = make_digits3();
+extern __shared__ uint4 s_dyn[];
+__device__ __forceinline__ uint32_t digits3(uint32_t v) { return reinterpret_cast<const uint32_t*>(s_dyn)[v]; }
+__device__ __forceinline__ void put_below_1000(WindowSink& s, uint32_t v) {
+  const uint32_t e = digits3(v), z = e >> 24;
+  s.put((e & 0xffffffu) >> z, (int)(3u - (z >> 3)));
+}
+__device__ __noinline__ uint64_t app_u32(Win win, uint32_t pos, uint32_t carry, uint32_t v) {
   WindowSink s = sink_at(win, pos, carry);
-  if (v < 10000u) {
-    const int n = 1 + (v >= 10u) + (v >= 100u) + (v >= 1000u);
-    s.put(ascii4(v) >> (8 * (4 - n)), n);
-  } else if (v < 100000000u) {
-    const uint32_t hi = v / 10000u, lo = v - hi * 10000u;
-    const int n = 1 + (hi >= 10u) + (hi >= 100u) + (hi >= 1000u);
-    s.put64((uint64_t)(ascii4(hi) >> (8 * (4 - n))) | ((uint64_t)ascii4(lo) << (8 * n)), (uint32_t)(n + 4));
-  } else {  // 9 or 10 digits
-    const uint32_t hi = v / 100000000u, lo = v - hi * 100000000u;
-    const int n = 1 + (hi >= 10u);
-    s.put(ascii4(hi) >> (8 * (4 - n)), n);
-    s.put64(ascii8(lo), 8u);
+  if (v < 1000u) put_below_1000(s, v);
+  else if (v < 1000000u) {
+    const uint32_t hi = v / 1000u, e = digits3(hi), f = digits3(v - hi * 1000u) & 0xffffffu, z = e >> 24, up = 24u - z;
+    s.put64(pack64(((e & 0xffffffu) >> z) | (f << up), __funnelshift_l(f, 0u, up)), 6u - (z >> 3));
+  } else {
+    uint32_t top = v / 1000000u;
+    const uint32_t low = v - top * 1000000u, mid = low / 1000u;
+    if (top >= 1000u) {  // ten digits
+      const uint32_t q = top / 1000u;
+      s.put(0x30u + q, 1);
+      s.put(digits3(top - q * 1000u) & 0xffffffu, 3);
+    } else put_below_1000(s, top);
+    const uint32_t a = digits3(mid) & 0xffffffu, b = digits3(low - mid * 1000u) & 0xffffffu;
+    s.put64(pack64(a | (b << 24), b >> 8), 6u);
   }
   return sink_state(s);
 }
-__device__ __noinline__ uint64_t app_i32(uint32_t* win, uint32_t pos, uint32_t carry, int32_t v) {
+__device__ __noinline__ uint64_t app_u64(Win win, uint32_t pos, uint32_t carry, uint64_t v) {
+  if ((v >> 32) == 0ull) return app_u32(win, pos, carry, (uint32_t)v);
   WindowSink s = sink_at(win, pos, carry);
-  uint32_t mag = (uint32_t)v;
-  if (v < 0) { put_char(s, '-'); mag = 0u - mag; }
-  return app_u32(win, s.pos, s.carry, mag);
-}
-__device__ __noinline__ uint64_t app_i64(uint32_t* win, uint32_t pos, uint32_t carry, int64_t v) {
-  WindowSink s = sink_at(win, pos, carry);
-  put_sdec(s, v);
+  put_u64(s, v);
   return sink_state(s);
 }
-__device__ __noinline__ uint64_t app_ts(uint32_t* win, uint32_t pos, uint32_t carry, uint64_t ns) {
+__device__ __noinline__ uint64_t app_i32(Win win, uint32_t pos, uint32_t carry, int32_t v) {
+  if (v >= 0) return app_u32(win, pos, carry, (uint32_t)v);
   WindowSink s = sink_at(win, pos, carry);
-  put_ts2(s, (int64_t)ns);
+  put_char(s, '-');
+  return app_u32(win, s.pos, s.carry, 0u - (uint32_t)v);
+}
+__device__ __noinline__ uint64_t app_i64(Win win, uint32_t pos, uint32_t carry, int64_t v) {
+  if (v >= 0) return app_u64(win, pos, carry, (uint64_t)v);
+  WindowSink s = sink_at(win, pos, carry);
+  put_char(s, '-');
+  return app_u64(win, s.pos, s.carry, 0ull - (uint64_t)v);
+}
+__device__ __noinline__ uint64_t app_ts(Win win, uint32_t pos, uint32_t carry, uint64_t ns) {
+  const uint64_t us = ns / 1000ull;
+  const uint32_t fr = (uint32_t)ns - (uint32_t)us * 1000u;
+  const uint64_t st = app_u64(win, pos, carry, us);
+  WindowSink s = sink_at(win, (uint32_t)st, (uint32_t)(st >> 32));
+  s.put4(0x2Eu | (digits3(fr) << 8));  // the table's top byte goes
   return sink_state(s);
 }
-__device__ __noinline__ uint64_t app_dbl(uint32_t* win, uint32_t pos, uint32_t carry, uint64_t bits) {
+__device__ __noinline__ uint64_t app_dbl(Win win, uint32_t pos, uint32_t carry, uint64_t bits) {
   WindowSink s = sink_at(win, pos, carry);
   put_dbl(s, __longlong_as_double((long long)bits));
   return sink_state(s);
 }
-// a constant string of the field table (at most longest_constant_string() bytes)
-__device__ __noinline__ uint64_t app_cstr(uint32_t* win, uint32_t pos, uint32_t carry, uint32_t index) {
-  WindowSink s = sink_at(win, pos, carry);
-  const FieldDesc cs = g_fields.f[CSTR_BASE + index];
-  const uint64_t* w = g_fields.w + cs.off;
-  for (uint32_t k = 0; k < ((uint32_t)cs.len >> 3); k++) s.put8w(w[k]);
-  const uint32_t rem = cs.len & 7u;
-  if (rem) s.put64(w[cs.len >> 3], rem);  // the table pads with zero bytes
-  return sink_state(s);
-}
-// Emit pass, the same fields as a loop: all lanes of a warp are at the same field at the same time, so the field's
-// descriptor and the words of its literal are warp-uniform constant loads, the loop's body is small enough to stay
-// in the instruction cache, and lanes whose event lacks a field sit out one iteration.  Descriptor (64 bits):
-// literal word offset 0..11, literal length 12..19, operation 20..23, value slot offset 24..35, group bytes 36..43
-// (non-zero: the field starts a group, see kGroupBytes), value type 44..49.
-enum : uint32_t { OP_NONE = 0, OP_U32, OP_I32, OP_U64, OP_I64, OP_TS, OP_DBL, OP_CSTR, OP_OTHER };
-constexpr uint32_t field_op(int type, int vk) {
-  switch (type) {
-    case T_NONE: return OP_NONE;
-    case T_U64: return vk == VK_64 ? OP_U64 : OP_U32;
-    case T_I64: return vk == VK_64 ? OP_I64 : (vk == VK_I32 ? OP_I32 : OP_U32);
-    case T_TS: return OP_TS;
-    case T_DBL: return OP_DBL;
-    case T_CSTR: return OP_CSTR;
-    default: return OP_OTHER;
+// A constant string of the field table by its index, which differs from lane to lane: from global memory (a constant-bank
+// load is repeated for every index in the warp).
+struct ConstString { uint64_t w[4]; uint64_t len; };
+struct ConstStrings { ConstString s[CS_HWC]; };
+constexpr ConstStrings make_const_strings() {
+  ConstStrings t{};
+  for (int k = 0; k < CS_HWC; k++) {
+    const char* text = kAllFields[CSTR_BASE + k].lit;
+    t.s[k].len = (uint64_t)c_strlen(text);
+    for (int i = 0; text[i]; i++) t.s[k].w[i / 8] |= (uint64_t)(unsigned char)text[i] << (8 * (i % 8));
   }
-}
-struct LoopDescs { uint64_t d[FIELD_COUNT]; };
-constexpr void fill_class_descs(LoopDescs& t, int base, int nf) {
-  for (int f = 0; f < nf; f++) {
-    const FieldSrc& src = kAllFields[base + f];
-    const uint64_t grp = group_starts_at(base, 0, f) ? group_bytes_from(base, f, nf) : 0;
-    t.d[base + f] = (uint64_t)field_word_offset(base + f) | ((uint64_t)c_strlen(src.lit) << 12) | ((uint64_t)field_op(src.type, src.vk) << 20) |
-                    ((uint64_t)src.voff << 24) | (grp << 36) | ((uint64_t)src.type << 44);  // type: 6 bits
-  }
-}
-constexpr LoopDescs make_loop_descs() {
-  LoopDescs t{};
-  fill_class_descs(t, API_BASE, A_COUNT); fill_class_descs(t, KERNEL_BASE, K_COUNT); fill_class_descs(t, MEM_BASE, M_COUNT);
-  fill_class_descs(t, OP_BASE, O_COUNT);
   return t;
 }
-constexpr uint32_t longest_group(const LoopDescs& t) {
-  uint32_t m = 0;
-  for (int f = 0; f < FIELD_COUNT; f++) if (((t.d[f] >> 36) & 0xffu) > m) m = (uint32_t)(t.d[f] >> 36) & 0xffu;
-  return m;
+static_assert(longest_constant_string() <= 32, "ConstString holds every constant string");
+__device__ const ConstStrings g_const_strings = make_const_strings();
+__device__ __noinline__ uint64_t app_cstr(Win win, uint32_t pos, uint32_t carry, uint32_t index) {
+  WindowSink s = sink_at(win, pos, carry);
+  const ConstString& cs = g_const_strings.s[index];
+  uint32_t len = (uint32_t)cs.len;
+  const uint64_t first = cs.w[0];
+  s.put64(first, len < 8u ? len : 8u);
+#pragma unroll 1
+  for (uint32_t k = 1; len > 8u; k++) { len -= 8u; s.put64(cs.w[k], len < 8u ? len : 8u); }
+  return sink_state(s);
 }
-// a field that is longer than a group on its own still has to fit behind the open block of a flushed window
-static_assert(longest_group(make_loop_descs()) + 32 + 8 <= (uint32_t)kWinBytes && longest_group(make_loop_descs()) < 256, "group does not fit the window");
-__constant__ LoopDescs g_loop = make_loop_descs();
-template <int BASE, int NF>
-__device__ __forceinline__ void loop_fields(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
-#pragma unroll 1
-  for (int f = 0; f < NF; f++) {
-    const bool on = (present >> f) & 1ull;
-    const uint64_t desc = g_loop.d[BASE + f];
-    const uint32_t grp = (uint32_t)(desc >> 36) & 0xffu;
-    if (grp != 0u) s.ensure(grp);  // also when no lane has the field: the group's other fields rely on it
-    if (on) {
-      const uint32_t len = (uint32_t)(desc >> 12) & 0xffu;
-      if (len != 0u) {
-        const uint64_t* w = g_fields.w + ((uint32_t)desc & 0xfffu);
-        const uint32_t ph = s.pos & 3u, sft = ph << 3, nw = (len + 7u) >> 3;
-        uint32_t* p = s.win + (s.pos >> 2) * (uint32_t)kWinStride;
-        uint32_t c = s.carry, t0 = 0, t1 = 0;
-#pragma unroll 1
-        for (uint32_t k = 0; k < nw; k++) {  // whole words; the table pads every literal with zero bytes
-          const uint64_t x = w[k];
-          const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
-          t0 = c | (lo << sft); t1 = funnel_l(lo, hi, sft);
-          p[0] = t0; p[kWinStride] = t1;
-          c = funnel_l(hi, 0u, sft);
-          p += 2 * kWinStride;
-        }
-        const uint32_t rem = len & 7u;  // bytes of the last word copied that belong to the literal (0: all eight)
-        const uint32_t k = rem == 0u ? 2u : (ph + rem) >> 2;  // words that last copy completed
-        s.carry = k == 0u ? t0 : (k == 1u ? t1 : c);
-        s.pos += len;
-      }
-      const uint32_t op = (uint32_t)(desc >> 20) & 0xfu, voff = (uint32_t)(desc >> 24) & 0xfffu;
-      if (op != OP_NONE) {
-        uint64_t st;
-        if (op == OP_U32) st = app_u32(s.win, s.pos, s.carry, a[voff >> 2]);
-        else if (op == OP_I32) st = app_i32(s.win, s.pos, s.carry, (int32_t)a[voff >> 2]);
-        else if (op == OP_TS) st = app_ts(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[voff >> 3]);
-        else if (op == OP_U64) st = app_u64(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[voff >> 3]);
-        else if (op == OP_CSTR) st = app_cstr(s.win, s.pos, s.carry, a[voff >> 2]);
-        else if (op == OP_DBL) st = app_dbl(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[voff >> 3]);
-        else if (op == OP_I64) st = app_i64(s.win, s.pos, s.carry, (int64_t)reinterpret_cast<const uint64_t*>(a)[voff >> 3]);
-        else {  // names, metadata entries: they ask the sink for room themselves
-          put_value<WindowSink, false, true>(s, d, (int)((uint32_t)(desc >> 44) & 0x3fu), (uint64_t)a[voff >> 2], name_bytes);
-          st = sink_state(s);
-        }
-        s.pos = (uint32_t)st; s.carry = (uint32_t)(st >> 32);
-      }
+// Emit pass, the classes nearly all events belong to: the same fields as straight-line code.  A literal's words are
+// immediates, so a word costs a funnel shift by the write position's phase and a store, and none of them waits for a load;
+// the literals of neighbouring fields that are always there are one literal where no value stands between them.  Values are
+// formatted by calls (small ones in line).  The code is cut into steps whose longest text fits the window behind its open
+// block, and one loop runs a class's steps: room is asked for once per step, at one place, so that there is one copy of the
+// flush (with one at each of some hundred places the kernel waits for instructions).
+//
+// What a class prints, as ranges of its fields: fields that are always there, or those whose presence the first one's bit
+// tells.
+struct FieldRange { int first, last; bool always; };
+constexpr FieldRange kKernelRanges[] = {{K_HEAD, K_ARGS, true}, {K_EXT, K_EXTC, false}, {K_QUEUED, K_CHTYPE, true},
+                                        {K_CLOSE, K_CLOSE, true} /* K_COLL: the other launch's events */, {K_FLOW, K_FEND, false}};
+constexpr FieldRange kApiRanges[] = {{A_HEAD_RT, A_HEAD_RT, false}, {A_HEAD_DR, A_HEAD_DR, false}, {A_NAME, A_NAME, false},
+                                     {A_INVALID, A_INVALID, false}, {A_PID, A_ARGS, true}, {A_EXT, A_EXTC, false}, {A_CBID, A_CLOSE, true},
+                                     {A_FLOW_S, A_FLOW_S, false}, {A_FLOW_F, A_FLOW_F, false}, {A_FPID, A_FCAT, false}, {A_FBP, A_FBP, false},
+                                     {A_FEND, A_FEND, false}};
+constexpr FieldRange kMemRanges[] = {{M_CPY_KIND, M_CPY_DST, false}, {M_SET_KIND, M_SET_KIND, false}, {M_PID, M_ARGS, true},
+                                     {M_EXT, M_EXTC, false}, {M_FROMDEV, M_TOCTX, false}, {M_DEV, M_CTX, false}, {M_STREAM, M_BYTES, true},
+                                     {M_BW, M_BW, false}, {M_GRAPH, M_CLOSE, true}, {M_FLOW, M_FEND, false}};
+// (CPU-side activities with a duration; instant and counter events are the other launch's)
+constexpr FieldRange kOpRanges[] = {{O_CAT, O_CAT, true}, {O_NAME, O_NAME, true}, {O_PID, O_PAD, true}, {O_ARGS, O_ARGS, false},
+                                    {O_EXT, O_EXT, false}, {O_EXTC, O_EXTC, false}, {O_MD, O_MD, false}, {P_ARGS_CLOSE, P_ARGS_CLOSE, false},
+                                    {P_CLOSE, P_CLOSE, true}, {P_FLOW_S, P_FLOW_S, false}, {P_FLOW_F, P_FLOW_F, false}, {P_FPID, P_FTS, false},
+                                    {P_FWDBWD, P_FWDBWD, false}, {P_AC2G, P_AC2G, false}, {P_FBP, P_FBP, false}, {P_FEND, P_FEND, false}};
+// A run: literals one behind the other, then the last field's value.  cond: the bit that tells whether it is printed, or -1.
+struct Run { int first, last, cond; };
+constexpr int kMaxRuns = 160, kMaxSteps = 48;
+constexpr uint32_t kStepBytes = 120;
+static_assert(31 + kStepBytes + 8 <= (uint32_t)kWinBytes, "a step must fit a window that has just been flushed");
+constexpr uint32_t run_lit_bytes(int first, int last) { uint32_t n = 0; for (int i = first; i <= last; i++) n += (uint32_t)c_strlen(kAllFields[i].lit); return n; }
+// Most bytes a run takes; a value of any length asks for room itself.
+constexpr uint32_t run_bytes(int first, int last) {
+  const uint32_t v = value_max_bytes(kAllFields[last].type, kAllFields[last].vk);
+  return run_lit_bytes(first, last) + (v == 0xffffu ? 0u : v);
+}
+struct Steps {
+  Run run[kMaxRuns];
+  int n_runs;
+  int step_run[kMaxSteps + 1];  // first run of every step
+  int n_steps;
+  int cls_step[5];              // first step of every class: kernel, api, mem, op
+};
+template <int N> constexpr void add_class(Steps& t, int base, const FieldRange (&ranges)[N]) {
+  uint32_t used = 0xffffu;  // the first run starts a step
+  for (int r = 0; r < N; r++) {
+    for (int f = ranges[r].first; f <= ranges[r].last;) {
+      int v = f;
+      while (v < ranges[r].last && kAllFields[base + v].type == T_NONE) v++;
+      const uint32_t need = run_bytes(base + f, base + v);
+      if (used + need > kStepBytes) { t.step_run[t.n_steps++] = t.n_runs; used = 0; }
+      used += need;
+      if (value_max_bytes(kAllFields[base + v].type, kAllFields[base + v].vk) == 0xffffu) used = 0xffffu;  // what follows it asks for room again
+      t.run[t.n_runs++] = Run{base + f, base + v, ranges[r].always ? -1 : ranges[r].first};
+      f = v + 1;
     }
   }
 }
-constexpr int kEventThreads = 128;
-constexpr size_t events_smem_bytes(bool write) {
-  return (size_t)kEventThreads * kRecStride * 8 + (write ? ((size_t)kEventThreads * kWinWords + kWinPadWords) * 4 : 0);
+constexpr Steps make_steps() {
+  Steps t{};
+  t.cls_step[0] = 0;
+  add_class(t, KERNEL_BASE, kKernelRanges); t.cls_step[1] = t.n_steps;
+  add_class(t, API_BASE, kApiRanges); t.cls_step[2] = t.n_steps;
+  add_class(t, MEM_BASE, kMemRanges); t.cls_step[3] = t.n_steps;
+  add_class(t, OP_BASE, kOpRanges); t.cls_step[4] = t.n_steps;
+  t.step_run[t.n_steps] = t.n_runs;
+  return t;
 }
+constexpr Steps kSteps = make_steps();
+constexpr int kNumSteps = kSteps.n_steps;
+constexpr bool steps_fit() {
+  for (int st = 0; st < kSteps.n_steps; st++) {
+    uint32_t n = 0;
+    for (int r = kSteps.step_run[st]; r < kSteps.step_run[st + 1]; r++) n += run_bytes(kSteps.run[r].first, kSteps.run[r].last);
+    if (n > kStepBytes) return false;
+  }
+  return kSteps.n_steps <= kMaxSteps && kSteps.n_runs <= kMaxRuns;
+}
+static_assert(steps_fit(), "a step is longer than the room it asks for");
+template <int R> struct RunOf {  // run R, as constants (device code calls no host function)
+  static constexpr Run r = kSteps.run[R];
+  static constexpr uint32_t len = run_lit_bytes(r.first, r.last);
+  static constexpr FieldSrc field = kAllFields[r.last];
+  static constexpr int cond = r.cond, type = field.type, vk = field.vk, voff = field.voff;
+};
+template <int ST> struct StepOf { static constexpr int first = kSteps.step_run[ST], end = kSteps.step_run[ST + 1]; };
+template <int C> struct ClassSteps { static constexpr int first = kSteps.cls_step[C], end = kSteps.cls_step[C + 1]; };
+template <int R> struct RunLit {
+  uint32_t w[RunOf<R>::len / 4 + 1];
+  K2J_CONSTEXPR RunLit() : w{} {
+    uint32_t p = 0;
+    for (int f = kSteps.run[R].first; f <= kSteps.run[R].last; f++)
+      for (int i = 0; kAllFields[f].lit[i]; i++, p++) w[p / 4] |= (uint32_t)(unsigned char)kAllFields[f].lit[i] << (8 * (p % 4));
+  }
+};
+template <int R> __device__ __forceinline__ void put_run(WindowSink& s, const Dev& d, const uint32_t* a, unsigned long long* name_bytes) {
+  using I = RunOf<R>;
+  constexpr uint32_t n = I::len, nw = (n + 3) / 4, rem = n % 4;
+  if constexpr (n != 0) {
+    constexpr RunLit<R> l;
+    const uint32_t ph = s.pos & 3u, sh = ph << 3;
+    const Win p = win_from(s.win, s.pos >> 2);
+    uint32_t t = s.carry | (l.w[0] << sh);
+    win_st(p, 0, t);
+#pragma unroll
+    for (uint32_t k = 1; k < nw; k++) { t = funnel_l(l.w[k - 1], l.w[k], sh); win_st(p, k, t); }
+    const uint32_t c = funnel_l(l.w[nw - 1], 0u, sh);  // what the last word pushes into the next one
+    s.carry = rem == 0 || ph + rem >= 4u ? c : t;
+    s.pos += n;
+  }
+  if constexpr (I::type != T_NONE) {
+    constexpr int w = I::voff >> 2, u = I::voff >> 3;
+    uint64_t st;
+    if constexpr (I::type == T_TS) st = app_ts(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
+    else if constexpr (I::type == T_DBL) st = app_dbl(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
+    else if constexpr (I::type == T_CSTR) st = app_cstr(s.win, s.pos, s.carry, a[w]);
+    else if constexpr (I::type == T_U64 && I::vk == VK_64) st = app_u64(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
+    else if constexpr (I::type == T_I64 && I::vk == VK_64) st = app_i64(s.win, s.pos, s.carry, (int64_t)reinterpret_cast<const uint64_t*>(a)[u]);
+    else if constexpr (I::type == T_U64 || I::type == T_I64) {
+      const uint32_t v = a[w];  // (a negative value counts as large)
+      if (v < 1000u) { put_below_1000(s, v); st = sink_state(s); }
+      else if constexpr (I::vk == VK_I32) st = app_i32(s.win, s.pos, s.carry, (int32_t)v);
+      else st = app_u32(s.win, s.pos, s.carry, v);
+    } else {  // names, metadata entries: they ask the sink for room themselves
+      put_value<WindowSink, false, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
+      st = sink_state(s);
+    }
+    s.pos = (uint32_t)st; s.carry = (uint32_t)(st >> 32);
+  }
+}
+template <int R, int END>
+__device__ __forceinline__ void put_runs(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
+  if constexpr (R < END) {
+    if constexpr (RunOf<R>::cond < 0) put_run<R>(s, d, a, name_bytes);
+    else if ((present >> RunOf<R>::cond) & 1ull) put_run<R>(s, d, a, name_bytes);
+    put_runs<R + 1, END>(s, d, a, present, name_bytes);
+  }
+}
+template <int ST>
+__device__ __forceinline__ void put_step(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
+  if constexpr (ST < kNumSteps) put_runs<StepOf<ST>::first, StepOf<ST>::end>(s, d, a, present, name_bytes);
+}
+__device__ __forceinline__ void run_steps(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, int step, int end, unsigned long long* name_bytes) {
+#pragma unroll 1
+  for (; step < end; step++) {
+    s.room(kStepBytes);
+    switch (step) {
+#define K2J_STEP(i) case i: put_step<i>(s, d, a, present, name_bytes); break;
+#define K2J_STEP8(i) K2J_STEP(i) K2J_STEP(i + 1) K2J_STEP(i + 2) K2J_STEP(i + 3) K2J_STEP(i + 4) K2J_STEP(i + 5) K2J_STEP(i + 6) K2J_STEP(i + 7)
+      K2J_STEP8(0) K2J_STEP8(8) K2J_STEP8(16) K2J_STEP8(24) K2J_STEP8(32) K2J_STEP8(40)
+#undef K2J_STEP8
+#undef K2J_STEP
+      default: break;
+    }
+  }
+}
+constexpr int kEventThreads = 128;  // size pass, annotations
+constexpr int kEmitThreads = 320, kEmitBlocks = 2;  // most threads of a block of the emit pass, and how many such blocks share an SM
+// Dynamic shared memory.  Size pass: the threads' record areas.  Emit pass: the digit table, the record areas, the windows
+// (per warp: [kWinWords][32 lanes]; a pad after the last warp).
+constexpr size_t size_smem_bytes() { return (size_t)kEventThreads * kRecStride * 8; }
+constexpr size_t emit_smem_bytes(int threads) { return sizeof(Digits3) + (size_t)threads * kRecStride * 8 + ((size_t)threads * kWinWords + kWinPadWords) * 4; }
+static_assert(kEmitBlocks * (emit_smem_bytes(kEmitThreads) + 1024) <= 228 * 1024, "the blocks of an SM fit its shared memory");
 
 // COLL (emit pass only): this launch writes the kernel events that carry collective metadata, and only those; the
 // launch without it writes everything else and holds no code for them.  Returns false when the event is left to
@@ -2387,11 +2466,13 @@ __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32
     if constexpr (COLL) run_fields<S, COLL>(s, d, a, base, p, nb);
     else {
       // the classes nearly all events belong to run compile-time field code; the others share the table-driven loop
-      if (base == API_BASE) loop_fields<API_BASE, A_COUNT>(s, d, a, p, nb);
-      else if (base == KERNEL_BASE) loop_fields<KERNEL_BASE, K_COUNT>(s, d, a, p, nb);
-      else if (base == MEM_BASE) loop_fields<MEM_BASE, M_COUNT>(s, d, a, p, nb);
-      else if (cls == C_OP) loop_fields<OP_BASE, O_COUNT>(s, d, a, p, nb);
-      else run_fields<S, COLL>(s, d, a, base, p, nb);
+      int step = -1, end = -1;
+      if (base == API_BASE) { step = ClassSteps<1>::first; end = ClassSteps<1>::end; }
+      else if (base == KERNEL_BASE) { step = ClassSteps<0>::first; end = ClassSteps<0>::end; }
+      else if (base == MEM_BASE) { step = ClassSteps<2>::first; end = ClassSteps<2>::end; }
+      else if (cls == C_OP) { step = ClassSteps<3>::first; end = ClassSteps<3>::end; }
+      if (step < 0) run_fields<S, COLL>(s, d, a, base, p, nb);
+      else if (p != 0ull) run_steps(s, d, a, p, step, end, nb);
     }
   }
   return true;
@@ -2409,17 +2490,20 @@ __device__ __forceinline__ uint32_t class_units(int cls) {
 // with coalesced loads (lane = 8-byte unit of a record); all later reads of record fields and of the
 // values computed from them are shared-memory reads at table-given offsets.
 template <bool WRITE, bool COLL = false>
-__global__ void __launch_bounds__(kEventThreads, WRITE ? 5 : 8) k_events(Dev d) {
-  // dynamic shared memory (events_smem_bytes): the threads' record areas, then (emit pass) their output windows
-  extern __shared__ uint64_t s_dyn[];
-  uint64_t* const s_rec = s_dyn;
-  uint32_t* const s_win = reinterpret_cast<uint32_t*>(s_dyn + kEventThreads * kRecStride);  // per warp: [kWinWords][32 lanes]; a pad after the last warp
+__global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? kEmitBlocks : 8) k_events(Dev d) {
+  const uint32_t threads = WRITE ? blockDim.x : (uint32_t)kEventThreads;
+  uint64_t* const s_rec = reinterpret_cast<uint64_t*>(s_dyn + (WRITE ? sizeof(Digits3) / 16 : 0));
+  uint32_t* const s_win = reinterpret_cast<uint32_t*>(s_rec + threads * kRecStride);
+  if (WRITE) {
+    for (uint32_t k = threadIdx.x; k < sizeof(Digits3) / 16; k += threads) s_dyn[k] = reinterpret_cast<const uint4*>(&g_digits3)[k];
+    __syncthreads();
+  }
   __shared__ unsigned long long s_cnt[8];
   if (!WRITE) {
     if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
     __syncthreads();
   }
-  uint64_t i = d.work_origin + (uint64_t)blockIdx.x * kEventThreads + threadIdx.x;
+  uint64_t i = d.work_origin + (uint64_t)blockIdx.x * threads + threadIdx.x;
   if (d.work_indirect != nullptr) i = i < d.n_indirect ? (uint64_t)d.work_indirect[i] : d.n_work;
   Tally t; t.x = 0; t.flow = 0; t.name_bytes = 0; t.ev = 0; t.work = i;
   uint32_t filt = 0;
@@ -2494,7 +2578,7 @@ __global__ void __launch_bounds__(kEventThreads, WRITE ? 5 : 8) k_events(Dev d) 
       if (cls != C_OP) d.ev_ext[ev] = ext;
     } else {
       WindowSink s;
-      s.init(d.out + off, size, s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u));
+      s.init(d.out + off, size, (Win)__cvta_generic_to_shared(s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u)));
       if (format_event<WindowSink, COLL>(s, d, cls, area, j, t, &filt, &ext) && !s.finish(d.out + off, size))
         atomicAdd(&d.counters->device_check, 1ull);
     }
@@ -2625,7 +2709,7 @@ __global__ void __launch_bounds__(kEventThreads) k_annotations(Dev d, const Span
     uint8_t* dst = d.out + out_base + offs[i];
     if (size < kMinEventBytes || out_base + offs[i] + size > d.out_cap) { atomicAdd(&d.counters->device_check, 1ull); return; }
     WindowSink s;
-    s.init(dst, size, s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u));
+    s.init(dst, size, (Win)__cvta_generic_to_shared(s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u)));
     run_fields(s, d, a, ANN_BASE, p, &nb);
     if (!s.finish(dst, size)) atomicAdd(&d.counters->device_check, 1ull);
   }

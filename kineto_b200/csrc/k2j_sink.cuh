@@ -53,55 +53,86 @@ constexpr uint32_t kWinSlack = 40;          // room that always stays free after
                                             // do not ask first, and the word past the end that an append may touch
 K2J_HD uint64_t pack64(uint32_t lo, uint32_t hi) { return (uint64_t)lo | ((uint64_t)hi << 32); }
 
+// A window: on the GPU the 32-bit shared-memory address of its word 0 (so that out-of-line functions that take one read and
+// write shared memory, not generic addresses), on a CPU a pointer to it.
+#if defined(__CUDACC__)
+using Win = uint32_t;
+__device__ __forceinline__ uint32_t win_ld(Win w, uint32_t k) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(w + k * (uint32_t)(4 * kWinStride)));
+  return v;
+}
+__device__ __forceinline__ void win_st(Win w, uint32_t k, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(w + k * (uint32_t)(4 * kWinStride)), "r"(v));
+}
+__device__ __forceinline__ Win win_from(Win w, uint32_t k) { return w + k * (uint32_t)(4 * kWinStride); }
+#else
+using Win = uint32_t*;
+inline uint32_t win_ld(Win w, uint32_t k) { return w[k * (uint32_t)kWinStride]; }
+inline void win_st(Win w, uint32_t k, uint32_t v) { w[k * (uint32_t)kWinStride] = v; }
+inline Win win_from(Win w, uint32_t k) { return w + k * (uint32_t)kWinStride; }
+#endif
+K2J_HD void win_block_out(Win win, uint8_t* gbase, uint32_t b) {
+  const uint32_t k = 8u * b;
+  const uint32_t x0 = win_ld(win, k), x1 = win_ld(win, k + 1), x2 = win_ld(win, k + 2), x3 = win_ld(win, k + 3), x4 = win_ld(win, k + 4),
+                 x5 = win_ld(win, k + 5), x6 = win_ld(win, k + 6), x7 = win_ld(win, k + 7);
+  store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
+}
+// Writes the complete 32-byte blocks of a window to global memory and moves the open block to the front; returns their
+// number.  `open`: 0, or the offset of the first word that the first block has still to write (its earlier words are out).
+K2J_HD uint32_t window_flush(Win win, uint32_t pos, uint32_t carry, uint8_t* gbase, uint32_t open) {
+  win_st(win, pos >> 2, carry);
+  const uint32_t nb = pos >> 5;
+  uint32_t b = 0;
+  if (open != 0u && nb != 0u) {  // a block whose first words are out already: whole words only
+    for (uint32_t o = open; o < 32u; o += 8u) *reinterpret_cast<uint64_t*>(gbase + o) = pack64(win_ld(win, o >> 2), win_ld(win, (o >> 2) + 1u));
+    b = 1;
+  }
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+  for (; b + 2u <= nb; b += 2u) {  // two blocks at a time: sixteen loads in flight before the two stores
+    const uint32_t k = 8u * b;
+    const uint32_t x0 = win_ld(win, k), x1 = win_ld(win, k + 1), x2 = win_ld(win, k + 2), x3 = win_ld(win, k + 3), x4 = win_ld(win, k + 4),
+                   x5 = win_ld(win, k + 5), x6 = win_ld(win, k + 6), x7 = win_ld(win, k + 7);
+    const uint32_t y0 = win_ld(win, k + 8), y1 = win_ld(win, k + 9), y2 = win_ld(win, k + 10), y3 = win_ld(win, k + 11), y4 = win_ld(win, k + 12),
+                   y5 = win_ld(win, k + 13), y6 = win_ld(win, k + 14), y7 = win_ld(win, k + 15);
+    store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
+    store32(gbase + 32u * b + 32u, pack64(y0, y1), pack64(y2, y3), pack64(y4, y5), pack64(y6, y7));
+  }
+  if (b < nb) win_block_out(win, gbase, b);
+  if (nb != 0u) {
+    const uint32_t k = 8u * nb;
+    const uint32_t x0 = win_ld(win, k), x1 = win_ld(win, k + 1), x2 = win_ld(win, k + 2), x3 = win_ld(win, k + 3), x4 = win_ld(win, k + 4),
+                   x5 = win_ld(win, k + 5), x6 = win_ld(win, k + 6), x7 = win_ld(win, k + 7);
+    win_st(win, 0, x0); win_st(win, 1, x1); win_st(win, 2, x2); win_st(win, 3, x3);
+    win_st(win, 4, x4); win_st(win, 5, x5); win_st(win, 6, x6); win_st(win, 7, x7);
+  }
+  return nb;
+}
+
 struct WindowSink {
   static constexpr bool kCounting = false;
-  uint32_t* win;          // word 0 of this thread's window; word k is win[k * kWinStride]
+  Win win;                // this thread's window
   uint32_t pos;           // window offset of the next byte
   uint32_t carry;         // the 32-bit word being filled: bytes below pos & 3 are set, the rest is zero
-  uint32_t w0;            // offset of the event's first 8-byte word in its first block; that block is open while head != 0
-  uint32_t head;          // 1 until the event's first block has left, if the event starts inside it
+  uint32_t open;          // 0, or: the window's first block has been written up to this offset (see window_flush)
   uint8_t* gbase;         // global address of window byte 0, 32-byte aligned
-  K2J_HD uint32_t& W(uint32_t k) const { return win[k * (uint32_t)kWinStride]; }
-  K2J_HD uint64_t W64(uint32_t k) const { return pack64(W(k), W(k + 1u)); }  // the 8 bytes from word k on
-  K2J_HD void init(uint8_t* dst, uint32_t, uint32_t* window) {
+  K2J_HD uint64_t W64(uint32_t k) const { return pack64(win_ld(win, k), win_ld(win, k + 1u)); }  // the 8 bytes from word k on
+  K2J_HD void init(uint8_t* dst, uint32_t, Win window) {
     const uint32_t phase32 = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 31u), phase = phase32 & 7u, sh = 8u * phase;
     win = window; gbase = dst - phase32; pos = phase32; carry = 0u;
-    w0 = phase32 & ~7u; head = phase32 ? 1u : 0u;
+    const uint32_t w0 = phase32 & ~7u;  // the event's first 8-byte word is written here and now
+    open = phase32 ? w0 + 8u : 0u;
     const uint64_t w = ((kEventTail8 >> 1) >> (63u - sh)) | (kEventHead8 << sh);
     if (phase < 4u) *reinterpret_cast<uint64_t*>(gbase + w0) = w;
     else *reinterpret_cast<uint32_t*>(gbase + w0 + 4) = (uint32_t)(w >> 32);
   }
-  K2J_HD void block_out(uint32_t b) {
-    const uint32_t k = 8u * b;
-    const uint32_t x0 = W(k), x1 = W(k + 1), x2 = W(k + 2), x3 = W(k + 3), x4 = W(k + 4), x5 = W(k + 5), x6 = W(k + 6), x7 = W(k + 7);
-    store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
-  }
   // Writes the complete 32-byte blocks of the window to global memory and moves the open block to the front.
   K2J_HD void flush() {
-    W(pos >> 2) = carry;
-    const uint32_t nb = pos >> 5;
-    uint32_t b = 0;
-    if (head != 0u && nb != 0u) {  // the event starts inside its first block: whole words only (init wrote the first one)
-      for (uint32_t o = w0 + 8u; o < 32u; o += 8u) *reinterpret_cast<uint64_t*>(gbase + o) = W64(o >> 2);
-      b = 1; head = 0u;
-    }
-#if defined(__CUDA_ARCH__)
-#pragma unroll 1
-#endif
-    for (; b + 2u <= nb; b += 2u) {  // two blocks at a time: sixteen loads in flight before the two stores
-      const uint32_t k = 8u * b;
-      const uint32_t x0 = W(k), x1 = W(k + 1), x2 = W(k + 2), x3 = W(k + 3), x4 = W(k + 4), x5 = W(k + 5), x6 = W(k + 6), x7 = W(k + 7);
-      const uint32_t y0 = W(k + 8), y1 = W(k + 9), y2 = W(k + 10), y3 = W(k + 11), y4 = W(k + 12), y5 = W(k + 13), y6 = W(k + 14), y7 = W(k + 15);
-      store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
-      store32(gbase + 32u * b + 32u, pack64(y0, y1), pack64(y2, y3), pack64(y4, y5), pack64(y6, y7));
-    }
-    if (b < nb) block_out(b);
-    if (nb != 0u) {
-      const uint32_t k = 8u * nb;
-      const uint32_t x0 = W(k), x1 = W(k + 1), x2 = W(k + 2), x3 = W(k + 3), x4 = W(k + 4), x5 = W(k + 5), x6 = W(k + 6), x7 = W(k + 7);
-      W(0) = x0; W(1) = x1; W(2) = x2; W(3) = x3; W(4) = x4; W(5) = x5; W(6) = x6; W(7) = x7;
-      gbase += 32u * nb; pos -= 32u * nb;
-    }
+    const uint32_t nb = window_flush(win, pos, carry, gbase, open);
+    if (nb != 0u) open = 0u;
+    gbase += 32u * nb; pos -= 32u * nb;
   }
   // After this call n more bytes fit, with kWinSlack to spare.  n <= kWinBytes - 32 - kWinSlack.
   // On the GPU the lanes of a warp that are executing together flush together, as soon as one of them needs
@@ -114,17 +145,26 @@ struct WindowSink {
     if (pos + n + kWinSlack > (uint32_t)kWinBytes) flush();
 #endif
   }
+  // The same without the slack, for callers that count every byte they append: n <= kWinBytes - 40 bytes fit (an append may
+  // touch the word behind its last byte).
+  K2J_HD void room(uint32_t n) {
+#if defined(__CUDA_ARCH__)
+    if (__any_sync(__activemask(), pos + n + 8u > (uint32_t)kWinBytes)) flush();
+#else
+    if (pos + n + 8u > (uint32_t)kWinBytes) flush();
+#endif
+  }
   // append the low `len` (0..4) bytes of w; bytes above len must be zero
   K2J_HD void put(uint32_t w, int len) {
     const uint32_t ph = pos & 3u, s = ph << 3;
     const uint32_t t = carry | (w << s);
-    W(pos >> 2) = t;
+    win_st(win, pos >> 2, t);
     carry = ph + (uint32_t)len >= 4u ? funnel_l(w, 0u, s) : t;  // the funnel shift gives w >> (32 - s), and 0 for s = 0
     pos += (uint32_t)len;
   }
   K2J_HD void put4(uint32_t w) {
     const uint32_t s = (pos & 3u) << 3;
-    W(pos >> 2) = carry | (w << s);
+    win_st(win, pos >> 2, carry | (w << s));
     carry = funnel_l(w, 0u, s);
     pos += 4u;
   }
@@ -133,7 +173,7 @@ struct WindowSink {
     const uint32_t lo = (uint32_t)w, hi = (uint32_t)(w >> 32);
     const uint32_t ph = pos & 3u, s = ph << 3, i = pos >> 2;
     const uint32_t t0 = carry | (lo << s), t1 = funnel_l(lo, hi, s), t2 = funnel_l(hi, 0u, s);
-    W(i) = t0; W(i + 1) = t1;
+    win_st(win, i, t0); win_st(win, i + 1, t1);
     const uint32_t k = (ph + len) >> 2;  // words completed: 0..2
     carry = k == 0u ? t0 : (k == 1u ? t1 : t2);
     pos += len;
@@ -141,7 +181,7 @@ struct WindowSink {
   K2J_HD void put8w(uint64_t w) {  // append 8 bytes
     const uint32_t lo = (uint32_t)w, hi = (uint32_t)(w >> 32);
     const uint32_t s = (pos & 3u) << 3, i = pos >> 2;
-    W(i) = carry | (lo << s); W(i + 1) = funnel_l(lo, hi, s);
+    win_st(win, i, carry | (lo << s)); win_st(win, i + 1, funnel_l(lo, hi, s));
     carry = funnel_l(hi, 0u, s);
     pos += 8u;
   }
@@ -186,7 +226,7 @@ struct WindowSink {
       for (uint32_t k = 0; k < 8u; k++) {
         if (k < nw) {
           const uint32_t lo = (uint32_t)x[k], hi = (uint32_t)(x[k] >> 32);
-          W(i) = c | (lo << s); W(i + 1) = funnel_l(lo, hi, s);
+          win_st(win, i, c | (lo << s)); win_st(win, i + 1, funnel_l(lo, hi, s));
           c = funnel_l(hi, 0u, s);
           i += 2;
         }
@@ -219,11 +259,11 @@ struct WindowSink {
   // event's end.  Returns false if the byte count differs from the size the event was given.
   K2J_HD bool finish(const uint8_t* dst, uint32_t size) {
     flush();
-    for (uint32_t o = head != 0u ? w0 + 8u : 0u; o + 8u <= pos; o += 8u)  // the event's very first word was written by init
+    for (uint32_t o = open; o + 8u <= pos; o += 8u)  // the event's very first word was written by init
       *reinterpret_cast<uint64_t*>(gbase + o) = W64(o >> 2);
     const uint32_t e = pos & 7u;
     if (e) {
-      const uint64_t lo = (pos & 4u) ? pack64(W((pos >> 2) - 1u), carry) : (uint64_t)carry;
+      const uint64_t lo = (pos & 4u) ? pack64(win_ld(win, (pos >> 2) - 1u), carry) : (uint64_t)carry;
       const uint64_t t = lo | (0x20200Aull << (8u * e));  // the next event begins "\n  "
       if (e > 4u) *reinterpret_cast<uint64_t*>(gbase + (pos & ~7u)) = t;
       else *reinterpret_cast<uint32_t*>(gbase + (pos & ~7u)) = (uint32_t)t;
