@@ -79,7 +79,7 @@ struct k2j_ctx {
   DevBuf slot_code, exit_map, chunk_entry, chunk_cnt, chunk_base, scan_sums, scan_totals;
   DevBuf ds_tab, span_key, span_nstart, span_end, span_nfirst, span_row, span_out, span_cnt, ann_size, ann_off;
   DevBuf sort_keys[2], sort_vals[2], sort_hist, sort_base, sort_rank;
-  DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, out, counters;
+  DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, hand, out, counters;
   uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans (23 and 27 are words of scan_totals, device memory: sort, filtered join keys)
   Counters* h_counters = nullptr; // pinned
   SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans, behind h_totals in one allocation
@@ -390,7 +390,7 @@ void k2j_destroy(k2j_ctx* c) {
                     &c->chunk_base, &c->scan_sums, &c->scan_totals, &c->ds_tab, &c->span_key, &c->span_nstart, &c->span_end, &c->span_nfirst, &c->span_row,
                     &c->span_out, &c->span_cnt, &c->ann_size, &c->ann_off, &c->sort_keys[0], &c->sort_keys[1], &c->sort_vals[0],
                     &c->sort_vals[1], &c->sort_hist, &c->sort_base, &c->sort_rank, &c->tid_tab, &c->corr_tab, &c->user_tab, &c->op_tab,
-                    &c->work_slot, &c->work_ev, &c->ev_size, &c->ev_off, &c->ev_ext, &c->out, &c->counters, &c->ext_local, &c->ctx_tab, &c->evt_recs,
+                    &c->work_slot, &c->work_ev, &c->ev_size, &c->ev_off, &c->ev_ext, &c->hand, &c->out, &c->counters, &c->ext_local, &c->ctx_tab, &c->evt_recs,
                     &c->seen_tab, &c->row_key, &c->row_first, &c->corr_zero, &c->str_class, &c->comms_flag, &c->coll_list, &c->corr0,
                     &c->exp_keys, &c->exp_first, &c->exp_list, &c->exp_out, &c->coll_tab})
     b->release();
@@ -1001,6 +1001,10 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   K2J_CUDA(c, c->ev_off.reserve(std::max<uint64_t>(1, d.n_events) * 8));
   K2J_CUDA(c, c->ev_ext.reserve(std::max<uint64_t>(1, d.n_events) * 4));
   d.ev_size = c->ev_size.as<uint32_t>(); d.ev_off = c->ev_off.as<uint64_t>(); d.ev_ext = c->ev_ext.as<int32_t>();
+  const uint64_t hand_kernels = d.cls_begin[C_MEMCPY] - d.cls_begin[C_KERNEL], hand_items = d.cls_begin[C_OVERHEAD] - d.cls_begin[C_KERNEL];
+  K2J_CUDA(c, c->hand.reserve(std::max<uint64_t>(1, hand_kernels * (3 * sizeof(uint4) + 8) + hand_items * 8)));
+  d.hand_occ = c->hand.as<uint4>(); d.hand_pitch = hand_kernels;
+  d.hand_wps = reinterpret_cast<uint64_t*>(d.hand_occ + 3 * hand_kernels); d.hand_dec = d.hand_wps + hand_kernels;
   // With gathered keys only those this shard's events can look up enter its tables (see k_mark_corr), so the tables
   // are sized by the shard: its events, plus the share of foreign keys the marking lets through by chance.
   const bool filter = c->have_global_join;

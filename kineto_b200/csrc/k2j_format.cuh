@@ -289,23 +289,8 @@ template <class S> K2J_HD void put_zeros(S& s, int n) {
   }
 }
 
-// fmt::format("{}", v) for finite v: the shortest digits that round-trip, fixed notation when the decimal
-// exponent lies in [-4, 16), exponent notation otherwise.
-template <class S> K2J_HD void put_double(S& s, double v) {
-  const DoubleLayout L = double_layout(v);
-  if (L.neg) put_char(s, '-');
-  if (L.zero) { put_char(s, '0'); return; }
-  const int nd = L.nd, e10 = L.e10;
-  if (S::kCounting) {
-    if (e10 < -4 || e10 >= 16) {
-      const int a = e10 < 0 ? -e10 : e10;
-      s.skip((uint32_t)(nd + (nd > 1 ? 1 : 0) + 2 + (a < 100 ? 2 : 3)));
-    } else if (e10 >= nd - 1) s.skip((uint32_t)(e10 + 1));
-    else if (e10 >= 0) s.skip((uint32_t)(nd + 1));
-    else s.skip((uint32_t)(nd + 1 - e10));
-    return;
-  }
-  const Digits17 D = digits17(L.dec);
+// nd significant digits, the last ones of D, as fixed or exponent notation by the decimal exponent e10
+template <class S> K2J_HD void put_placed(S& s, const Digits17& D, int nd, int e10) {
   const int z = 17 - nd;  // leading zeros of the padded string
   if (e10 < -4 || e10 >= 16) {
     s.put64(digits_at(D, z) & 0xffull, 1);
@@ -327,6 +312,41 @@ template <class S> K2J_HD void put_double(S& s, double v) {
     s.put64(0x303030302E30ull & (~0ull >> (8 * (7 + e10))), (uint32_t)(1 - e10));  // "0." and -e10 - 1 zeros
     put_digits(s, D, z, nd);
   }
+}
+// fmt::format("{}", v) for finite v: the shortest digits that round-trip, fixed notation when the decimal
+// exponent lies in [-4, 16), exponent notation otherwise.
+template <class S> K2J_HD void put_layout(S& s, const DoubleLayout& L);
+template <class S> K2J_HD void put_double(S& s, double v) { put_layout(s, double_layout(v)); }
+// A positive finite double's digits in one word, for a pass that writes what an earlier one has worked out: the significand
+// (below 10^17 < 2^57) with its decimal exponent + kPackedExp10 above it; 0 for every other value (and for magnitudes that
+// do not fit, below 1e-46 and from 1e81 on): those are worked out again.
+constexpr int kPackedExp10 = 47;
+K2J_HD uint64_t pack_double(double v) {
+  if (!double_is_finite(v)) return 0;
+  const DoubleLayout L = double_layout(v);
+  const int code = L.e10 + kPackedExp10;
+  if (L.neg || L.zero || code < 1 || code > 127) return 0;
+  return L.dec | ((uint64_t)code << 57);
+}
+template <class S> K2J_HD void put_packed_double(S& s, uint64_t w) {  // w != 0
+  DoubleLayout L;
+  L.dec = w & ((1ull << 57) - 1ull); L.nd = ndigits64(L.dec); L.e10 = (int)(w >> 57) - kPackedExp10; L.neg = false; L.zero = false;
+  put_layout(s, L);
+}
+template <class S> K2J_HD void put_layout(S& s, const DoubleLayout& L) {
+  if (L.neg) put_char(s, '-');
+  if (L.zero) { put_char(s, '0'); return; }
+  const int nd = L.nd, e10 = L.e10;
+  if (S::kCounting) {
+    if (e10 < -4 || e10 >= 16) {
+      const int a = e10 < 0 ? -e10 : e10;
+      s.skip((uint32_t)(nd + (nd > 1 ? 1 : 0) + 2 + (a < 100 ? 2 : 3)));
+    } else if (e10 >= nd - 1) s.skip((uint32_t)(e10 + 1));
+    else if (e10 >= 0) s.skip((uint32_t)(nd + 1));
+    else s.skip((uint32_t)(nd + 1 - e10));
+    return;
+  }
+  put_placed(s, digits17(L.dec), nd, e10);
 }
 // TypedMetadataJson.h:172-178: finite values bare, non-finite values quoted.
 template <class S> K2J_HD void put_double_value(S& s, double v) {

@@ -183,6 +183,10 @@ struct Dev {
   uint32_t* corr_zero;     // one bit per correlation-table slot: the entry links to a CPU op whose id is 0
   uint32_t* ev_size; const uint64_t* ev_off; uint64_t n_events;
   int32_t* ev_ext;        // per event: id of the linked CPU op found by the size pass (0 = none)
+  // What the size pass has worked out for the emit pass, per work item of the kernel, copy and memset classes (index 0 =
+  // the first kernel): doubles as pack_double's words (kernels: blocks per SM; copies and memsets: the bandwidth), and for
+  // kernels warps per SM and the occupancy calculator's results (hand_occ: 3 rows of hand_pitch).
+  uint64_t* hand_dec; uint64_t* hand_wps; uint4* hand_occ; uint64_t hand_pitch;
   uint8_t* out; uint64_t out_cap;  // address of output byte 0 (of the whole text), bytes of the whole text
   // Sharded traces: records in front of guest_front (a slot index) and from guest_back on are other shards' records
   // that only feed this shard's lookups (contexts, CUDA event records, streams with GPU work, first stream syncs):
@@ -953,7 +957,8 @@ enum : uint8_t { T_NONE = 0, T_U64, T_I64, T_TS, T_DBL, T_NAME, T_CSTR, T_MD /* 
                  T_RAWSTR = 12 /* a pool string as it is */, T_RAWSTRIP /* ... minus one surrounding pair of quotes */,
                  T_MDRAW /* metadata entries with keys and strings as they are */,
                  T_MDCNT /* the counter values of a counter event: "name": value,... */,
-                 T_HWC /* one whole counter event per counter value (HARDWARE_COUNTERS) */ };
+                 T_HWC /* one whole counter event per counter value (HARDWARE_COUNTERS) */,
+                 T_DEC /* a positive finite double as pack_double's word */ };
 enum : uint8_t { VK_U32 = 0, VK_I32 /* sign-extended */, VK_64 };
 struct FieldSrc { const char* lit; uint8_t type; uint8_t vk; uint16_t voff; };
 struct FieldDesc { uint16_t off, len; uint8_t type, vk; uint16_t voff; };
@@ -1004,7 +1009,7 @@ enum : int { KS_COLLROW = 0 /* row of the linked record_param_comms op */, KS_RE
              KS_LSMEM = 112, KS_LWARPS = 116, KR_QUEUED = 120, KS_WPS = 128, KS_LBLOCKS = 136, KS_LBARR = 140, KR_NODE = 144,
              KS_AREGS = 152, KR_GRAPH = 156, KS_ASMEM = 160, KR_CHAN = 168, KR_CHTYPE = 172 };
 enum : int { K_HEAD, K_PID, K_TID, K_TS, K_DUR, K_ARGS, K_EXT, K_EXTC, K_QUEUED, K_DEV, K_CTX, K_STREAM, K_CORR, K_REGS, K_SMEM,
-             K_BPS, K_WPS, K_GX, K_GY, K_GZ, K_BX, K_BY, K_BZ, K_OCCPCT, K_ACTIVE, K_LIMIT, K_LREGS, K_LSMEM, K_LWARPS, K_LBLOCKS,
+             K_BPS, K_WPS, K_BPSRAW, K_WPSRAW /* values pack_double leaves out */, K_GX, K_GY, K_GZ, K_BX, K_BY, K_BZ, K_OCCPCT, K_ACTIVE, K_LIMIT, K_LREGS, K_LSMEM, K_LWARPS, K_LBLOCKS,
              K_LBARR, K_AREGS, K_ASMEM, K_GRAPH, K_NODE, K_CHAN, K_CHTYPE, K_COLL, K_CLOSE, K_FLOW, K_FPID, K_FTID, K_FTS, K_FEND, K_COUNT };
 #define K2J_KERNEL_FIELDS \
     {XHEAD("kernel"), T_NAME, VK_U32, KR_NAME}, {"\",\n    \"pid\": ", T_U64, VK_U32, KR_DEV}, {",\n    \"tid\": ", T_U64, VK_U32, KR_STREAM}, \
@@ -1013,6 +1018,7 @@ enum : int { K_HEAD, K_PID, K_TID, K_TS, K_DUR, K_ARGS, K_EXT, K_EXTC, K_QUEUED,
     {"\"queued\": ", T_U64, VK_64, KR_QUEUED}, {", \"device\": ", T_U64, VK_U32, KR_DEV}, {", \"context\": ", T_U64, VK_U32, KR_CTX}, \
     {", \"stream\": ", T_U64, VK_U32, KR_STREAM}, {", \"correlation\": ", T_U64, VK_U32, KR_CORR}, \
     {", \"registers per thread\": ", T_U64, VK_U32, KS_REGS}, {", \"shared memory\": ", T_I64, VK_I32, KS_SMEM}, \
+    {", \"blocks per SM\": ", T_DEC, VK_64, KS_BPS}, {", \"warps per SM\": ", T_DEC, VK_64, KS_WPS}, \
     {", \"blocks per SM\": ", T_DBL, VK_64, KS_BPS}, {", \"warps per SM\": ", T_DBL, VK_64, KS_WPS}, \
     {", \"grid\": [", T_I64, VK_I32, KR_GRID}, {", ", T_I64, VK_I32, KR_GRID + 4}, {", ", T_I64, VK_I32, KR_GRID + 8}, \
     {"], \"block\": [", T_I64, VK_I32, KR_BLOCK}, {", ", T_I64, VK_I32, KR_BLOCK + 4}, {", ", T_I64, VK_I32, KR_BLOCK + 8}, \
@@ -1034,7 +1040,7 @@ enum : int { MR_BYTES = 8, MS_TS = 16, MS_DUR = 24, MR_DEV = 32, MR_CTX = 36, MR
              MR_TODEV = 52, MR_TOCTX = 56, MS_KIND0 = 100, MS_KIND1 = 104, MS_KIND2 = 108, MS_EXT = 112, MS_BW = 120, MS_GRAPH = 128,
              MS_NODE = 136, MS_CHAN = 144, MS_CHTYPE = 148, MS_CORR = 152 };
 enum : int { M_CPY_KIND, M_CPY_SRC, M_CPY_DST, M_SET_KIND, M_PID, M_TID, M_TS, M_DUR, M_ARGS, M_EXT, M_EXTC, M_FROMDEV, M_INDEV,
-             M_TODEV, M_FROMCTX, M_INCTX, M_TOCTX, M_DEV, M_CTX, M_STREAM, M_CORR, M_BYTES, M_BW, M_GRAPH, M_NODE, M_CHAN, M_CHTYPE,
+             M_TODEV, M_FROMCTX, M_INCTX, M_TOCTX, M_DEV, M_CTX, M_STREAM, M_CORR, M_BYTES, M_BW, M_BWRAW, M_GRAPH, M_NODE, M_CHAN, M_CHTYPE,
              M_CLOSE, M_FLOW, M_FPID, M_FTID, M_FTS, M_FEND, M_COUNT };
 #define K2J_MEM_FIELDS \
     {XHEAD("gpu_memcpy") "Memcpy ", T_CSTR, VK_U32, MS_KIND0}, {" (", T_CSTR, VK_U32, MS_KIND1}, {" -> ", T_CSTR, VK_U32, MS_KIND2}, \
@@ -1046,7 +1052,7 @@ enum : int { M_CPY_KIND, M_CPY_SRC, M_CPY_DST, M_SET_KIND, M_PID, M_TID, M_TS, M
     {", \"fromContext\": ", T_U64, VK_U32, MR_FROMCTX}, {", \"inContext\": ", T_U64, VK_U32, MR_CTX}, {", \"toContext\": ", T_U64, VK_U32, MR_TOCTX}, \
     {"\"device\": ", T_U64, VK_U32, MR_DEV}, {", \"context\": ", T_U64, VK_U32, MR_CTX}, \
     {", \"stream\": ", T_U64, VK_U32, MR_STREAM}, {", \"correlation\": ", T_U64, VK_U32, MS_CORR}, {", \"bytes\": ", T_U64, VK_64, MR_BYTES}, \
-    {", \"memory bandwidth (GB/s)\": ", T_DBL, VK_64, MS_BW}, \
+    {", \"memory bandwidth (GB/s)\": ", T_DEC, VK_64, MS_BW}, {", \"memory bandwidth (GB/s)\": ", T_DBL, VK_64, MS_BW}, \
     {", \"graph id\": ", T_U64, VK_U32, MS_GRAPH}, {", \"graph node id\": ", T_U64, VK_64, MS_NODE}, {", \"channel\": ", T_U64, VK_U32, MS_CHAN}, \
     {", \"channel_type\": ", T_U64, VK_U32, MS_CHTYPE}, \
     {"\n    }\n  },", T_NONE}, \
@@ -1610,19 +1616,37 @@ __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tal
   const int sm_count = have_dev ? d.props[dev].num_sms : 0;
   const float bps = sm_count == 0 ? __int_as_float(0x7f800000) : __fdiv_rn(__int2float_rn(grid_prod), __int2float_rn(sm_count));
   const float wps = __fdiv_rn(__fmul_rn(bps, __int2float_rn(block_prod)), 32.0f);
-  cudaOccResult occ;
-  float occupancy;
-  occupancy_metrics(d, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm, &occ, &occupancy);
-  s32(a, KS_PCT, (uint32_t)(int32_t)llround(__dmul_rn((double)occupancy, 100.0)));
-  s32(a, KS_ACTIVE, (uint32_t)occ.activeBlocksPerMultiprocessor); s32(a, KS_LIMIT, (uint32_t)(CS_LIMIT + (int)(occ.limitingFactors & 31u)));
-  s32(a, KS_LREGS, (uint32_t)occ.blockLimitRegs); s32(a, KS_LSMEM, (uint32_t)occ.blockLimitSharedMem);
-  s32(a, KS_LWARPS, (uint32_t)occ.blockLimitWarps); s32(a, KS_LBLOCKS, (uint32_t)occ.blockLimitBlocks);
-  s32(a, KS_LBARR, (uint32_t)occ.blockLimitBarriers); s32(a, KS_AREGS, (uint32_t)occ.allocatedRegistersPerBlock);
-  s64(a, KS_ASMEM, (uint64_t)occ.allocatedSharedMemPerBlock);
-  s64(a, KS_BPS, (uint64_t)__double_as_longlong((double)bps)); s64(a, KS_WPS, (uint64_t)__double_as_longlong((double)wps));
+  // The calculator's results and the digits of both doubles are worked out once, by the size pass: in the emit pass they
+  // took 61 of a kernel event's 456 warp instructions; 64 bytes written and read stand for them.
+  const uint64_t h = t.work - d.cls_begin[C_KERNEL];
+  uint4 o0, o1, o2;
+  uint64_t bps10, wps10;
+  if (counting) {
+    cudaOccResult occ;
+    float occupancy;
+    occupancy_metrics(d, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm, &occ, &occupancy);
+    const uint64_t asmem = (uint64_t)occ.allocatedSharedMemPerBlock;
+    o0 = make_uint4((uint32_t)(int32_t)llround(__dmul_rn((double)occupancy, 100.0)), (uint32_t)occ.activeBlocksPerMultiprocessor,
+                    (uint32_t)(CS_LIMIT + (int)(occ.limitingFactors & 31u)), (uint32_t)occ.blockLimitRegs);
+    o1 = make_uint4((uint32_t)occ.blockLimitSharedMem, (uint32_t)occ.blockLimitWarps, (uint32_t)occ.blockLimitBlocks, (uint32_t)occ.blockLimitBarriers);
+    o2 = make_uint4((uint32_t)occ.allocatedRegistersPerBlock, 0u, (uint32_t)asmem, (uint32_t)(asmem >> 32));
+    bps10 = pack_double((double)bps); wps10 = pack_double((double)wps);
+    d.hand_occ[h] = o0; d.hand_occ[d.hand_pitch + h] = o1; d.hand_occ[2 * d.hand_pitch + h] = o2;
+    d.hand_dec[h] = bps10; d.hand_wps[h] = wps10;
+  } else {
+    o0 = d.hand_occ[h]; o1 = d.hand_occ[d.hand_pitch + h]; o2 = d.hand_occ[2 * d.hand_pitch + h];
+    bps10 = d.hand_dec[h]; wps10 = d.hand_wps[h];
+  }
+  const bool packed = bps10 != 0ull && wps10 != 0ull;
+  s32(a, KS_PCT, o0.x); s32(a, KS_ACTIVE, o0.y); s32(a, KS_LIMIT, o0.z); s32(a, KS_LREGS, o0.w);
+  s32(a, KS_LSMEM, o1.x); s32(a, KS_LWARPS, o1.y); s32(a, KS_LBLOCKS, o1.z); s32(a, KS_LBARR, o1.w);
+  s32(a, KS_AREGS, o2.x); s64(a, KS_ASMEM, pack64(o2.z, o2.w));
+  s64(a, KS_BPS, packed ? bps10 : (uint64_t)__double_as_longlong((double)bps));
+  s64(a, KS_WPS, packed ? wps10 : (uint64_t)__double_as_longlong((double)wps));
   s64(a, KS_TS, (uint64_t)rel_ts(d, ts)); s64(a, KS_DUR, (uint64_t)(dur < 0 ? 0 : dur));
   s32(a, KS_REGS, regs); s32(a, KS_SMEM, (uint32_t)ssm + (uint32_t)dsm); s32(a, KS_EXT, (uint32_t)ext);
   uint64_t p = ((1ull << K_COUNT) - 1ull) & ~(1ull << K_COLL);  // every field except the optional ones below
+  p &= packed ? ~((1ull << K_BPSRAW) | (1ull << K_WPSRAW)) : ~((1ull << K_BPS) | (1ull << K_WPS));
   if (!has_ext) p &= ~((1ull << K_EXT) | (1ull << K_EXTC));
   else if (d.has_comms != nullptr && (*d.has_comms & 1u) != 0u) {
     // a kernel launched by a record_param_comms op carries that op's collective metadata (output_json.cpp:900-906)
@@ -1679,8 +1703,12 @@ __device__ __forceinline__ uint64_t gather_mem(const Dev& d, uint32_t* a, Tally&
   else { on(M_DEV); on(M_CTX); }
   on(M_STREAM); on(M_CORR); on(M_BYTES);
   if (dur != 0) {  // addBandwidthTypedMetadata, CuptiActivity.h:460-470
-    on(M_BW);
-    s64(a, MS_BW, (uint64_t)__double_as_longlong(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur))));
+    const uint64_t h = t.work - d.cls_begin[C_KERNEL];
+    uint64_t bw10;
+    if (counting) d.hand_dec[h] = bw10 = pack_double(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur)));
+    else bw10 = d.hand_dec[h];
+    on(bw10 != 0ull ? M_BW : M_BWRAW);
+    s64(a, MS_BW, bw10 != 0ull ? bw10 : (uint64_t)__double_as_longlong(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur))));
   }
   on(M_GRAPH); on(M_NODE); on(M_CHAN); on(M_CHTYPE); on(M_CLOSE);
   t.x++;
@@ -2071,6 +2099,7 @@ __device__ __forceinline__ void put_value(S& s, const Dev& d, int type, uint64_t
         if (COLL && coll && !double_is_finite(x)) put_nonfinite(s, x); else put_dbl(s, x);
         break;
       }
+      case T_DEC: put_packed_double(s, v); break;
       case T_NAME: put_name(s, d, (uint32_t)v, name_bytes); break;
       case T_CSTR: { const FieldDesc cs = g_fields.f[CSTR_BASE + (uint32_t)v]; s.words(g_fields.w + cs.off, cs.len); break; }
       case T_BOOL: if (v) s.put4(0x65757274u); else s.put64(0x65736C6166ull, 5); break;  // true / false
@@ -2136,6 +2165,7 @@ constexpr uint32_t value_max_bytes(int type, int vk) {
     case T_U64: return vk == VK_64 ? 20u : 10u;
     case T_I64: return vk == VK_64 ? 20u : 11u;
     case T_TS: return 24u;       // up to 20 digits, '.', three digits
+    case T_DEC: return 26u;
     case T_DBL: return 26u;      // 24 characters of a finite value; a non-finite one is shorter, in quotes
     case T_CSTR: return longest_constant_string();
     default: return 0xffffu;
@@ -2236,6 +2266,20 @@ __device__ __noinline__ uint64_t app_dbl(Win win, uint32_t pos, uint32_t carry, 
   put_dbl(s, __longlong_as_double((long long)bits));
   return sink_state(s);
 }
+__device__ __noinline__ uint64_t app_dec(Win win, uint32_t pos, uint32_t carry, uint64_t packed) {
+  WindowSink s = sink_at(win, pos, carry);
+  const uint64_t dec = packed & ((1ull << 57) - 1ull);
+  const uint32_t hi = (uint32_t)(dec / 1000000000ull), lo = (uint32_t)dec - hi * 1000000000u;  // below 10^8 and 10^9
+  const uint32_t h0 = hi / 1000000u, h = hi - h0 * 1000000u, h1 = h / 1000u, l0 = lo / 1000000u, l = lo - l0 * 1000000u, l1 = l / 1000u;
+  const uint64_t a = digits3(h1) & 0xffffffu, b = digits3(h - h1 * 1000u) & 0xffffffu, c = digits3(l0) & 0xffffffu, e = digits3(l1) & 0xffffffu,
+                 f = digits3(l - l1 * 1000u) & 0xffffffu;
+  Digits17 D;
+  D.x0 = ((digits3(h0) >> 8) & 0xffffu) | (a << 16) | (b << 40); D.x1 = c | (e << 24) | (f << 48); D.x2 = f >> 16;
+  const uint64_t n0 = D.x0 ^ 0x3030303030303030ull, n1 = D.x1 ^ 0x3030303030303030ull;
+  const int zeros = n0 != 0ull ? (__ffsll((long long)n0) - 1) >> 3 : n1 != 0ull ? 8 + ((__ffsll((long long)n1) - 1) >> 3) : 16;
+  put_placed(s, D, 17 - zeros, (int)(packed >> 57) - kPackedExp10);
+  return sink_state(s);
+}
 // A constant string of the field table by its index, which differs from lane to lane: from global memory (a constant-bank
 // load is repeated for every index in the warp).
 struct ConstString { uint64_t w[4]; uint64_t len; };
@@ -2271,7 +2315,8 @@ __device__ __noinline__ uint64_t app_cstr(Win win, uint32_t pos, uint32_t carry,
 // What a class prints, as ranges of its fields: fields that are always there, or those whose presence the first one's bit
 // tells.
 struct FieldRange { int first, last; bool always; };
-constexpr FieldRange kKernelRanges[] = {{K_HEAD, K_ARGS, true}, {K_EXT, K_EXTC, false}, {K_QUEUED, K_CHTYPE, true},
+constexpr FieldRange kKernelRanges[] = {{K_HEAD, K_ARGS, true}, {K_EXT, K_EXTC, false}, {K_QUEUED, K_SMEM, true}, {K_BPS, K_WPS, false},
+                                        {K_BPSRAW, K_WPSRAW, false}, {K_GX, K_CHTYPE, true},
                                         {K_CLOSE, K_CLOSE, true} /* K_COLL: the other launch's events */, {K_FLOW, K_FEND, false}};
 constexpr FieldRange kApiRanges[] = {{A_HEAD_RT, A_HEAD_RT, false}, {A_HEAD_DR, A_HEAD_DR, false}, {A_NAME, A_NAME, false},
                                      {A_INVALID, A_INVALID, false}, {A_PID, A_ARGS, true}, {A_EXT, A_EXTC, false}, {A_CBID, A_CLOSE, true},
@@ -2279,7 +2324,7 @@ constexpr FieldRange kApiRanges[] = {{A_HEAD_RT, A_HEAD_RT, false}, {A_HEAD_DR, 
                                      {A_FEND, A_FEND, false}};
 constexpr FieldRange kMemRanges[] = {{M_CPY_KIND, M_CPY_DST, false}, {M_SET_KIND, M_SET_KIND, false}, {M_PID, M_ARGS, true},
                                      {M_EXT, M_EXTC, false}, {M_FROMDEV, M_TOCTX, false}, {M_DEV, M_CTX, false}, {M_STREAM, M_BYTES, true},
-                                     {M_BW, M_BW, false}, {M_GRAPH, M_CLOSE, true}, {M_FLOW, M_FEND, false}};
+                                     {M_BW, M_BW, false}, {M_BWRAW, M_BWRAW, false}, {M_GRAPH, M_CLOSE, true}, {M_FLOW, M_FEND, false}};
 // (CPU-side activities with a duration; instant and counter events are the other launch's)
 constexpr FieldRange kOpRanges[] = {{O_CAT, O_CAT, true}, {O_NAME, O_NAME, true}, {O_PID, O_PAD, true}, {O_ARGS, O_ARGS, false},
                                     {O_EXT, O_EXT, false}, {O_EXTC, O_EXTC, false}, {O_MD, O_MD, false}, {P_ARGS_CLOSE, P_ARGS_CLOSE, false},
@@ -2375,6 +2420,7 @@ template <int R> __device__ __forceinline__ void put_run(WindowSink& s, const De
     uint64_t st;
     if constexpr (I::type == T_TS) st = app_ts(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
     else if constexpr (I::type == T_DBL) st = app_dbl(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
+    else if constexpr (I::type == T_DEC) st = app_dec(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
     else if constexpr (I::type == T_CSTR) st = app_cstr(s.win, s.pos, s.carry, a[w]);
     else if constexpr (I::type == T_U64 && I::vk == VK_64) st = app_u64(s.win, s.pos, s.carry, reinterpret_cast<const uint64_t*>(a)[u]);
     else if constexpr (I::type == T_I64 && I::vk == VK_64) st = app_i64(s.win, s.pos, s.carry, (int64_t)reinterpret_cast<const uint64_t*>(a)[u]);
