@@ -1219,9 +1219,11 @@ template <class S> __device__ __forceinline__ void put_name(S& s, const Dev& d, 
   put_pool_words(s, d.esc_name + esc_name_pos(d, id), len);
   *name_bytes += len;
 }
+template <bool ROOM> __device__ __forceinline__ void put_string(WindowSink& s, const uint64_t* w, uint32_t len);
 template <class S> __device__ __forceinline__ void put_mdstr(S& s, const Dev& d, uint32_t id) {
   if (id >= d.n_strings) { atomicAdd(&d.counters->device_check, 1ull); return; }
-  put_pool_words(s, d.esc_md + esc_md_pos(d, id), d.esc_md_len[id]);
+  if constexpr (S::kCounting) s.skip(d.esc_md_len[id]);
+  else put_string<false>(s, reinterpret_cast<const uint64_t*>(d.esc_md + esc_md_pos(d, id)), d.esc_md_len[id]);
 }
 
 __device__ __noinline__ int64_t tsc_convert(uint64_t t, uint64_t t0a, int64_t t0, uint64_t mant, int exp) {
@@ -2157,7 +2159,8 @@ constexpr uint32_t longest_constant_string() {  // among those a T_CSTR value ca
   for (int f = CSTR_BASE; f < CSTR_BASE + CS_HWC; f++) if ((uint32_t)c_strlen(kAllFields[f].lit) > m) m = (uint32_t)c_strlen(kAllFields[f].lit);
   return m;
 }
-// Most bytes a field's value can take; 0xffff for values of any length (names, metadata entries), which ask the
+constexpr uint32_t kNameWindowBytes = 64;  // most bytes of a name that go through a window (put_string)
+// Most bytes a field's value can take; 0xffff for values of any length (metadata entries), which ask the
 // sink for room themselves.
 constexpr uint32_t value_max_bytes(int type, int vk) {
   switch (type) {
@@ -2168,6 +2171,7 @@ constexpr uint32_t value_max_bytes(int type, int vk) {
     case T_DEC: return 26u;
     case T_DBL: return 26u;      // 24 characters of a finite value; a non-finite one is shorter, in quotes
     case T_CSTR: return longest_constant_string();
+    case T_NAME: return kNameWindowBytes;
     default: return 0xffffu;
   }
 }
@@ -2189,6 +2193,43 @@ __device__ __forceinline__ void count_fields(S& s, const Dev& d, const uint32_t*
     }
     count_fields<BASE, F + 1, NF>(s, d, a, present, name_bytes);
   }
+}
+// A sanitised pool string by its length: one or two words through the window where all strings of the warp are that short,
+// one 64-byte piece of it, else straight to the output (out of line; the sink's state goes there and back in registers,
+// `open` in the low bits of the 32-byte aligned address).  In 64-byte pieces through the window, a flush behind each, a
+// kernel name of 20 to 400 bytes took 58 of its event's 456 warp instructions; by the lanes of the warp together, half a
+// warp to a name, 77 (the copies are coalesced, but every piece is addressed anew).
+__device__ __noinline__ ulonglong2 app_long(Win win, uint32_t pos, uint32_t carry, uint64_t place, const uint64_t* w, uint32_t len) {
+  WindowSink s;
+  s.win = win; s.pos = pos; s.carry = carry; s.open = 8u * ((uint32_t)place & 7u); s.gbase = reinterpret_cast<uint8_t*>((uintptr_t)(place & ~31ull));
+  s.long_words(w, len);
+  return make_ulonglong2(pack64(s.pos, s.carry), (uint64_t)reinterpret_cast<uintptr_t>(s.gbase) | (s.open >> 3));
+}
+// ROOM: kNameWindowBytes are known to fit.
+template <bool ROOM> __device__ __forceinline__ void put_string(WindowSink& s, const uint64_t* w, uint32_t len) {
+  const uint32_t active = __activemask();
+  if (!__any_sync(active, len > 16u)) {
+    if (!ROOM) s.ensure(16);
+    const uint64_t x = len != 0u ? w[0] : 0ull, y = len > 8u ? w[1] : 0ull;
+    const uint32_t n = len < 8u ? len : 8u;
+    s.put64(n != 0u ? x & (~0ull >> (8u * (8u - n))) : 0ull, n);
+    if (len > 8u) s.put64(y & (~0ull >> (8u * (16u - len))), len - 8u);
+  } else if (!__any_sync(active, len > kNameWindowBytes)) {
+    if (!ROOM) s.ensure(kNameWindowBytes);
+    uint64_t x[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) x[k] = 8u * k < len ? w[k] : 0ull;
+    s.piece(x, len);
+  } else {
+    if (!ROOM) s.ensure(16);
+    const ulonglong2 r = app_long(s.win, s.pos, s.carry, (uint64_t)reinterpret_cast<uintptr_t>(s.gbase) | (s.open >> 3), w, len);
+    s.pos = (uint32_t)r.x; s.carry = (uint32_t)(r.x >> 32); s.open = 8u * ((uint32_t)r.y & 7u);
+    s.gbase = reinterpret_cast<uint8_t*>((uintptr_t)(r.y & ~31ull));
+  }
+}
+__device__ __forceinline__ void put_pool_name(WindowSink& s, const Dev& d, uint32_t id) {
+  if (id >= d.n_strings) { atomicAdd(&d.counters->device_check, 1ull); return; }
+  put_string<true>(s, reinterpret_cast<const uint64_t*>(d.esc_name + esc_name_pos(d, id)), d.esc_name_len[id]);
 }
 // Number formatting of the hot classes: one out-of-line copy of each formatter per kernel, so that a field costs a call
 // instead of a copy of the formatter (with the formatters inlined the kernel is bound by instruction fetch).  The sink travels in registers: window, position and open word in, position
@@ -2429,7 +2470,10 @@ template <int R> __device__ __forceinline__ void put_run(WindowSink& s, const De
       if (v < 1000u) { put_below_1000(s, v); st = sink_state(s); }
       else if constexpr (I::vk == VK_I32) st = app_i32(s.win, s.pos, s.carry, (int32_t)v);
       else st = app_u32(s.win, s.pos, s.carry, v);
-    } else {  // names, metadata entries: they ask the sink for room themselves
+    } else if constexpr (I::type == T_NAME) {
+      put_pool_name(s, d, a[w]);
+      st = sink_state(s);
+    } else {  // metadata entries: they ask the sink for room themselves
       put_value<WindowSink, false, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
       st = sink_state(s);
     }

@@ -16,6 +16,14 @@ K2J_HD uint32_t funnel_l(uint32_t lo, uint32_t hi, uint32_t s) {
   return s ? (hi << s) | (lo >> (32u - s)) : hi;
 #endif
 }
+// the 32 bits of (hi:lo) from bit s on, s in 0..31
+K2J_HD uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t s) {
+#if defined(__CUDA_ARCH__)
+  return __funnelshift_r(lo, hi, s);
+#else
+  return s ? (lo >> s) | (hi << (32u - s)) : lo;
+#endif
+}
 // one 256-bit store to a 32-byte aligned address
 K2J_HD void store32(uint8_t* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
 #if defined(__CUDA_ARCH__)
@@ -72,14 +80,29 @@ inline uint32_t win_ld(Win w, uint32_t k) { return w[k * (uint32_t)kWinStride]; 
 inline void win_st(Win w, uint32_t k, uint32_t v) { w[k * (uint32_t)kWinStride] = v; }
 inline Win win_from(Win w, uint32_t k) { return w + k * (uint32_t)kWinStride; }
 #endif
-K2J_HD void win_block_out(Win win, uint8_t* gbase, uint32_t b) {
+// the same as two 128-bit stores, for code out of line: in a function that was called, 256-bit stores left three quarters of
+// a block unwritten (ptxas 12.9; the same source in line is right)
+K2J_HD void store16x2(uint8_t* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+#if defined(__CUDA_ARCH__)
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a, b);
+  *reinterpret_cast<ulonglong2*>(p + 16) = make_ulonglong2(c, d);
+#else
+  uint64_t v[4] = {a, b, c, d};
+  memcpy(p, v, 32);
+#endif
+}
+template <bool WIDE> K2J_HD void store_block(uint8_t* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+  if (WIDE) store32(p, a, b, c, d); else store16x2(p, a, b, c, d);
+}
+template <bool WIDE> K2J_HD void win_block_out(Win win, uint8_t* gbase, uint32_t b) {
   const uint32_t k = 8u * b;
   const uint32_t x0 = win_ld(win, k), x1 = win_ld(win, k + 1), x2 = win_ld(win, k + 2), x3 = win_ld(win, k + 3), x4 = win_ld(win, k + 4),
                  x5 = win_ld(win, k + 5), x6 = win_ld(win, k + 6), x7 = win_ld(win, k + 7);
-  store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
+  store_block<WIDE>(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
 }
 // Writes the complete 32-byte blocks of a window to global memory and moves the open block to the front; returns their
 // number.  `open`: 0, or the offset of the first word that the first block has still to write (its earlier words are out).
+template <bool WIDE>
 K2J_HD uint32_t window_flush(Win win, uint32_t pos, uint32_t carry, uint8_t* gbase, uint32_t open) {
   win_st(win, pos >> 2, carry);
   const uint32_t nb = pos >> 5;
@@ -97,10 +120,10 @@ K2J_HD uint32_t window_flush(Win win, uint32_t pos, uint32_t carry, uint8_t* gba
                    x5 = win_ld(win, k + 5), x6 = win_ld(win, k + 6), x7 = win_ld(win, k + 7);
     const uint32_t y0 = win_ld(win, k + 8), y1 = win_ld(win, k + 9), y2 = win_ld(win, k + 10), y3 = win_ld(win, k + 11), y4 = win_ld(win, k + 12),
                    y5 = win_ld(win, k + 13), y6 = win_ld(win, k + 14), y7 = win_ld(win, k + 15);
-    store32(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
-    store32(gbase + 32u * b + 32u, pack64(y0, y1), pack64(y2, y3), pack64(y4, y5), pack64(y6, y7));
+    store_block<WIDE>(gbase + 32u * b, pack64(x0, x1), pack64(x2, x3), pack64(x4, x5), pack64(x6, x7));
+    store_block<WIDE>(gbase + 32u * b + 32u, pack64(y0, y1), pack64(y2, y3), pack64(y4, y5), pack64(y6, y7));
   }
-  if (b < nb) win_block_out(win, gbase, b);
+  if (b < nb) win_block_out<WIDE>(win, gbase, b);
   if (nb != 0u) {
     const uint32_t k = 8u * nb;
     const uint32_t x0 = win_ld(win, k), x1 = win_ld(win, k + 1), x2 = win_ld(win, k + 2), x3 = win_ld(win, k + 3), x4 = win_ld(win, k + 4),
@@ -129,8 +152,8 @@ struct WindowSink {
     else *reinterpret_cast<uint32_t*>(gbase + w0 + 4) = (uint32_t)(w >> 32);
   }
   // Writes the complete 32-byte blocks of the window to global memory and moves the open block to the front.
-  K2J_HD void flush() {
-    const uint32_t nb = window_flush(win, pos, carry, gbase, open);
+  template <bool WIDE = true> K2J_HD void flush() {
+    const uint32_t nb = window_flush<WIDE>(win, pos, carry, gbase, open);
     if (nb != 0u) open = 0u;
     gbase += 32u * nb; pos -= 32u * nb;
   }
@@ -153,6 +176,56 @@ struct WindowSink {
 #else
     if (pos + n + 8u > (uint32_t)kWinBytes) flush();
 #endif
+  }
+  // A long string from an 8-byte aligned word array (words up to one behind its last byte are readable): past the window,
+  // straight from registers to the output.  The bytes up to the output's next 8-byte boundary and those behind the last one
+  // go through the window.  For code out of line (see store16x2).
+  K2J_HD void long_words(const uint64_t* w, uint32_t len) {
+    uint32_t h = (0u - pos) & 7u;
+    h = h < len ? h : len;
+    uint64_t cur = len != 0u ? w[0] : 0ull;
+    put64(h != 0u ? cur & (~0ull >> (8u * (8u - h))) : 0ull, h);
+    uint32_t n = (len - h) >> 3;  // whole words of output
+    if (n != 0u) {
+      flush<false>();
+      for (uint32_t o = open; o < pos; o += 8u) *reinterpret_cast<uint64_t*>(gbase + o) = W64(o >> 2);
+      uint8_t* dst = gbase + pos;
+      const uint32_t odd = h & 4u, sh = 8u * (h & 3u);
+      auto shifted = [&](uint64_t x, uint64_t y) {  // the 8 bytes from byte h of (x, y) on
+        const uint32_t w0 = odd ? (uint32_t)(x >> 32) : (uint32_t)x, w1 = odd ? (uint32_t)y : (uint32_t)(x >> 32), w2 = odd ? (uint32_t)(y >> 32) : (uint32_t)y;
+        return pack64(funnel_r(w0, w1, sh), funnel_r(w1, w2, sh));
+      };
+      for (; n != 0u && (reinterpret_cast<uintptr_t>(dst) & 31u) != 0u; n--, dst += 8) {
+        const uint64_t y = *++w;
+        *reinterpret_cast<uint64_t*>(dst) = shifted(cur, y);
+        cur = y;
+      }
+      uint64_t y0 = 0, y1 = 0, y2 = 0, y3 = 0;
+      if (n >= 4u) { y0 = w[1]; y1 = w[2]; y2 = w[3]; y3 = w[4]; }
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+      for (; n >= 4u; n -= 4u, dst += 32) {  // the next block's words are on their way while this one is written
+        const uint64_t x0 = y0, x1 = y1, x2 = y2, x3 = y3;
+        w += 4;
+        if (n >= 8u) { y0 = w[1]; y1 = w[2]; y2 = w[3]; y3 = w[4]; }
+        store16x2(dst, shifted(cur, x0), shifted(x0, x1), shifted(x1, x2), shifted(x2, x3));
+        cur = x3;
+      }
+      for (; n != 0u; n--, dst += 8) {
+        const uint64_t y = *++w;
+        *reinterpret_cast<uint64_t*>(dst) = shifted(cur, y);
+        cur = y;
+      }
+      pos = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 31u); open = pos; carry = 0u;
+      gbase = dst - pos;
+    }
+    const uint32_t r = (len - h) & 7u;  // (h is below 8: cur holds the first of them)
+    if (r != 0u) {
+      const uint64_t y = h + r > 8u ? w[1] : 0ull;
+      const uint64_t x = (cur >> (8u * h)) | ((y << 1) << (63u - 8u * h));
+      put64(x & (~0ull >> (8u * (8u - r))), r);
+    }
   }
   // append the low `len` (0..4) bytes of w; bytes above len must be zero
   K2J_HD void put(uint32_t w, int len) {
@@ -193,6 +266,28 @@ struct WindowSink {
     for (int i = 0; i < N / 4; i++) put4(l.w[i]);
     if (N % 4) put(l.w[N / 4], N % 4);
   }
+  // the first n (at most 64) bytes of eight words; the caller has asked for the room
+  K2J_HD void piece(const uint64_t (&x)[8], uint32_t n) {
+    const uint32_t nw = n >> 3;
+    const uint32_t s = (pos & 3u) << 3;
+    uint32_t i = pos >> 2, c = carry;
+    uint64_t last = x[0];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (uint32_t k = 0; k < 8u; k++) {
+      if (k < nw) {
+        const uint32_t lo = (uint32_t)x[k], hi = (uint32_t)(x[k] >> 32);
+        win_st(win, i, c | (lo << s)); win_st(win, i + 1, funnel_l(lo, hi, s));
+        c = funnel_l(hi, 0u, s);
+        i += 2;
+      }
+      if (k == nw) last = x[k];
+    }
+    carry = c; pos += 8u * nw;
+    const uint32_t rem = n & 7u;
+    if (rem) put64(last & (~0ull >> (8u * (8u - rem))), rem);
+  }
   // `len` bytes from an 8-byte aligned word array, any length: 64 bytes at a time, asking for room first.  The
   // words of a piece are all loaded before the first one is appended: a load that waits behind the append of
   // the word before it (the compiler cannot move it across the window's stores) pays the memory latency once
@@ -216,25 +311,7 @@ struct WindowSink {
         for (uint32_t k = 0; k < 8u; k++) y[k] = k < touched ? w[8 + k] : 0ull;
       }
       ensure(n);
-      const uint32_t nw = n >> 3;
-      const uint32_t s = (pos & 3u) << 3;
-      uint32_t i = pos >> 2, c = carry;
-      uint64_t last = x[0];
-#if defined(__CUDA_ARCH__)
-#pragma unroll
-#endif
-      for (uint32_t k = 0; k < 8u; k++) {
-        if (k < nw) {
-          const uint32_t lo = (uint32_t)x[k], hi = (uint32_t)(x[k] >> 32);
-          win_st(win, i, c | (lo << s)); win_st(win, i + 1, funnel_l(lo, hi, s));
-          c = funnel_l(hi, 0u, s);
-          i += 2;
-        }
-        if (k == nw) last = x[k];
-      }
-      carry = c; pos += 8u * nw;
-      const uint32_t rem = n & 7u;
-      if (rem) put64(last & (~0ull >> (8u * (8u - rem))), rem);
+      piece(x, n);
       len -= n;
       if (len == 0u) break;
       w += 8;
