@@ -594,13 +594,8 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
 
   K2J_CUDA(c, cudaEventRecord(c->ev[0], s));
 
-  // ---- string pool: sanitised copies (once per pool) ----
-  if (c->strings_dirty && c->n_strings) {
-    const uint32_t blocks = (uint32_t)((c->n_strings * 32 + 255) / 256);
-    k_escape_pool<<<blocks, 256, 0, s>>>(d);
-    c->launches++;
-    c->strings_dirty = false;
-  }
+  // ---- string pool: sanitised copies (once per pool), by the first blocks of the segmentation's first launch ----
+  const uint32_t pool_blocks = c->strings_dirty ? (uint32_t)((c->n_strings + kSegWarps - 1) / kSegWarps) : 0u;
 
   // ---- segmentation ----
   const uint32_t nch = c->n_chunks;
@@ -617,7 +612,8 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     d.slot_code = c->slot_code.as<uint8_t>(); d.exit_map = c->exit_map.as<uint8_t>(); d.walk_cnt = c->walk_cnt.as<uint32_t>();
     d.chunk_entry = c->chunk_entry.as<uint8_t>(); d.chunk_cnt = c->chunk_cnt.as<uint32_t>();
     d.chunk_base = c->chunk_base.as<uint64_t>();
-    k_seg_chunks<<<seg_blocks, kSegWarps * 32, 0, s>>>(d);
+    k_seg_chunks<<<pool_blocks + seg_blocks, kSegWarps * 32, 0, s>>>(d, pool_blocks);
+    c->strings_dirty = false;
     k_seg_compose<<<c->n_buf, 256, 0, s>>>(d);
     c->launches += 2;
     K2J_CUDA(c, cudaGetLastError());
@@ -625,6 +621,11 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     if (st) return st;
     K2J_CUDA(c, cudaStreamSynchronize(s));
     for (int i = 0; i < C_NCOL; i++) totals[i] = c->h_totals[i];
+  } else if (pool_blocks) {
+    k_seg_chunks<<<pool_blocks, kSegWarps * 32, 0, s>>>(d, pool_blocks);
+    c->launches++;
+    c->strings_dirty = false;
+    K2J_CUDA(c, cudaGetLastError());
   }
 
   // ---- class-sorted work lists, compacted EXTERNAL_CORRELATION records ----

@@ -3,8 +3,7 @@
 // bandwidth (there is no dense contraction anywhere on this path).
 //
 // Data flow (one run):
-//   k_escape_pool    per distinct string: JSON-sanitised copies (name flavour, metadata flavour)
-//   k_seg_chunks     per 4 KiB chunk of every CUPTI buffer: record length per 8-byte slot, and for
+//   k_seg_chunks     per distinct string: JSON-sanitised copies (name flavour, metadata flavour); per 4 KiB chunk of every CUPTI buffer: record length per 8-byte slot, and for
 //                    each of the 26 possible entry slots the slot at which a walk leaves the chunk
 //                    and the records per class it meets
 //   k_seg_compose    per buffer: chains the exit maps -> true entry slot of every chunk -> its counts
@@ -288,8 +287,7 @@ __constant__ char g_coll_str[1 + kCollKeys][28] = {
     "Output Tensors start", "In split size", "Out split size", "Process Group Name", "Process Group Description",
     "Process Group Ranks", "Dst Rank", "Src Rank", "Seq", "Comms Id"};
 __constant__ uint8_t g_coll_len[1 + kCollKeys] = {18, 15, 13, 14, 10, 5, 19, 20, 13, 14, 18, 25, 19, 8, 8, 3, 8};
-__global__ void k_escape_pool(Dev d) {
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__device__ __forceinline__ void escape_pool(const Dev& d, uint32_t warp) {
   const uint32_t lane = threadIdx.x & 31;
   if (warp >= d.n_strings) return;
   const uint64_t b = d.pool_off[warp], e = d.pool_off[warp + 1];
@@ -386,7 +384,11 @@ __device__ __forceinline__ uint32_t code_class(uint32_t code) {
 // 244, 192 517 and 247, 512 (never) 561 and 260; at 32 long records keep walks apart (120 k nested operators 120-126 us,
 // else 118).
 constexpr uint32_t kMergeSlots = 96;
-__global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
+//
+// The string pool's sanitised copies have no part in this and are wanted only by the size pass; the first `pool_blocks`
+// blocks of the launch make them (as a launch in front of this one: segmentation of 150 launches 52 us, this way 45).
+__global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, uint32_t pool_blocks) {
+  if (blockIdx.x < pool_blocks) { escape_pool(d, (blockIdx.x * (kSegWarps * 32) + threadIdx.x) >> 5); return; }
   __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots];
   __shared__ uint32_t s_lead[kSegWarps * 32], s_rest[kSegWarps * 32][4], s_n_lead;  // walks that go on: chunk << 16 | slot; where they end, counts
   __shared__ uint16_t s_nvalid[kSegWarps];
@@ -407,7 +409,7 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d) {
   if (threadIdx.x == 0) s_n_lead = 0;
   __syncthreads();
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t chunk = blockIdx.x * kSegWarps + w;
+  const uint32_t chunk = (blockIdx.x - pool_blocks) * kSegWarps + w;
   const bool live = chunk < d.n_chunks;
   ChunkGeom g{0, 0, false};
   if (live) g = chunk_geom(d, chunk);
