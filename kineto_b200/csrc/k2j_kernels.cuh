@@ -2360,7 +2360,7 @@ __device__ __noinline__ uint64_t app_cstr(Win win, uint32_t pos, uint32_t carry,
 struct FieldRange { int first, last; bool always; };
 constexpr FieldRange kKernelRanges[] = {{K_HEAD, K_ARGS, true}, {K_EXT, K_EXTC, false}, {K_QUEUED, K_SMEM, true}, {K_BPS, K_WPS, false},
                                         {K_BPSRAW, K_WPSRAW, false}, {K_GX, K_CHTYPE, true},
-                                        {K_CLOSE, K_CLOSE, true} /* K_COLL: the other launch's events */, {K_FLOW, K_FEND, false}};
+                                        {K_COLL, K_COLL, false} /* in the launch for them only */, {K_CLOSE, K_CLOSE, true}, {K_FLOW, K_FEND, false}};
 constexpr FieldRange kApiRanges[] = {{A_HEAD_RT, A_HEAD_RT, false}, {A_HEAD_DR, A_HEAD_DR, false}, {A_NAME, A_NAME, false},
                                      {A_INVALID, A_INVALID, false}, {A_PID, A_ARGS, true}, {A_EXT, A_EXTC, false}, {A_CBID, A_CLOSE, true},
                                      {A_FLOW_S, A_FLOW_S, false}, {A_FLOW_F, A_FLOW_F, false}, {A_FPID, A_FCAT, false}, {A_FBP, A_FBP, false},
@@ -2443,7 +2443,7 @@ template <int R> struct RunLit {
       for (int i = 0; kAllFields[f].lit[i]; i++, p++) w[p / 4] |= (uint32_t)(unsigned char)kAllFields[f].lit[i] << (8 * (p % 4));
   }
 };
-template <int R> __device__ __forceinline__ void put_run(WindowSink& s, const Dev& d, const uint32_t* a, unsigned long long* name_bytes) {
+template <int R, bool COLL> __device__ __forceinline__ void put_run(WindowSink& s, const Dev& d, const uint32_t* a, unsigned long long* name_bytes) {
   using I = RunOf<R>;
   constexpr uint32_t n = I::len, nw = (n + 3) / 4, rem = n % 4;
   if constexpr (n != 0) {
@@ -2476,30 +2476,32 @@ template <int R> __device__ __forceinline__ void put_run(WindowSink& s, const De
       put_pool_name(s, d, a[w]);
       st = sink_state(s);
     } else {  // metadata entries: they ask the sink for room themselves
-      put_value<WindowSink, false, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
+      if constexpr (COLL || I::type != T_COLL) put_value<WindowSink, COLL, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
       st = sink_state(s);
     }
     s.pos = (uint32_t)st; s.carry = (uint32_t)(st >> 32);
   }
 }
-template <int R, int END>
+template <int R, int END, bool COLL>
 __device__ __forceinline__ void put_runs(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
   if constexpr (R < END) {
-    if constexpr (RunOf<R>::cond < 0) put_run<R>(s, d, a, name_bytes);
-    else if ((present >> RunOf<R>::cond) & 1ull) put_run<R>(s, d, a, name_bytes);
-    put_runs<R + 1, END>(s, d, a, present, name_bytes);
+    if constexpr (RunOf<R>::cond < 0) put_run<R, COLL>(s, d, a, name_bytes);
+    else if ((present >> RunOf<R>::cond) & 1ull) put_run<R, COLL>(s, d, a, name_bytes);
+    put_runs<R + 1, END, COLL>(s, d, a, present, name_bytes);
   }
 }
-template <int ST>
+template <int ST, bool COLL>
 __device__ __forceinline__ void put_step(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
-  if constexpr (ST < kNumSteps) put_runs<StepOf<ST>::first, StepOf<ST>::end>(s, d, a, present, name_bytes);
+  // (the launch for kernels with collective metadata holds the kernel class's code only)
+  if constexpr (ST < kNumSteps && (!COLL || ST < ClassSteps<0>::end)) put_runs<StepOf<ST>::first, StepOf<ST>::end, COLL>(s, d, a, present, name_bytes);
 }
+template <bool COLL>
 __device__ __forceinline__ void run_steps(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, int step, int end, unsigned long long* name_bytes) {
 #pragma unroll 1
   for (; step < end; step++) {
     s.room(kStepBytes);
     switch (step) {
-#define K2J_STEP(i) case i: put_step<i>(s, d, a, present, name_bytes); break;
+#define K2J_STEP(i) case i: put_step<i, COLL>(s, d, a, present, name_bytes); break;
 #define K2J_STEP8(i) K2J_STEP(i) K2J_STEP(i + 1) K2J_STEP(i + 2) K2J_STEP(i + 3) K2J_STEP(i + 4) K2J_STEP(i + 5) K2J_STEP(i + 6) K2J_STEP(i + 7)
       K2J_STEP8(0) K2J_STEP8(8) K2J_STEP8(16) K2J_STEP8(24) K2J_STEP8(32) K2J_STEP8(40)
 #undef K2J_STEP8
@@ -2555,8 +2557,10 @@ __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32
     const bool rare = (cls == C_KERNEL && ((p >> K_COLL) & 1ull) != 0) ||
                       (cls == C_OP && (p & ((1ull << I_HEAD) | (1ull << C_HEAD) | (1ull << H_ALL))) != 0);
     if (rare != COLL) return false;
-    if constexpr (COLL) run_fields<S, COLL>(s, d, a, base, p, nb);
-    else {
+    if constexpr (COLL) {
+      if (base == KERNEL_BASE) run_steps<COLL>(s, d, a, p, ClassSteps<0>::first, ClassSteps<0>::end, nb);
+      else run_fields<S, COLL>(s, d, a, base, p, nb);
+    } else {
       // the classes nearly all events belong to run compile-time field code; the others share the table-driven loop
       int step = -1, end = -1;
       if (base == API_BASE) { step = ClassSteps<1>::first; end = ClassSteps<1>::end; }
@@ -2564,7 +2568,7 @@ __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32
       else if (base == MEM_BASE) { step = ClassSteps<2>::first; end = ClassSteps<2>::end; }
       else if (cls == C_OP) { step = ClassSteps<3>::first; end = ClassSteps<3>::end; }
       if (step < 0) run_fields<S, COLL>(s, d, a, base, p, nb);
-      else if (p != 0ull) run_steps(s, d, a, p, step, end, nb);
+      else if (p != 0ull) run_steps<COLL>(s, d, a, p, step, end, nb);
     }
   }
   return true;
