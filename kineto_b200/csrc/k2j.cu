@@ -153,17 +153,16 @@ uint32_t pow2_at_least(uint64_t n) {
 }
 
 // Exclusive scan of `cols` columns of n u32 each (column stride n) into u64; totals land in
-// totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length.  Each line lies
-// where its shape still beats what stood for every length before, three launches and a copy of the total.  One column,
+// totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length.  One column,
 // us per call of k2j_exclusive_scan_u32 with its wait:
 //   elements                   200   4096   8192   12 288   16 384  |  tiles of 2048   4096   4097   6144   8192   16 384
 //   one launch                  16     19     21       25       27  |
 //   two launches                17     18     18       18       18  |                    66     69     93    121      244
 //   three launches                                                  |                    72     72     99    127      237
 //   three launches and a copy   27     27     27       28       31  |                    82     81
-// Among themselves the first two meet near 4096 elements (a block's serial rounds of 8192 against a launch), the last two
-// between 8192 and 16 384 tiles (sums that every block adds up again against a launch).
-constexpr uint64_t kScanSmallMax = 2 * kScanSmallTile;
+// One launch serves up to 4096 elements, where it meets two (a block's serial rounds of 8192 against a launch); the last
+// two meet between 8192 and 16 384 tiles (sums that every block adds up again against a launch).
+constexpr uint64_t kScanSmallMax = kScanSmallTile / 2;
 constexpr uint32_t kScanDirectBlocks = 4096;
 k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches,
                     const ScanReport& rep = ScanReport{}) {
@@ -614,7 +613,7 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     d.chunk_base = c->chunk_base.as<uint64_t>();
     k_seg_chunks<<<pool_blocks + seg_blocks, kSegWarps * 32, 0, s>>>(d, pool_blocks);
     c->strings_dirty = false;
-    k_seg_compose<<<c->n_buf, 256, 0, s>>>(d);
+    k_seg_compose<<<c->n_buf, kComposeThreads, 0, s>>>(d);
     c->launches += 2;
     K2J_CUDA(c, cudaGetLastError());
     k2j_status st = run_scan(c, d.chunk_cnt, nch, C_NCOL, d.chunk_base, c->h_totals, &c->launches);

@@ -500,7 +500,10 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, uint32_t p
 // three short phases instead of 1024 dependent steps: (A) for each of 32 segments of 32 chunks and each
 // possible entry, where a walk leaves the segment; (B) one thread chains the 32 segment maps;
 // (C) one lane per segment walks its 32 chunks from the segment's true entry.
-__global__ void __launch_bounds__(256) k_seg_compose(Dev d) {
+// A block to a buffer leaves most SMs idle, so the block is as wide as phase (A) and skips the segments that a short
+// buffer does not have.
+constexpr int kComposeThreads = 1024;
+__global__ void __launch_bounds__(kComposeThreads) k_seg_compose(Dev d) {
   constexpr int kTile = 1024, kSeg = 32;
   __shared__ uint8_t s_map[kTile * 32];
   __shared__ uint8_t s_ent[kTile];
@@ -516,14 +519,14 @@ __global__ void __launch_bounds__(256) k_seg_compose(Dev d) {
     return x >= kMaxEntry ? (uint32_t)kEntryNone : (uint32_t)x;
   };
   for (uint32_t t0 = c0; t0 < c1; t0 += kTile) {
-    const uint32_t n = min((uint32_t)kTile, c1 - t0);
+    const uint32_t n = min((uint32_t)kTile, c1 - t0), n_seg = (n + kSeg - 1) / kSeg;
     __syncthreads();
     const uint4* src = reinterpret_cast<const uint4*>(d.exit_map + (uint64_t)t0 * 32);
     uint4* dst = reinterpret_cast<uint4*>(s_map);
     for (uint32_t i = threadIdx.x; i < n * 2; i += blockDim.x) dst[i] = src[i];
     __syncthreads();
     // (A) 32 segments x 26 entries independent chains of 32 steps
-    for (uint32_t q = threadIdx.x; q < (kTile / kSeg) * 32; q += blockDim.x) {
+    for (uint32_t q = threadIdx.x; q < n_seg * 32; q += blockDim.x) {
       const uint32_t seg = q >> 5, e0 = q & 31u;
       uint32_t e = e0 < (uint32_t)kMaxEntry ? e0 : (uint32_t)kEntryNone;
       for (uint32_t c = seg * kSeg; c < (seg + 1) * kSeg; c++) e = step(e, c, n);
@@ -533,7 +536,7 @@ __global__ void __launch_bounds__(256) k_seg_compose(Dev d) {
     // (B) chain the segments
     if (threadIdx.x == 0) {
       uint32_t e = s_entry;
-      for (uint32_t seg = 0; seg < kTile / kSeg; seg++) {
+      for (uint32_t seg = 0; seg < n_seg; seg++) {
         s_segent[seg] = (uint8_t)e;
         if (e != kEntryNone) e = s_segmap[seg][e];
       }
@@ -541,7 +544,7 @@ __global__ void __launch_bounds__(256) k_seg_compose(Dev d) {
     }
     __syncthreads();
     // (C) entries of the chunks of each segment
-    if (threadIdx.x < kTile / kSeg) {
+    if (threadIdx.x < n_seg) {
       const uint32_t seg = threadIdx.x;
       uint32_t e = s_segent[seg];
       for (uint32_t c = seg * kSeg; c < (seg + 1) * kSeg; c++) { s_ent[c] = (uint8_t)e; e = step(e, c, n); }
