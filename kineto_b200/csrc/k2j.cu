@@ -69,9 +69,11 @@ struct k2j_ctx {
   DevBuf d_props;
   Input pool_off, pool_data, rt_names, dr_names, tid_pairs, cupti;
   Input op_start, op_end, op_id, op_device, op_resource, op_thread, op_type, op_name, op_flow, op_flowt, op_mdoff, op_md;
-  uint64_t n_strings = 0, n_ops = 0, n_md = 0, cupti_bytes = 0;
+  uint64_t n_strings = 0, n_ops = 0, cupti_bytes = 0;
   uint32_t n_rt = 0, n_dr = 0, n_tid = 0, n_buf = 0, n_chunks = 0;
   bool strings_dirty = true;
+  uint64_t pool_total = 0;        // bytes of the last pool whose size the host has learned
+  bool pool_unread = false;       // the pool is in device memory and its size is not known yet (k2j_set_strings)
   std::vector<uint64_t> h_buf_off, h_buf_valid;
   std::vector<uint32_t> h_buf_chunk_base;
   DevBuf d_buf_off, d_buf_valid, d_buf_chunk_base;
@@ -80,7 +82,7 @@ struct k2j_ctx {
   DevBuf ds_tab, span_key, span_nstart, span_end, span_nfirst, span_row, span_out, span_cnt, ann_size, ann_off;
   DevBuf sort_keys[2], sort_vals[2], sort_hist, sort_base, sort_rank;
   DevBuf tid_tab, corr_tab, user_tab, op_tab, work_slot, work_ev, ev_size, ev_off, ev_ext, hand, out, counters;
-  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans (23 and 27 are words of scan_totals, device memory: sort, filtered join keys)
+  uint64_t* h_totals = nullptr;   // pinned, 32 words: [0, C_NCOL) column totals, 20 text bytes, 21 bytes of CPU-op text, 22 annotation bytes, 24 scan entry point, 25 the record_param_comms flag, 26 kernel events with collective metadata, 28 user-annotation spans, 29 bytes of the string pool (23 and 27 are words of scan_totals, device memory: sort, filtered join keys)
   Counters* h_counters = nullptr; // pinned
   SpanRec* h_spans = nullptr;     // pinned, kPinnedSpans, behind h_totals in one allocation
   void* h_stage[2] = {nullptr, nullptr};            // pinned staging buffers of k2j_write_output
@@ -343,6 +345,27 @@ k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint3
   return K2J_OK;
 }
 
+// Workspaces of the sanitised copies: closed-form capacities of the two flavours (see esc_name_pos / esc_md_pos).
+k2j_status reserve_pool(k2j_ctx* c, uint64_t total) {
+  const uint64_t n = c->n_strings;
+  K2J_CUDA(c, c->esc_name.reserve(2 * total + 16 * (n + 1) + 16));
+  K2J_CUDA(c, c->esc_md.reserve(total + 8 * (n + 1) + 16));
+  K2J_CUDA(c, c->esc_name_len.reserve((n + 1) * 4));
+  K2J_CUDA(c, c->esc_md_len.reserve((n + 1) * 4));
+  K2J_CUDA(c, c->str_class.reserve(n + 1));
+  return K2J_OK;
+}
+// Bytes of a pool that the workspaces hold.
+uint64_t pool_room(const k2j_ctx* c) {
+  const uint64_t n = c->n_strings;
+  return std::min<uint64_t>((c->esc_name.cap - 16 * (n + 1) - 16) / 2, c->esc_md.cap - 8 * (n + 1) - 16);
+}
+void pool_pointers(const k2j_ctx* c, Dev& d) {
+  d.esc_name = c->esc_name.as<uint8_t>(); d.esc_md = c->esc_md.as<uint8_t>();
+  d.esc_name_len = c->esc_name_len.as<uint32_t>(); d.esc_md_len = c->esc_md_len.as<uint32_t>();
+  d.str_class = c->str_class.as<uint8_t>();
+}
+
 }  // namespace
 
 extern "C" {
@@ -455,22 +478,26 @@ k2j_status k2j_set_strings(k2j_ctx* c, const uint64_t* off, const uint8_t* data,
   K2J_CUDA(c, cudaSetDevice(c->device));
   c->n_strings = n;
   c->strings_dirty = true;
+  // A pool in device memory: its size is the last offset.  The context's workspaces are made for a pool as large as the one
+  // before, the segmentation's first launch reports the size, and only a larger pool is done over (a copy of eight bytes
+  // that the host waits for here, and one of four for the metadata entries in k2j_set_ops, cost every trace 28 us).
   uint64_t total = 0;
-  if (n > 0) {
-    if (is_device_ptr(off)) K2J_CUDA(c, cudaMemcpy(&total, off + n, 8, cudaMemcpyDeviceToHost));
-    else total = off[n];
+  c->pool_unread = n > 0 && c->pool_total > 0 && data && is_device_ptr(off) && is_device_ptr(data);
+  if (c->pool_unread) {
+    total = c->pool_total;
+    c->pool_off.dev = off; c->pool_data.dev = data;
+  } else {
+    if (n > 0) {
+      if (is_device_ptr(off)) K2J_CUDA(c, cudaMemcpy(&total, off + n, 8, cudaMemcpyDeviceToHost));
+      else total = off[n];
+    }
+    k2j_status st = stage(c, c->pool_off, off, (n + 1) * 8);
+    if (st) return st;
+    st = stage(c, c->pool_data, data, total);
+    if (st) return st;
+    c->pool_total = total;
   }
-  k2j_status st = stage(c, c->pool_off, off, (n + 1) * 8);
-  if (st) return st;
-  st = stage(c, c->pool_data, data, total);
-  if (st) return st;
-  // closed-form capacities of the two sanitised flavours (see esc_name_pos / esc_md_pos)
-  K2J_CUDA(c, c->esc_name.reserve(2 * total + 16 * (n + 1) + 16));
-  K2J_CUDA(c, c->esc_md.reserve(total + 8 * (n + 1) + 16));
-  K2J_CUDA(c, c->esc_name_len.reserve((n + 1) * 4));
-  K2J_CUDA(c, c->esc_md_len.reserve((n + 1) * 4));
-  K2J_CUDA(c, c->str_class.reserve(n + 1));
-  return K2J_OK;
+  return reserve_pool(c, total);
 }
 
 k2j_status k2j_set_cbid_names(k2j_ctx* c, const uint32_t* rt, uint32_t n_rt, const uint32_t* dr, uint32_t n_dr) {
@@ -502,21 +529,24 @@ k2j_status k2j_set_ops(k2j_ctx* c, const k2j_ops* o) {
   c->n_ops = n;
   c->n_guest_ops = 0;  // new rows: k2j_set_guest_ops says again which of them are guests
   uint64_t n_md = 0;
+  bool md_in_place = false;  // entries in device memory are used where they are: nobody asks how many there are
   if (n > 0) {
     if (!o->md_off) return fail(c, K2J_ERR_INVALID_ARGUMENT, "null md_off");
     uint32_t last = 0;
-    if (is_device_ptr(o->md_off)) K2J_CUDA(c, cudaMemcpy(&last, o->md_off + n, 4, cudaMemcpyDeviceToHost));
-    else last = o->md_off[n];
+    if (!is_device_ptr(o->md_off)) last = o->md_off[n];
+    else if (o->md && is_device_ptr(o->md)) md_in_place = true;
+    else K2J_CUDA(c, cudaMemcpy(&last, o->md_off + n, 4, cudaMemcpyDeviceToHost));
     n_md = last;
   }
-  c->n_md = n_md;
   k2j_status st;
 #define STAGE(field, src, bytes) if ((st = stage(c, c->field, src, bytes)) != K2J_OK) return st
   STAGE(op_start, o->start_ns, n * 8); STAGE(op_end, o->end_ns, n * 8); STAGE(op_id, o->id, n * 4);
   STAGE(op_device, o->device, n * 4); STAGE(op_resource, o->resource, n * 8); STAGE(op_thread, o->thread, n * 4);
   STAGE(op_type, o->type, n * 4);
   STAGE(op_name, o->name, n * 4); STAGE(op_flow, o->flow_id, n * 4); STAGE(op_flowt, o->flow_info, n);
-  STAGE(op_mdoff, o->md_off, n ? (n + 1) * 4 : 0); STAGE(op_md, o->md, n_md * sizeof(k2j_md_entry));
+  STAGE(op_mdoff, o->md_off, n ? (n + 1) * 4 : 0);
+  if (md_in_place) c->op_md.dev = o->md;
+  else STAGE(op_md, o->md, n_md * sizeof(k2j_md_entry));
 #undef STAGE
   return K2J_OK;
 }
@@ -572,9 +602,7 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
   d.conv_exp = c->params.conv_scale_exp;
   d.props = c->d_props.as<DevProps>();
   d.pool_off = (const uint64_t*)c->pool_off.dev; d.pool_data = (const uint8_t*)c->pool_data.dev; d.n_strings = (uint32_t)c->n_strings;
-  d.esc_name = c->esc_name.as<uint8_t>(); d.esc_md = c->esc_md.as<uint8_t>();
-  d.esc_name_len = c->esc_name_len.as<uint32_t>(); d.esc_md_len = c->esc_md_len.as<uint32_t>();
-  d.str_class = c->str_class.as<uint8_t>();
+  pool_pointers(c, d);
   d.rt_names = (const uint32_t*)c->rt_names.dev; d.n_rt = c->n_rt; d.dr_names = (const uint32_t*)c->dr_names.dev; d.n_dr = c->n_dr;
   d.tid_pairs = (const int32_t*)c->tid_pairs.dev; d.n_tid_pairs = c->n_tid;
   d.cupti = (const uint8_t*)c->cupti.dev; d.cupti_bytes = c->cupti_bytes;
@@ -594,7 +622,12 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
   K2J_CUDA(c, cudaEventRecord(c->ev[0], s));
 
   // ---- string pool: sanitised copies (once per pool), by the first blocks of the segmentation's first launch ----
-  const uint32_t pool_blocks = c->strings_dirty ? (uint32_t)((c->n_strings + kSegWarps - 1) / kSegWarps) : 0u;
+  PoolJob pool{};
+  if (c->strings_dirty && c->n_strings) {
+    pool.blocks = (uint32_t)((c->n_strings + kSegWarps - 1) / kSegWarps);
+    pool.room = pool_room(c);
+    if (c->pool_unread) pool.total = c->h_totals + 29;
+  }
 
   // ---- segmentation ----
   const uint32_t nch = c->n_chunks;
@@ -611,8 +644,7 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     d.slot_code = c->slot_code.as<uint8_t>(); d.exit_map = c->exit_map.as<uint8_t>(); d.walk_cnt = c->walk_cnt.as<uint32_t>();
     d.chunk_entry = c->chunk_entry.as<uint8_t>(); d.chunk_cnt = c->chunk_cnt.as<uint32_t>();
     d.chunk_base = c->chunk_base.as<uint64_t>();
-    k_seg_chunks<<<pool_blocks + seg_blocks, kSegWarps * 32, 0, s>>>(d, pool_blocks);
-    c->strings_dirty = false;
+    k_seg_chunks<<<pool.blocks + seg_blocks, kSegWarps * 32, 0, s>>>(d, pool);
     k_seg_compose<<<c->n_buf, kComposeThreads, 0, s>>>(d);
     c->launches += 2;
     K2J_CUDA(c, cudaGetLastError());
@@ -620,12 +652,26 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     if (st) return st;
     K2J_CUDA(c, cudaStreamSynchronize(s));
     for (int i = 0; i < C_NCOL; i++) totals[i] = c->h_totals[i];
-  } else if (pool_blocks) {
-    k_seg_chunks<<<pool_blocks, kSegWarps * 32, 0, s>>>(d, pool_blocks);
+  } else if (pool.blocks) {
+    k_seg_chunks<<<pool.blocks, kSegWarps * 32, 0, s>>>(d, pool);
     c->launches++;
-    c->strings_dirty = false;
     K2J_CUDA(c, cudaGetLastError());
+    if (pool.total) K2J_CUDA(c, cudaStreamSynchronize(s));
   }
+  if (pool.total) {  // the pool's size has arrived with the synchronisation above
+    c->pool_total = c->h_totals[29];
+    c->pool_unread = false;
+    if (c->pool_total > pool.room) {
+      k2j_status st = reserve_pool(c, c->pool_total);
+      if (st) return st;
+      pool_pointers(c, d);
+      pool.room = pool_room(c); pool.total = nullptr;
+      k_seg_chunks<<<pool.blocks, kSegWarps * 32, 0, s>>>(d, pool);
+      c->launches++;
+      K2J_CUDA(c, cudaGetLastError());
+    }
+  }
+  c->strings_dirty = false;
 
   // ---- class-sorted work lists, compacted EXTERNAL_CORRELATION records ----
   uint64_t pos = 0;

@@ -287,10 +287,15 @@ __constant__ char g_coll_str[1 + kCollKeys][28] = {
     "Output Tensors start", "In split size", "Out split size", "Process Group Name", "Process Group Description",
     "Process Group Ranks", "Dst Rank", "Src Rank", "Seq", "Comms Id"};
 __constant__ uint8_t g_coll_len[1 + kCollKeys] = {18, 15, 13, 14, 10, 5, 19, 20, 13, 14, 18, 25, 19, 8, 8, 3, 8};
-__device__ __forceinline__ void escape_pool(const Dev& d, uint32_t warp) {
+// blocks: of the launch, in front of the others.  room: bytes of a pool that the copies' workspaces hold; strings that end
+// behind it are left out.  total: where the pool's size is reported (pinned host memory), or nullptr.
+struct PoolJob { uint32_t blocks; uint64_t room; uint64_t* total; };
+__device__ __forceinline__ void escape_pool(const Dev& d, const PoolJob& job, uint32_t warp) {
   const uint32_t lane = threadIdx.x & 31;
   if (warp >= d.n_strings) return;
+  if (warp == 0 && lane == 0 && job.total != nullptr) *job.total = d.pool_off[d.n_strings];
   const uint64_t b = d.pool_off[warp], e = d.pool_off[warp + 1];
+  if (e > job.room) return;
   const uint32_t len = (uint32_t)(e - b);
   const uint8_t* src = d.pool_data + b;
   uint8_t* dn = d.esc_name + esc_name_pos(d, warp);
@@ -385,10 +390,10 @@ __device__ __forceinline__ uint32_t code_class(uint32_t code) {
 // else 118).
 constexpr uint32_t kMergeSlots = 96;
 //
-// The string pool's sanitised copies have no part in this and are wanted only by the size pass; the first `pool_blocks`
-// blocks of the launch make them (as a launch in front of this one: segmentation of 150 launches 52 us, this way 45).
-__global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, uint32_t pool_blocks) {
-  if (blockIdx.x < pool_blocks) { escape_pool(d, (blockIdx.x * (kSegWarps * 32) + threadIdx.x) >> 5); return; }
+// The string pool's sanitised copies have no part in this and are wanted only by the size pass; the first blocks
+// of the launch make them (as a launch in front of this one: segmentation of 150 launches 52 us, this way 45).
+__global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, PoolJob pool) {
+  if (blockIdx.x < pool.blocks) { escape_pool(d, pool, (blockIdx.x * (kSegWarps * 32) + threadIdx.x) >> 5); return; }
   __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots];
   __shared__ uint32_t s_lead[kSegWarps * 32], s_rest[kSegWarps * 32][4], s_n_lead;  // walks that go on: chunk << 16 | slot; where they end, counts
   __shared__ uint16_t s_nvalid[kSegWarps];
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, uint32_t p
   if (threadIdx.x == 0) s_n_lead = 0;
   __syncthreads();
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t chunk = (blockIdx.x - pool_blocks) * kSegWarps + w;
+  const uint32_t chunk = (blockIdx.x - pool.blocks) * kSegWarps + w;
   const bool live = chunk < d.n_chunks;
   ChunkGeom g{0, 0, false};
   if (live) g = chunk_geom(d, chunk);
