@@ -180,14 +180,14 @@ struct WindowSink {
   // A long string from an 8-byte aligned word array (words up to one behind its last byte are readable): past the window,
   // straight from registers to the output.  The bytes up to the output's next 8-byte boundary and those behind the last one
   // go through the window.  For code out of line (see store16x2).
-  K2J_HD void long_words(const uint64_t* w, uint32_t len) {
+  template <bool WIDE = false> K2J_HD void long_words(const uint64_t* w, uint32_t len) {
     uint32_t h = (0u - pos) & 7u;
     h = h < len ? h : len;
     uint64_t cur = len != 0u ? w[0] : 0ull;
     put64(h != 0u ? cur & (~0ull >> (8u * (8u - h))) : 0ull, h);
     uint32_t n = (len - h) >> 3;  // whole words of output
     if (n != 0u) {
-      flush<false>();
+      flush<WIDE>();
       for (uint32_t o = open; o < pos; o += 8u) *reinterpret_cast<uint64_t*>(gbase + o) = W64(o >> 2);
       uint8_t* dst = gbase + pos;
       const uint32_t odd = h & 4u, sh = 8u * (h & 3u);
@@ -200,17 +200,33 @@ struct WindowSink {
         *reinterpret_cast<uint64_t*>(dst) = shifted(cur, y);
         cur = y;
       }
-      uint64_t y0 = 0, y1 = 0, y2 = 0, y3 = 0;
-      if (n >= 4u) { y0 = w[1]; y1 = w[2]; y2 = w[3]; y3 = w[4]; }
+      uint64_t y[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+      for (uint32_t k = 0; k < 8u; k++) if (k < (n & ~3u)) y[k] = w[k + 1u];
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
-      for (; n >= 4u; n -= 4u, dst += 32) {  // the next block's words are on their way while this one is written
-        const uint64_t x0 = y0, x1 = y1, x2 = y2, x3 = y3;
-        w += 4;
-        if (n >= 8u) { y0 = w[1]; y1 = w[2]; y2 = w[3]; y3 = w[4]; }
-        store16x2(dst, shifted(cur, x0), shifted(x0, x1), shifted(x1, x2), shifted(x2, x3));
-        cur = x3;
+      while (n >= 4u) {  // two blocks a round; the next round's words are on their way while these are written
+        uint64_t x[8];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (uint32_t k = 0; k < 8u; k++) x[k] = y[k];
+        const uint32_t m = n >= 8u ? 8u : 4u;
+        w += m; n -= m;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (uint32_t k = 0; k < 8u; k++) if (k < (n & ~3u)) y[k] = w[k + 1u];
+        store_block<WIDE>(dst, shifted(cur, x[0]), shifted(x[0], x[1]), shifted(x[1], x[2]), shifted(x[2], x[3]));
+        cur = x[3];
+        if (m == 8u) {
+          store_block<WIDE>(dst + 32, shifted(cur, x[4]), shifted(x[4], x[5]), shifted(x[5], x[6]), shifted(x[6], x[7]));
+          cur = x[7];
+        }
+        dst += 8u * m;
       }
       for (; n != 0u; n--, dst += 8) {
         const uint64_t y = *++w;
