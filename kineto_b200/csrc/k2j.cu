@@ -283,8 +283,8 @@ k2j_status sort_gpu_events(k2j_ctx* c, uint64_t n) {
   return K2J_OK;
 }
 
-// The span table as a list on the host (no order), after a stream synchronisation that followed k_span_collect: the
-// kernel puts the first kPinnedSpans of them into pinned memory, so that a trace with few spans pays no copy for them.
+// The span table as a list on the host, after a stream synchronisation that followed k_span_collect and k_span_order: up
+// to kPinnedSpans of them are in pinned memory, ordered; a longer list is copied as it is.
 constexpr uint32_t kPinnedSpans = 4096;
 k2j_status take_spans(k2j_ctx* c, std::vector<SpanRec>* spans) {
   const uint32_t n = (uint32_t)c->h_totals[28];
@@ -312,9 +312,10 @@ k2j_status size_annotations(k2j_ctx* c, const std::vector<SpanRec>& spans, uint3
   // trace of 10 annotations over 256 streams holds 2 560 of them.
   std::vector<const SpanRec*> by_use(listed);
   for (unsigned int i = 0; i < listed; i++) by_use[i] = &spans[i];
-  std::sort(by_use.begin(), by_use.end(), [](const SpanRec* a, const SpanRec* b) {
+  const auto earlier = [](const SpanRec* a, const SpanRec* b) {
     return a->device != b->device ? a->device < b->device : a->stream != b->stream ? a->stream < b->stream : a->first_event < b->first_event;
-  });
+  };
+  if (!std::is_sorted(by_use.begin(), by_use.end(), earlier)) std::sort(by_use.begin(), by_use.end(), earlier);  // (ordered by the GPU as a rule)
   std::vector<SpanRec> room;
   SpanRec* ordered = c->h_spans;  // (the spans were copied out of it)
   if (listed > kPinnedSpans) { room.resize(listed); ordered = room.data(); }
@@ -1233,8 +1234,9 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
     if (d.has_comms) { rep.flag = d.has_comms; rep.flag_dst = c->h_totals + 25; }
     if (d.coll_list) { rep.count = &d.counters->n_coll; rep.count_dst = c->h_totals + 26; }
     if (spans_on) {  // the span table is complete: the host has the list when it learns the text's size
-      k_span_collect<<<(span_cap + 255) / 256, 256, 0, s>>>(d, c->span_out.as<SpanRec>(), c->span_cnt.as<unsigned long long>(), c->h_spans, kPinnedSpans);
-      c->launches++;
+      k_span_collect<<<(span_cap + 255) / 256, 256, 0, s>>>(d, c->span_out.as<SpanRec>(), c->span_cnt.as<unsigned long long>());
+      k_span_order<<<(std::min(span_cap, kPinnedSpans) + 7) / 8, 256, 0, s>>>(c->span_out.as<SpanRec>(), c->span_cnt.as<unsigned long long>(), c->h_spans, kPinnedSpans);
+      c->launches += 2;
       rep.spans = c->span_cnt.as<unsigned long long>(); rep.spans_dst = c->h_totals + 28;
     }
     k2j_status st = run_scan(c, d.ev_size, d.n_events, 1, c->ev_off.as<uint64_t>(), c->h_totals + 20, &c->launches, rep);
