@@ -148,6 +148,18 @@ k2j_status stage(k2j_ctx* c, Input& in, const void* src, size_t bytes) {
   return K2J_OK;
 }
 
+// A launch whose blocks may take their places while the kernel in front of it ends (that kernel lets it start, this one waits
+// for it: see wait_for_previous).
+template <class... P, class... A>
+void launch_behind(void (*kernel)(P...), dim3 grid, int threads, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.stream = s; cfg.attrs = &at; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // (an error is picked up by the caller's cudaGetLastError)
+}
+
 uint32_t pow2_at_least(uint64_t n) {
   uint32_t p = 16;
   while (p < n && p < (1u << 31)) p <<= 1;
@@ -169,7 +181,7 @@ constexpr uint32_t kScanDirectBlocks = 4096;
 k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches,
                     const ScanReport& rep = ScanReport{}) {
   if (n <= kScanSmallMax) {
-    k_scan_small<<<cols, kScanSmallThreads, 0, c->stream>>>(in, n, totals, out, rep);
+    launch_behind(k_scan_small, dim3(cols), kScanSmallThreads, c->stream, in, n, totals, out, rep);
     *launches += 1;
     K2J_CUDA(c, cudaGetLastError());
     return K2J_OK;
@@ -177,8 +189,8 @@ k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, u
   const uint32_t nb = (uint32_t)((n + kScanTile - 1) / kScanTile);
   K2J_CUDA(c, c->scan_sums.reserve((size_t)nb * cols * 8));
   uint64_t* sums = c->scan_sums.as<uint64_t>();
-  k_scan_reduce<<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb);
-  if (nb <= kScanDirectBlocks) k_scan_apply<true><<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb, out, totals, rep);
+  launch_behind(k_scan_reduce, dim3(nb, cols), kScanThreads, c->stream, in, n, n, sums, nb);
+  if (nb <= kScanDirectBlocks) launch_behind(k_scan_apply<true>, dim3(nb, cols), kScanThreads, c->stream, in, n, n, sums, nb, out, totals, rep);
   else {
     k_scan_sums<<<cols, kScanThreads, 0, c->stream>>>(sums, nb, totals);
     k_scan_apply<false><<<dim3(nb, cols), kScanThreads, 0, c->stream>>>(in, n, n, sums, nb, out, nullptr, rep);
@@ -646,7 +658,7 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
     d.chunk_entry = c->chunk_entry.as<uint8_t>(); d.chunk_cnt = c->chunk_cnt.as<uint32_t>();
     d.chunk_base = c->chunk_base.as<uint64_t>();
     k_seg_chunks<<<pool.blocks + seg_blocks, kSegWarps * 32, 0, s>>>(d, pool);
-    k_seg_compose<<<c->n_buf, kComposeThreads, 0, s>>>(d);
+    launch_behind(k_seg_compose, dim3(c->n_buf), kComposeThreads, s, d);
     c->launches += 2;
     K2J_CUDA(c, cudaGetLastError());
     k2j_status st = run_scan(c, d.chunk_cnt, nch, C_NCOL, d.chunk_base, c->h_totals, &c->launches);
@@ -1195,12 +1207,12 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
                                      ops ? jobs.ops_last - jobs.ops_first : 0, others ? d.n_ext_all : 0};
     uint32_t blocks = 0;
     for (int k = 0; k < J_COUNT; k++) jobs.end[k] = blocks += (uint32_t)((items[k] + kJoinThreads - 1) / kJoinThreads);
-    if (blocks) { k_build_join<<<blocks, kJoinThreads, 0, s>>>(d, jobs); c->launches++; }
+    if (blocks) { launch_behind(k_build_join, dim3(blocks), kJoinThreads, s, d, jobs); c->launches++; }
   };
   // with a filter the ops job asks which ids the correlation records name, so it waits for them
   launch_join(!filter, true);
   if (filter) launch_join(true, false);
-  if (d.n_ext_all) { k_resolve_corr<<<(corr_cap + 255) / 256, 256, 0, s>>>(d); c->launches++; }
+  if (d.n_ext_all) { launch_behind(k_resolve_corr, dim3((corr_cap + 255) / 256), 256, s, d); c->launches++; }
   K2J_CUDA(c, cudaGetLastError());
   K2J_CUDA(c, cudaEventRecord(c->ev[2], s));
 

@@ -366,6 +366,11 @@ __device__ __forceinline__ ChunkGeom chunk_geom(const Dev& d, uint32_t chunk) {
   return g;
 }
 
+// Kernels of a chain that the host launches back to back (launch_behind): a kernel lets the next one's blocks take their
+// places once its own all have theirs, and that one waits for the whole of it before it touches memory.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 constexpr int kSegWarps = 8;
 
 // Class column of a slot code for the count matrix (C_EXT_USER counts as C_EXT; see C_USER).
@@ -392,6 +397,7 @@ constexpr uint32_t kMergeSlots = 96;
 // The string pool's sanitised copies have no part in this and are wanted only by the size pass; the first blocks
 // of the launch make them (as a launch in front of this one: segmentation of 150 launches 52 us, this way 45).
 __global__ void __launch_bounds__(kSegWarps * 32) k_seg_chunks(Dev d, PoolJob pool) {
+  let_next_start();
   if (blockIdx.x < pool.blocks) { escape_pool(d, pool, (blockIdx.x * (kSegWarps * 32) + threadIdx.x) >> 5); return; }
   __shared__ __align__(4) uint8_t s_code[kSegWarps][kChunkSlots];
   __shared__ uint32_t s_lead[kSegWarps * 32], s_rest[kSegWarps * 32][4], s_n_lead;  // walks that go on: chunk << 16 | slot; where they end, counts
@@ -514,6 +520,8 @@ __global__ void __launch_bounds__(kComposeThreads) k_seg_compose(Dev d) {
   __shared__ uint8_t s_segmap[kTile / kSeg][32];
   __shared__ uint8_t s_segent[kTile / kSeg];
   __shared__ uint32_t s_entry;
+  let_next_start();
+  wait_for_previous();
   const uint32_t b = blockIdx.x;
   const uint32_t c0 = d.buf_chunk_base[b], c1 = d.buf_chunk_base[b + 1];
   if (threadIdx.x == 0) s_entry = 0;
@@ -790,6 +798,8 @@ struct JoinJobs {
   uint32_t* comms_flag;
 };
 __global__ void __launch_bounds__(kJoinThreads) k_build_join(Dev d, JoinJobs j) {
+  let_next_start();
+  wait_for_previous();
   const uint32_t b = blockIdx.x;
   auto at = [&](uint32_t first) { return (uint64_t)(b - first) * kJoinThreads + threadIdx.x; };
   if (b < j.end[J_TIDS]) build_tids(d, at(0u));
@@ -809,6 +819,7 @@ struct ClearList {
   }
 };
 __global__ void __launch_bounds__(kClearThreads) k_clear(const __grid_constant__ ClearList l) {
+  let_next_start();
   const uint64_t first = (uint64_t)blockIdx.x * kClearThreads + threadIdx.x, step = (uint64_t)gridDim.x * kClearThreads;
   for (uint32_t k = 0; k < l.n; k++) {
     const uint32_t x = (l.ones >> k) & 1u ? 0xFFFFFFFFu : 0u;
@@ -876,6 +887,7 @@ __device__ __forceinline__ void scan_store(uint64_t* dst, uint64_t base, uint64_
 }
 
 __global__ void __launch_bounds__(kScanSmallThreads) k_scan_small(const uint32_t* in, uint64_t n, uint64_t* totals, uint64_t* out, ScanReport rep) {
+  wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.x * n;
   uint64_t* dst = out + (uint64_t)blockIdx.x * n;
   uint64_t carry = 0;
@@ -892,6 +904,8 @@ __global__ void __launch_bounds__(kScanSmallThreads) k_scan_small(const uint32_t
   if (threadIdx.x == 0) { totals[blockIdx.x] = carry; scan_report(rep); }
 }
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* in, uint64_t n, uint64_t col_stride, uint64_t* block_sums, uint32_t n_blocks) {
+  let_next_start();
+  wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.y * col_stride;
   const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
   uint64_t s = 0;
@@ -925,6 +939,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint64_t* block_sums
 template <bool DIRECT>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint64_t n, uint64_t col_stride, const uint64_t* block_sums, uint32_t n_blocks,
                                                              uint64_t* out, uint64_t* totals, ScanReport rep) {
+  wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.y * col_stride;
   uint64_t* dst = out + (uint64_t)blockIdx.y * col_stride;
   const uint64_t* sums = block_sums + (uint64_t)blockIdx.y * n_blocks;
@@ -1279,6 +1294,7 @@ __global__ void k_op_id_bits(Dev d, int64_t min_id, uint64_t n_bits, uint32_t* b
   atomicOr(&bits[k >> 5], 1u << (k & 31));
 }
 __global__ void k_resolve_corr(Dev d) {
+  wait_for_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0u && d.corr0[0] != 0ull) {  // correlation id 0
     ExtRec z; ext_at(d, d.corr0[0] - 1ull, &z);
