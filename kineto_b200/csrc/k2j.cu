@@ -232,14 +232,13 @@ k2j_status sort_passes(k2j_ctx* c, uint64_t n, int passes, int* cur_io) {
   const uint32_t tiles = sort_tiles(n);
   int cur = *cur_io;
   for (int pass = 0; pass < passes; pass++) {
-    k_rs_hist<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), n, sort_rounds(n), 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
+    launch_behind(k_rs_hist, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), n, sort_rounds(n), 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
     c->launches++;
     k2j_status st = run_scan(c, c->sort_hist.as<uint32_t>(), (uint64_t)tiles * 256, 1, c->sort_base.as<uint64_t>(),
                              c->scan_totals.as<uint64_t>() + 23, &c->launches);
     if (st) return st;
-    k_rs_scatter<<<tiles, kSortThreads, 0, s>>>(c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, sort_rounds(n), 8 * pass,
-                                                c->sort_base.as<uint64_t>(), tiles, c->sort_keys[cur ^ 1].as<uint64_t>(),
-                                                c->sort_vals[cur ^ 1].as<uint32_t>());
+    launch_behind(k_rs_scatter, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, sort_rounds(n),
+                  8 * pass, c->sort_base.as<uint64_t>(), tiles, c->sort_keys[cur ^ 1].as<uint64_t>(), c->sort_vals[cur ^ 1].as<uint32_t>());
     c->launches++;
     cur ^= 1;
   }
@@ -288,8 +287,8 @@ k2j_status sort_gpu_events(k2j_ctx* c, uint64_t n) {
   c->launches++;
   int cur = 0;
   if ((st0 = sort_passes(c, n, passes, &cur))) return st0;
-  k_rs_invert<<<(uint32_t)((n + 255) / 256), 256, 0, s>>>(c->sort_vals[cur].as<uint32_t>(), n, c->sort_rank.as<uint32_t>());
-  k_sort_remap<<<wl_blocks, 256, 0, s>>>(d, c->sort_rank.as<uint32_t>());
+  launch_behind(k_rs_invert, dim3((uint32_t)((n + 255) / 256)), 256, s, c->sort_vals[cur].as<uint32_t>(), n, c->sort_rank.as<uint32_t>());
+  launch_behind(k_sort_remap, dim3(wl_blocks), 256, s, d, c->sort_rank.as<uint32_t>());
   c->launches += 2;
   K2J_CUDA(c, cudaGetLastError());
   return K2J_OK;

@@ -887,6 +887,7 @@ __device__ __forceinline__ void scan_store(uint64_t* dst, uint64_t base, uint64_
 }
 
 __global__ void __launch_bounds__(kScanSmallThreads) k_scan_small(const uint32_t* in, uint64_t n, uint64_t* totals, uint64_t* out, ScanReport rep) {
+  let_next_start();
   wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.x * n;
   uint64_t* dst = out + (uint64_t)blockIdx.x * n;
@@ -939,6 +940,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(uint64_t* block_sums
 template <bool DIRECT>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* in, uint64_t n, uint64_t col_stride, const uint64_t* block_sums, uint32_t n_blocks,
                                                              uint64_t* out, uint64_t* totals, ScanReport rep) {
+  let_next_start();
   wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.y * col_stride;
   uint64_t* dst = out + (uint64_t)blockIdx.y * col_stride;
@@ -2759,6 +2761,7 @@ __global__ void k_tile_bounds(Dev d, uint64_t slab, uint32_t n_tiles, uint64_t t
 // Sort key of every GPU-side event: converted start time relative to the window start (records outside
 // the window emit nothing, their position does not matter).  Values are the buffer-order event numbers.
 __global__ void k_sort_keys(Dev d, uint64_t* keys, uint32_t* vals, uint64_t span) {
+  let_next_start();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ops_begin) return;
   int cls = 0;
@@ -2776,6 +2779,7 @@ __global__ void k_sort_keys(Dev d, uint64_t* keys, uint32_t* vals, uint64_t span
   vals[e] = e;
 }
 __global__ void k_sort_remap(Dev d, const uint32_t* rank) {
+  wait_for_previous();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ops_begin) return;
   int cls = 0;

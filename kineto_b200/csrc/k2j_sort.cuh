@@ -26,6 +26,8 @@ inline uint32_t sort_tiles(uint64_t n) {
 // hist[digit * n_tiles + tile] = number of keys of the tile with that digit
 __global__ void __launch_bounds__(kSortThreads) k_rs_hist(const uint64_t* keys, uint64_t n, uint32_t rounds, int shift, uint32_t* hist, uint32_t n_tiles) {
   __shared__ uint32_t s_h[256];
+  let_next_start();
+  wait_for_previous();
   s_h[threadIdx.x] = 0;
   __syncthreads();
   const uint64_t base = (uint64_t)blockIdx.x * rounds * kSortThreads;
@@ -44,6 +46,8 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const uint64_t* key
   __shared__ uint32_t s_cnt[kSortThreads / 32][256];  // per warp and digit: count, then offset within the round
   __shared__ uint32_t s_run[256];                      // keys of each digit placed by earlier rounds
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  let_next_start();
+  wait_for_previous();
   s_run[threadIdx.x] = 0;
   const uint64_t tile0 = (uint64_t)blockIdx.x * rounds * kSortThreads;
   for (uint32_t r = 0; r < rounds; r++) {
@@ -78,6 +82,8 @@ __global__ void __launch_bounds__(kSortThreads) k_rs_scatter(const uint64_t* key
 
 // rank[vals_sorted[pos]] = pos
 __global__ void k_rs_invert(const uint32_t* vals_sorted, uint64_t n, uint32_t* rank) {
+  let_next_start();
+  wait_for_previous();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) rank[vals_sorted[i]] = (uint32_t)i;
 }
