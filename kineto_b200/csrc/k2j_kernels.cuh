@@ -973,9 +973,9 @@ struct CountSink2 : CountSink {
 
 // ---- event programs ------------------------------------------------------------------------------------
 // An event is a fixed sequence of fields, each a literal followed by a value.  The sequence of a
-// record class is data (a table in constant memory), so all classes share one small formatting loop
-// and the lanes of a warp, which format events of one class, run it in lock step.  A field's value
-// is read from the thread's area in shared memory: the staged record itself, with the values that
+// record class is a table: straight-line code is made of it for the size pass (count_fields) and for the
+// classes nearly all events belong to in the emit pass (run_steps), and the rare shapes walk it (run_fields).
+// The lanes of a warp format events of one class in lock step.  A field's value is read from the thread's area in shared memory: the staged record itself, with the values that
 // are computed rather than stored (converted times, the linked op, occupancy ...) written by the
 // class's gather step into parts of the record that no field reads.
 enum : uint8_t { T_NONE = 0, T_U64, T_I64, T_TS, T_DBL, T_NAME, T_CSTR, T_MD /* the metadata entries of a CPU-side activity */,
@@ -2147,7 +2147,7 @@ __device__ __forceinline__ void put_value(S& s, const Dev& d, int type, uint64_t
   } while (md_mode && more);
 }
 
-// Emit pass: walks the set bits of `present`.  Descriptor and value of the NEXT field are fetched before
+// Emit pass, rare shapes and spans: walks the set bits of `present`.  Descriptor and value of the NEXT field are fetched before
 // the current one is formatted, so their latency hides behind the formatting work.
 template <class S, bool COLL = true>
 __device__ __forceinline__ void run_fields(S& s, const Dev& d, const uint32_t* a, int base, uint64_t present,
@@ -2176,11 +2176,6 @@ __device__ __forceinline__ void run_fields(S& s, const Dev& d, const uint32_t* a
 
 // Size pass: the same fields as straight-line code.  Field types, literal lengths and value slots are
 // compile-time constants here, so each present field costs its value's digit count and one addition.
-constexpr int field_word_offset(int i) {  // position of field i's literal in g_fields.w (as make_prog lays it out)
-  int w = 0;
-  for (int f = 0; f < i; f++) w += (c_strlen(kAllFields[f].lit) + 7) / 8;
-  return w;
-}
 constexpr uint32_t longest_constant_string() {  // among those a T_CSTR value can name (the counter-event pieces are written by put_counters)
   uint32_t m = 0;
   for (int f = CSTR_BASE; f < CSTR_BASE + CS_HWC; f++) if ((uint32_t)c_strlen(kAllFields[f].lit) > m) m = (uint32_t)c_strlen(kAllFields[f].lit);
@@ -2207,8 +2202,6 @@ template <int I> struct FieldInfo {
   static constexpr uint32_t len = (uint32_t)c_strlen(kAllFields[I].lit);
   static constexpr uint32_t voff = kAllFields[I].voff;
   static constexpr uint32_t vk = kAllFields[I].vk;
-  static constexpr int woff = field_word_offset(I);
-  static constexpr uint32_t vmax = value_max_bytes(kAllFields[I].type, kAllFields[I].vk);
 };
 template <int BASE, int F, int NF, class S>
 __device__ __forceinline__ void count_fields(S& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
@@ -2567,7 +2560,7 @@ __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32
   } else {
     uint64_t p;
     int base;
-    switch (cls) {  // one copy of the field loop for all classes
+    switch (cls) {
       case C_API: p = gather_api(d, a, t, filt, false, ext); base = API_BASE; break;
       case C_KERNEL: p = gather_kernel(d, a, t, filt, false, ext); base = KERNEL_BASE; break;
       case C_MEMCPY: p = gather_mem<C_MEMCPY>(d, a, t, filt, false, ext); base = MEM_BASE; break;
