@@ -367,10 +367,13 @@ k2j_status reserve_pool(k2j_ctx* c, uint64_t total) {
   K2J_CUDA(c, c->str_class.reserve(n + 1));
   return K2J_OK;
 }
-// Bytes of a pool that the workspaces hold.
+// Bytes of a pool that the workspaces hold; 0 where one of them could not be had.
 uint64_t pool_room(const k2j_ctx* c) {
-  const uint64_t n = c->n_strings;
-  return std::min<uint64_t>((c->esc_name.cap - 16 * (n + 1) - 16) / 2, c->esc_md.cap - 8 * (n + 1) - 16);
+  const uint64_t n = c->n_strings, name_fixed = 16 * (n + 1) + 16, md_fixed = 8 * (n + 1) + 16;
+  if (c->esc_name.cap < name_fixed || c->esc_md.cap < md_fixed || c->esc_name_len.cap < (n + 1) * 4 || c->esc_md_len.cap < (n + 1) * 4 ||
+      c->str_class.cap < n + 1)
+    return 0;
+  return std::min<uint64_t>((c->esc_name.cap - name_fixed) / 2, c->esc_md.cap - md_fixed);
 }
 void pool_pointers(const k2j_ctx* c, Dev& d) {
   d.esc_name = c->esc_name.as<uint8_t>(); d.esc_md = c->esc_md.as<uint8_t>();
@@ -636,6 +639,10 @@ k2j_status k2j_segment(k2j_ctx* c, k2j_segment_info* info) {
   // ---- string pool: sanitised copies (once per pool), by the first blocks of the segmentation's first launch ----
   PoolJob pool{};
   if (c->strings_dirty && c->n_strings) {
+    // (does nothing unless an allocation failed earlier, here or in k2j_set_strings, and the caller tries again)
+    k2j_status st = reserve_pool(c, c->pool_total);
+    if (st) return st;
+    pool_pointers(c, d);
     pool.blocks = (uint32_t)((c->n_strings + kSegWarps - 1) / kSegWarps);
     pool.room = pool_room(c);
     if (c->pool_unread) pool.total = c->h_totals + 29;

@@ -1,0 +1,97 @@
+"""libk2j's host side without a GPU: a child process runs it on a CUDA runtime of host memory (tests/native/fake_cudart.cpp)
+whose allocations can be made to fail and whose kernels are noted and not run."""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+import helpers
+
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+PRELUDE = """
+import ctypes as C, os, sys
+import numpy as np
+from kineto_b200 import api
+fake = C.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_most.argtypes = [C.c_size_t]
+fake.fake_pool_total.argtypes = [C.c_uint64]
+OK, CUDA = 0, 2
+lib = api.load_library()
+ctx = C.c_void_p()
+assert lib.k2j_create(0, None, C.byref(ctx)) == OK
+params = api.Params()
+assert lib.k2j_set_params(ctx, C.byref(params), None) == OK
+
+def log():
+    text = C.create_string_buffer(1 << 16)
+    assert fake.fake_log(text, len(text)) >= 0
+    return [l.split() for l in text.value.decode().splitlines()]
+
+def rooms():  # of the launches that make the pool's sanitised copies
+    return [int(l[2]) for l in log() if l[0] == "pool"]
+
+def on_device(a):
+    p = C.c_void_p()
+    assert fake.cudaMalloc(C.byref(p), C.c_size_t(a.nbytes)) == OK
+    C.memmove(p, a.ctypes.data, a.nbytes)
+    return p
+
+def pool(n, each):
+    return np.arange(n + 1, dtype=np.uint64) * each, np.full(max(n * each, 1), 65, np.uint8)
+
+def set_pool(n, each, device):
+    off, data = pool(n, each)
+    if not device:
+        return lib.k2j_set_strings(ctx, off.ctypes.data, data.ctypes.data, n)
+    fake.fake_pool_total(n * each)
+    return lib.k2j_set_strings(ctx, on_device(off), on_device(data), n)
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    from kineto_b200 import build
+    build.build()
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc()))), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I" + include,
+                    os.path.join(helpers.ROOT, "tests", "native", "fake_cudart.cpp"), "-o", so], check=True)
+    return so
+
+
+def run(fake, body):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(body)], cwd=helpers.ROOT, capture_output=True, text=True,
+                       env=dict(os.environ, LD_PRELOAD=fake), timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_a_pool_that_does_not_fit_is_never_written_by_a_retry(fake):
+    """The workspaces of a larger pool in device memory are allocated during the segmentation.  Where that fails, every
+    later try fails the same way or has the room: no launch is told of room that there is not."""
+    run(fake, """
+        assert set_pool(10, 10, True) == OK and lib.k2j_segment(ctx, None) == OK
+        assert all(100 <= r < 10_000 for r in rooms())
+        assert set_pool(10, 1 << 20, True) == OK     # its size is learned by the segmentation
+        fake.fake_most(1 << 20)
+        for again in range(3):
+            assert lib.k2j_segment(ctx, None) == CUDA
+            assert all(r < 10_000 for r in rooms()), again
+        fake.fake_most(1 << 40)
+        assert lib.k2j_segment(ctx, None) == OK
+        assert [r >= 10 << 20 for r in rooms()] == [True]
+    """)
+
+
+def test_workspaces_that_could_not_be_had_in_set_strings_are_asked_for_again(fake):
+    run(fake, """
+        fake.fake_most(1_500_000)
+        assert set_pool(10, 100_000, False) == CUDA   # (the copy of the pool fits, its sanitised copies do not)
+        assert lib.k2j_segment(ctx, None) == CUDA and rooms() == []
+        fake.fake_most(1 << 40)
+        assert lib.k2j_segment(ctx, None) == OK
+        assert [r >= 1_000_000 for r in rooms()] == [True]
+    """)
