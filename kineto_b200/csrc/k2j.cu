@@ -491,7 +491,7 @@ k2j_status k2j_set_strings(k2j_ctx* c, const uint64_t* off, const uint8_t* data,
   if (n >= 0xFFFFFFF0ull) return fail(c, K2J_ERR_INVALID_ARGUMENT, "too many strings");
   if (n > 0 && !off) return fail(c, K2J_ERR_INVALID_ARGUMENT, "null string offsets");
   K2J_CUDA(c, cudaSetDevice(c->device));
-  c->n_strings = n;
+  c->n_strings = 0;  // (a setter that fails leaves no arrays of its kind: those of the call before may be gone)
   c->strings_dirty = true;
   // A pool in device memory: its size is the last offset.  The context's workspaces are made for a pool as large as the one
   // before, the segmentation's first launch reports the size, and only a larger pool is done over (a copy of eight bytes
@@ -512,16 +512,21 @@ k2j_status k2j_set_strings(k2j_ctx* c, const uint64_t* off, const uint8_t* data,
     if (st) return st;
     c->pool_total = total;
   }
+  c->n_strings = n;
   return reserve_pool(c, total);
 }
 
 k2j_status k2j_set_cbid_names(k2j_ctx* c, const uint32_t* rt, uint32_t n_rt, const uint32_t* dr, uint32_t n_dr) {
   if (!c) return K2J_ERR_INVALID_ARGUMENT;
   K2J_CUDA(c, cudaSetDevice(c->device));
-  c->n_rt = n_rt; c->n_dr = n_dr;
+  c->n_rt = c->n_dr = 0;
   k2j_status st = stage(c, c->rt_names, rt, (size_t)n_rt * 4);
   if (st) return st;
-  return stage(c, c->dr_names, dr, (size_t)n_dr * 4);
+  c->n_rt = n_rt;
+  st = stage(c, c->dr_names, dr, (size_t)n_dr * 4);
+  if (st) return st;
+  c->n_dr = n_dr;
+  return K2J_OK;
 }
 
 k2j_status k2j_set_thread_map(k2j_ctx* c, const int32_t* pairs, uint32_t n) {
@@ -529,9 +534,10 @@ k2j_status k2j_set_thread_map(k2j_ctx* c, const int32_t* pairs, uint32_t n) {
   if (n > 0 && !pairs) return fail(c, K2J_ERR_INVALID_ARGUMENT, "null thread map");
   if (n > 0 && is_device_ptr(pairs)) return fail(c, K2J_ERR_INVALID_ARGUMENT, "thread map must be host memory");
   K2J_CUDA(c, cudaSetDevice(c->device));
-  c->n_tid = n;
+  c->n_tid = 0;
   k2j_status st = stage(c, c->tid_pairs, pairs, (size_t)n * 8);
   if (st) return st;
+  c->n_tid = n;
   return K2J_OK;
 }
 
@@ -541,7 +547,7 @@ k2j_status k2j_set_ops(k2j_ctx* c, const k2j_ops* o) {
   if (o->n_ops >= 0x7FFFFFF0ull) return fail(c, K2J_ERR_INVALID_ARGUMENT, "too many CPU activities");
   K2J_CUDA(c, cudaSetDevice(c->device));
   const uint64_t n = o->n_ops;
-  c->n_ops = n;
+  c->n_ops = 0;
   c->n_guest_ops = 0;  // new rows: k2j_set_guest_ops says again which of them are guests
   uint64_t n_md = 0;
   bool md_in_place = false;  // entries in device memory are used where they are: nobody asks how many there are
@@ -563,6 +569,7 @@ k2j_status k2j_set_ops(k2j_ctx* c, const k2j_ops* o) {
   if (md_in_place) c->op_md.dev = o->md;
   else STAGE(op_md, o->md, n_md * sizeof(k2j_md_entry));
 #undef STAGE
+  c->n_ops = n;
   return K2J_OK;
 }
 
@@ -572,6 +579,7 @@ k2j_status k2j_set_cupti(k2j_ctx* c, const uint8_t* bytes, uint64_t n_bytes, con
   if (n_buf > 0 && (!buftab || !bytes)) return fail(c, K2J_ERR_INVALID_ARGUMENT, "null CUPTI buffers");
   if (n_buf > 0 && is_device_ptr(buftab)) return fail(c, K2J_ERR_INVALID_ARGUMENT, "buffer table must be host memory");
   K2J_CUDA(c, cudaSetDevice(c->device));
+  c->n_buf = c->n_chunks = 0; c->cupti_bytes = 0;
   c->h_buf_off.clear(); c->h_buf_valid.clear(); c->h_buf_chunk_base.assign(1, 0);
   uint64_t chunks = 0;
   for (uint32_t b = 0; b < n_buf; b++) {
@@ -584,20 +592,19 @@ k2j_status k2j_set_cupti(k2j_ctx* c, const uint8_t* bytes, uint64_t n_bytes, con
     if (chunks >= 0xFFFFFFF0ull) return fail(c, K2J_ERR_INVALID_ARGUMENT, "too many chunks");
     c->h_buf_chunk_base.push_back((uint32_t)chunks);
   }
-  c->n_buf = (uint32_t)c->h_buf_off.size();
-  c->n_chunks = (uint32_t)chunks;
+  const uint32_t bufs = (uint32_t)c->h_buf_off.size();
   c->guest_front_bytes = 0; c->guest_back_bytes = ~0ull; c->guests_declared = false;
-  c->cupti_bytes = n_bytes;
   k2j_status st = stage(c, c->cupti, bytes, n_bytes);
   if (st) return st;
-  K2J_CUDA(c, c->d_buf_off.reserve(std::max<size_t>(8, c->n_buf * 8)));
-  K2J_CUDA(c, c->d_buf_valid.reserve(std::max<size_t>(8, c->n_buf * 8)));
-  K2J_CUDA(c, c->d_buf_chunk_base.reserve((c->n_buf + 1) * 4));
-  if (c->n_buf) {
-    K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_off.p, c->h_buf_off.data(), c->n_buf * 8, cudaMemcpyHostToDevice, c->stream));
-    K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_valid.p, c->h_buf_valid.data(), c->n_buf * 8, cudaMemcpyHostToDevice, c->stream));
+  K2J_CUDA(c, c->d_buf_off.reserve(std::max<size_t>(8, bufs * 8)));
+  K2J_CUDA(c, c->d_buf_valid.reserve(std::max<size_t>(8, bufs * 8)));
+  K2J_CUDA(c, c->d_buf_chunk_base.reserve((bufs + 1) * 4));
+  if (bufs) {
+    K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_off.p, c->h_buf_off.data(), bufs * 8, cudaMemcpyHostToDevice, c->stream));
+    K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_valid.p, c->h_buf_valid.data(), bufs * 8, cudaMemcpyHostToDevice, c->stream));
   }
-  K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_chunk_base.p, c->h_buf_chunk_base.data(), (c->n_buf + 1) * 4, cudaMemcpyHostToDevice, c->stream));
+  K2J_CUDA(c, cudaMemcpyAsync(c->d_buf_chunk_base.p, c->h_buf_chunk_base.data(), (bufs + 1) * 4, cudaMemcpyHostToDevice, c->stream));
+  c->n_buf = bufs; c->n_chunks = (uint32_t)chunks; c->cupti_bytes = n_bytes;
   return K2J_OK;
 }
 

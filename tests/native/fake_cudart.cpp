@@ -26,6 +26,7 @@ void note(const char* what, const void* a, uint64_t b = 0) {
 }
 cudaError_t launched(const void* f, void** args) {
   const std::string& name = g_kernels[f];
+  g_log.push_back("launch " + name);
   if (name.find("k_seg_chunks") != std::string::npos) {
     const PoolJob* job = static_cast<const PoolJob*>(args[1]);
     if (job->total) *job->total = g_pool_total;

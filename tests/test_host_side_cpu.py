@@ -95,3 +95,31 @@ def test_workspaces_that_could_not_be_had_in_set_strings_are_asked_for_again(fak
         assert lib.k2j_segment(ctx, None) == OK
         assert [r >= 1_000_000 for r in rooms()] == [True]
     """)
+
+
+def test_a_setter_that_fails_leaves_no_arrays_of_its_kind(fake):
+    """The staged copies of the call before are gone by then: nothing may read them."""
+    run(fake, """
+        def ops(n):
+            cols = {name: np.zeros(n, np.int64) for name in ("start_ns", "end_ns", "id", "device", "resource", "thread", "type", "name", "flow_id", "flow_info")}
+            off = np.zeros(n + 1, np.uint32)
+            keep.append((cols, off))
+            return lib.k2j_set_ops(ctx, C.byref(api.Ops(n, *[a.ctypes.data for a in cols.values()], off.ctypes.data, None)))
+
+        def cupti(n):
+            data, table = np.zeros(n, np.uint8), np.array([0, n], np.uint64)
+            return lib.k2j_set_cupti(ctx, data.ctypes.data, n, table.ctypes.data, 1)
+
+        keep, info = [], api.SegmentInfo()
+        assert set_pool(10, 10, False) == OK and ops(10) == OK and cupti(4096) == OK
+        assert lib.k2j_segment(ctx, C.byref(info)) == OK and info.n_ops == 10
+        assert sum("k_seg_chunks" in l[1] for l in log() if l[0] == "launch") == 1
+        fake.fake_most(1 << 16)
+        assert set_pool(100_000, 1, False) == CUDA and ops(100_000) == CUDA and cupti(1 << 20) == CUDA
+        fake.fake_most(1 << 40)
+        log()
+        assert lib.k2j_segment(ctx, C.byref(info)) == OK and info.n_ops == 0
+        assert sum("k_seg_chunks" in l[1] for l in log() if l[0] == "launch") == 0
+        assert set_pool(100_000, 1, False) == OK and ops(100_000) == OK and cupti(1 << 20) == OK
+        assert lib.k2j_segment(ctx, C.byref(info)) == OK and info.n_ops == 100_000
+    """)
