@@ -14,7 +14,10 @@
  * kernels on the context's stream: its contents must be complete before the call that uses them, or be
  * produced by work that is ordered before the context's stream (the same stream, or an event the stream
  * waits on).  A caller that fills such arrays on another stream (NCCL, a framework's current stream)
- * either passes that stream to k2j_create or synchronises it first; the library inserts no such wait.
+ * either passes that stream to k2j_create or synchronises it first; the library inserts no such wait,
+ * but for one: k2j_set_strings and k2j_set_ops put everything the context runs from then on behind the
+ * work that the legacy default stream holds when they are called, if the pool (the metadata entries and
+ * their offsets) is in device memory.
  */
 #ifndef K2J_H_
 #define K2J_H_

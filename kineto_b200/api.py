@@ -232,7 +232,9 @@ class K2J:
               "op_resource", "op_thread", "op_type", "op_name", "op_flow", "op_flowt", "op_mdoff", "md", "cupti"]
 
     def load(self, trace: tf.Trace, arrays: dict | None = None):
-        """Stages a whole trace.  `arrays` overrides the numpy arrays of `trace` (e.g. device tensors)."""
+        """Stages a whole trace.  `arrays` overrides the numpy arrays of `trace` (e.g. device tensors).  Tensors on the GPU are
+        read on the context's stream: they are complete, or being filled on torch's default stream; work on any other
+        stream is synchronised first, or the context is made on that stream."""
         self.set_params(trace)
         a = {k: np.ascontiguousarray(getattr(trace, k)) for k in self.ARRAYS}
         if arrays:

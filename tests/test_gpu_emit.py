@@ -97,3 +97,25 @@ def test_pools_in_device_memory_that_grow_and_shrink_between_traces_of_one_conte
     ctx.run()
     assert ctx.copy_output().tobytes() == traces[0][2]
     ctx.close()
+
+
+def test_inputs_that_the_default_stream_is_still_writing():
+    """Device arrays filled on the legacy default stream just before a load, by a program that does not synchronise: the
+    context's first trace and the later ones (which read no sizes back) see them complete."""
+    import torch
+    from kineto_b200 import api
+    trace = synth.gen_kernel_launches(3000, seed=67, pool_size=50)
+    want = helpers.run_port(trace)[0]
+    full = api.device_arrays(trace, "cuda:0")
+    ctx = api.K2J(0)
+    for _ in range(3):
+        arrays = {k: torch.zeros_like(a) for k, a in full.items()}
+        torch.cuda.synchronize()
+        assert torch.cuda.current_stream() == torch.cuda.default_stream()
+        torch.cuda._sleep(20_000_000)  # some 10 ms
+        for k, a in arrays.items():
+            a.copy_(full[k])
+        ctx.load(trace, arrays)
+        ctx.run()
+        assert ctx.copy_output().tobytes() == want
+    ctx.close()

@@ -123,3 +123,25 @@ def test_a_setter_that_fails_leaves_no_arrays_of_its_kind(fake):
         assert set_pool(100_000, 1, False) == OK and ops(100_000) == OK and cupti(1 << 20) == OK
         assert lib.k2j_segment(ctx, C.byref(info)) == OK and info.n_ops == 100_000
     """)
+
+
+def test_arrays_in_device_memory_are_read_behind_the_default_stream(fake):
+    """A pool's offsets and the metadata entries in device memory may still be in the making on the legacy default stream:
+    either a blocking copy has waited for it, or the context's stream does."""
+    run(fake, """
+        def ordered():
+            lines, recorded = log(), set()
+            for l in lines:
+                if l[0] == "record" and l[2] == "1":   # cudaStreamLegacy
+                    recorded.add(l[1])
+            return any(l[0] == "copy_and_wait" or (l[0] == "wait" and l[1] in recorded) for l in lines)
+
+        cols = [on_device(np.zeros(8, np.int64)) for _ in range(10)]
+        off, md = on_device(np.arange(9, dtype=np.uint32)), on_device(np.zeros(8 * 4, np.uint64))
+        log()
+        for trace in range(3):
+            assert set_pool(10, 10, True) == OK and ordered(), trace
+            assert lib.k2j_set_ops(ctx, C.byref(api.Ops(8, *cols, off, md))) == OK and ordered(), trace
+            assert lib.k2j_segment(ctx, None) == OK
+            log()
+    """)
