@@ -1245,7 +1245,7 @@ template <class S> __device__ __forceinline__ void put_name(S& s, const Dev& d, 
   put_pool_words(s, d.esc_name + esc_name_pos(d, id), len);
   *name_bytes += len;
 }
-template <bool ROOM> __device__ __forceinline__ void put_string(WindowSink& s, const uint64_t* w, uint32_t len);
+template <bool ROOM> __device__ __forceinline__ void put_string(InlineSink& s, const uint64_t* w, uint32_t len);
 template <class S> __device__ __forceinline__ void put_mdstr(S& s, const Dev& d, uint32_t id) {
   if (id >= d.n_strings) { atomicAdd(&d.counters->device_check, 1ull); return; }
   if constexpr (S::kCounting) s.skip(d.esc_md_len[id]);
@@ -2226,7 +2226,7 @@ __device__ __noinline__ ulonglong2 app_long(Win win, uint32_t pos, uint32_t carr
   return make_ulonglong2(pack64(s.pos, s.carry), (uint64_t)reinterpret_cast<uintptr_t>(s.gbase) | (s.open >> 3));
 }
 // ROOM: kNameWindowBytes are known to fit.
-template <bool ROOM> __device__ __forceinline__ void put_string(WindowSink& s, const uint64_t* w, uint32_t len) {
+template <bool ROOM> __device__ __forceinline__ void put_string(InlineSink& s, const uint64_t* w, uint32_t len) {
   const uint32_t active = __activemask();
   if (!__any_sync(active, len > 16u)) {
     if (!ROOM) s.ensure(16);
@@ -2248,7 +2248,7 @@ template <bool ROOM> __device__ __forceinline__ void put_string(WindowSink& s, c
     s.gbase = reinterpret_cast<uint8_t*>((uintptr_t)(r.y & ~31ull));
   }
 }
-__device__ __forceinline__ void put_pool_name(WindowSink& s, const Dev& d, uint32_t id) {
+__device__ __forceinline__ void put_pool_name(InlineSink& s, const Dev& d, uint32_t id) {
   if (id >= d.n_strings) { atomicAdd(&d.counters->device_check, 1ull); return; }
   put_string<true>(s, reinterpret_cast<const uint64_t*>(d.esc_name + esc_name_pos(d, id)), d.esc_name_len[id]);
 }
@@ -2260,7 +2260,7 @@ __device__ __forceinline__ WindowSink sink_at(Win win, uint32_t pos, uint32_t ca
   s.win = win; s.pos = pos; s.carry = carry; s.open = 0; s.gbase = nullptr;
   return s;
 }
-__device__ __forceinline__ uint64_t sink_state(const WindowSink& s) { return (uint64_t)s.pos | ((uint64_t)s.carry << 32); }
+template <class S> __device__ __forceinline__ uint64_t sink_state(const S& s) { return (uint64_t)s.pos | ((uint64_t)s.carry << 32); }
 // Three decimal digits per look-up: the zero-padded characters in the low three bytes, most significant first, and eight
 // times the number of leading zeros (of at most two) in the top byte.  The table is in front of the emit kernel's dynamic
 // shared memory.  A number below 1000 costs some 25 instructions with its append, by arithmetic on four digits some 40.
@@ -2274,7 +2274,7 @@ constexpr Digits3 make_digits3() {
 __device__ const Digits3 g_digits3 = make_digits3();
 extern __shared__ uint4 s_dyn[];
 __device__ __forceinline__ uint32_t digits3(uint32_t v) { return reinterpret_cast<const uint32_t*>(s_dyn)[v]; }
-__device__ __forceinline__ void put_below_1000(WindowSink& s, uint32_t v) {
+template <class S> __device__ __forceinline__ void put_below_1000(S& s, uint32_t v) {
   const uint32_t e = digits3(v), z = e >> 24;
   s.put((e & 0xffffffu) >> z, (int)(3u - (z >> 3)));
 }
@@ -2462,7 +2462,7 @@ template <int R> struct RunLit {
       for (int i = 0; kAllFields[f].lit[i]; i++, p++) w[p / 4] |= (uint32_t)(unsigned char)kAllFields[f].lit[i] << (8 * (p % 4));
   }
 };
-template <int R, bool COLL> __device__ __forceinline__ void put_run(WindowSink& s, const Dev& d, const uint32_t* a, unsigned long long* name_bytes) {
+template <int R, bool COLL> __device__ __forceinline__ void put_run(InlineSink& s, const Dev& d, const uint32_t* a, unsigned long long* name_bytes) {
   using I = RunOf<R>;
   constexpr uint32_t n = I::len, nw = (n + 3) / 4, rem = n % 4;
   if constexpr (n != 0) {
@@ -2495,14 +2495,14 @@ template <int R, bool COLL> __device__ __forceinline__ void put_run(WindowSink& 
       put_pool_name(s, d, a[w]);
       st = sink_state(s);
     } else {  // metadata entries: they ask the sink for room themselves
-      if constexpr (COLL || I::type != T_COLL) put_value<WindowSink, COLL, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
+      if constexpr (COLL || I::type != T_COLL) put_value<InlineSink, COLL, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
       st = sink_state(s);
     }
     s.pos = (uint32_t)st; s.carry = (uint32_t)(st >> 32);
   }
 }
 template <int R, int END, bool COLL>
-__device__ __forceinline__ void put_runs(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
+__device__ __forceinline__ void put_runs(InlineSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
   if constexpr (R < END) {
     if constexpr (RunOf<R>::cond < 0) put_run<R, COLL>(s, d, a, name_bytes);
     else if ((present >> RunOf<R>::cond) & 1ull) put_run<R, COLL>(s, d, a, name_bytes);
@@ -2510,12 +2510,12 @@ __device__ __forceinline__ void put_runs(WindowSink& s, const Dev& d, const uint
   }
 }
 template <int ST, bool COLL>
-__device__ __forceinline__ void put_step(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
+__device__ __forceinline__ void put_step(InlineSink& s, const Dev& d, const uint32_t* a, uint64_t present, unsigned long long* name_bytes) {
   // (the launch for kernels with collective metadata holds the kernel class's code only)
   if constexpr (ST < kNumSteps && (!COLL || ST < ClassSteps<0>::end)) put_runs<StepOf<ST>::first, StepOf<ST>::end, COLL>(s, d, a, present, name_bytes);
 }
 template <bool COLL>
-__device__ __forceinline__ void run_steps(WindowSink& s, const Dev& d, const uint32_t* a, uint64_t present, int step, int end, unsigned long long* name_bytes) {
+__device__ __forceinline__ void run_steps(InlineSink& s, const Dev& d, const uint32_t* a, uint64_t present, int step, int end, unsigned long long* name_bytes) {
 #pragma unroll 1
   for (; step < end; step++) {
     s.room(kStepBytes);
@@ -2692,9 +2692,9 @@ __global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? 
       d.ev_size[ev] = filt ? 0u : s.n;
       if (cls != C_OP) d.ev_ext[ev] = ext;
     } else {
-      WindowSink s;
+      InlineSink s;
       s.init(d.out + off, size, (Win)__cvta_generic_to_shared(s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u)));
-      if (format_event<WindowSink, COLL>(s, d, cls, area, j, t, &filt, &ext) && !s.finish(d.out + off, size))
+      if (format_event<InlineSink, COLL>(s, d, cls, area, j, t, &filt, &ext) && !s.finish(d.out + off, size))
         atomicAdd(&d.counters->device_check, 1ull);
     }
   }
@@ -2841,7 +2841,7 @@ __global__ void __launch_bounds__(kEventThreads) k_annotations(Dev d, const Span
     const uint32_t size = sizes[i];
     uint8_t* dst = d.out + out_base + offs[i];
     if (size < kMinEventBytes || out_base + offs[i] + size > d.out_cap) { atomicAdd(&d.counters->device_check, 1ull); return; }
-    WindowSink s;
+    InlineSink s;
     s.init(dst, size, (Win)__cvta_generic_to_shared(s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u)));
     run_fields(s, d, a, ANN_BASE, p, &nb);
     if (!s.finish(dst, size)) atomicAdd(&d.counters->device_check, 1ull);

@@ -81,7 +81,7 @@ inline void win_st(Win w, uint32_t k, uint32_t v) { w[k * (uint32_t)kWinStride] 
 inline Win win_from(Win w, uint32_t k) { return w + k * (uint32_t)kWinStride; }
 #endif
 // the same as two 128-bit stores, for code out of line: in a function that was called, 256-bit stores left three quarters of
-// a block unwritten (ptxas 12.9; the same source in line is right)
+// a block unwritten (ptxas 12.9; the same source in line is right; why was not found)
 K2J_HD void store16x2(uint8_t* p, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
 #if defined(__CUDA_ARCH__)
   *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a, b);
@@ -134,8 +134,10 @@ K2J_HD uint32_t window_flush(Win win, uint32_t pos, uint32_t carry, uint8_t* gba
   return nb;
 }
 
-struct WindowSink {
-  static constexpr bool kCounting = false;
+// WIDE: blocks leave as 256-bit stores.  Only a sink that lives in a kernel's own code, with everything it is handed to in
+// line, may do that (see store16x2): such a kernel names InlineSink.  WindowSink is right everywhere.
+template <bool WIDE> struct Sink {
+  static constexpr bool kCounting = false, kWide = WIDE;
   Win win;                // this thread's window
   uint32_t pos;           // window offset of the next byte
   uint32_t carry;         // the 32-bit word being filled: bytes below pos & 3 are set, the rest is zero
@@ -152,8 +154,8 @@ struct WindowSink {
     else *reinterpret_cast<uint32_t*>(gbase + w0 + 4) = (uint32_t)(w >> 32);
   }
   // Writes the complete 32-byte blocks of the window to global memory and moves the open block to the front.
-  template <bool WIDE = true> K2J_HD void flush() {
-    const uint32_t nb = window_flush<WIDE>(win, pos, carry, gbase, open);
+  template <bool W = WIDE> K2J_HD void flush() {
+    const uint32_t nb = window_flush<W>(win, pos, carry, gbase, open);
     if (nb != 0u) open = 0u;
     gbase += 32u * nb; pos -= 32u * nb;
   }
@@ -179,15 +181,15 @@ struct WindowSink {
   }
   // A long string from an 8-byte aligned word array (words up to one behind its last byte are readable): past the window,
   // straight from registers to the output.  The bytes up to the output's next 8-byte boundary and those behind the last one
-  // go through the window.  For code out of line (see store16x2).
-  template <bool WIDE = false> K2J_HD void long_words(const uint64_t* w, uint32_t len) {
+  // go through the window.
+  template <bool W = WIDE> K2J_HD void long_words(const uint64_t* w, uint32_t len) {
     uint32_t h = (0u - pos) & 7u;
     h = h < len ? h : len;
     uint64_t cur = len != 0u ? w[0] : 0ull;
     put64(h != 0u ? cur & (~0ull >> (8u * (8u - h))) : 0ull, h);
     uint32_t n = (len - h) >> 3;  // whole words of output
     if (n != 0u) {
-      flush<WIDE>();
+      flush<W>();
       for (uint32_t o = open; o < pos; o += 8u) *reinterpret_cast<uint64_t*>(gbase + o) = W64(o >> 2);
       uint8_t* dst = gbase + pos;
       const uint32_t odd = h & 4u, sh = 8u * (h & 3u);
@@ -220,10 +222,10 @@ struct WindowSink {
 #pragma unroll
 #endif
         for (uint32_t k = 0; k < 8u; k++) if (k < (n & ~3u)) y[k] = w[k + 1u];
-        store_block<WIDE>(dst, shifted(cur, x[0]), shifted(x[0], x[1]), shifted(x[1], x[2]), shifted(x[2], x[3]));
+        store_block<W>(dst, shifted(cur, x[0]), shifted(x[0], x[1]), shifted(x[1], x[2]), shifted(x[2], x[3]));
         cur = x[3];
         if (m == 8u) {
-          store_block<WIDE>(dst + 32, shifted(cur, x[4]), shifted(x[4], x[5]), shifted(x[5], x[6]), shifted(x[6], x[7]));
+          store_block<W>(dst + 32, shifted(cur, x[4]), shifted(x[4], x[5]), shifted(x[5], x[6]), shifted(x[6], x[7]));
           cur = x[7];
         }
         dst += 8u * m;
@@ -364,5 +366,7 @@ struct WindowSink {
     return gbase + pos == dst + size;
   }
 };
+using WindowSink = Sink<false>;
+using InlineSink = Sink<true>;
 
 }  // namespace k2j

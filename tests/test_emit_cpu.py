@@ -1,6 +1,7 @@
 """Parts of the emit pass that compile for the host."""
 import ctypes
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -38,3 +39,16 @@ def test_packed_doubles_print_as_the_doubles(ec):
     special = np.array([0.0, -0.0, -1.5, np.inf, -np.inf, np.nan])
     assert ec.ec_packed_doubles(special.ctypes.data_as(ctypes.c_void_p), ctypes.c_int64(6), ctypes.byref(left)) == 0
     assert left.value == 6
+
+
+def test_code_out_of_line_uses_the_sink_without_wide_stores():
+    """256-bit stores are right only in a kernel's own code: WindowSink has none, and no function that is called names the other."""
+    csrc = os.path.join(helpers.ROOT, "kineto_b200", "csrc")
+    src = '#include <string>\n#include "k2j_sink.cuh"\nstatic_assert(!k2j::WindowSink::kWide && k2j::InlineSink::kWide, "");\n'
+    r = subprocess.run(["g++", "-std=c++17", "-I" + csrc, "-fsyntax-only", "-x", "c++", "-"], input=src, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    with open(os.path.join(csrc, "k2j_kernels.cuh")) as f:
+        text = f.read()
+    called = [text[at:text.index("\n}\n", at)] for at in (m.start() for m in re.finditer("__noinline__", text))]
+    assert sum("WindowSink" in body for body in called) >= 8
+    assert not [body for body in called if re.search(r"InlineSink|Sink<true>|flush<true>|long_words<true>|\bstore32\b", body)]
