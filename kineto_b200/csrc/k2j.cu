@@ -60,6 +60,7 @@ struct Input {
 
 struct k2j_ctx {
   int device = 0;
+  uint32_t sms = 0;  // multiprocessors of the device
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::string err;
@@ -220,7 +221,7 @@ k2j_status run_clear(k2j_ctx* c, const ClearList& l) {
   for (uint32_t k = 0; k < l.n; k++) words = std::max(words, l.r[k].words);
   if (words == 0) return K2J_OK;
   const uint64_t blocks = (words / 2 + kClearThreads) / kClearThreads;
-  k_clear<<<(uint32_t)std::min<uint64_t>(blocks, 148 * 8), kClearThreads, 0, c->stream>>>(l);
+  k_clear<<<(uint32_t)std::min<uint64_t>(blocks, 8ull * c->sms), kClearThreads, 0, c->stream>>>(l);
   c->launches++;
   K2J_CUDA(c, cudaGetLastError());
   return K2J_OK;
@@ -228,7 +229,7 @@ k2j_status run_clear(k2j_ctx* c, const ClearList& l) {
 
 // Workspaces of the radix sort for n pairs.
 k2j_status sort_reserve(k2j_ctx* c, uint64_t n) {
-  const uint32_t tiles = sort_tiles(n);
+  const uint32_t tiles = sort_tiles(n, c->sms);
   for (int i = 0; i < 2; i++) {
     K2J_CUDA(c, c->sort_keys[i].reserve(n * 8));
     K2J_CUDA(c, c->sort_vals[i].reserve(n * 4));
@@ -241,15 +242,15 @@ k2j_status sort_reserve(k2j_ctx* c, uint64_t n) {
 // the buffers that hold the result.
 k2j_status sort_passes(k2j_ctx* c, uint64_t n, int passes, int* cur_io) {
   cudaStream_t s = c->stream;
-  const uint32_t tiles = sort_tiles(n);
+  const uint32_t tiles = sort_tiles(n, c->sms);
   int cur = *cur_io;
   for (int pass = 0; pass < passes; pass++) {
-    launch_behind(k_rs_hist, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), n, sort_rounds(n), 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
+    launch_behind(k_rs_hist, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), n, sort_rounds(n, c->sms), 8 * pass, c->sort_hist.as<uint32_t>(), tiles);
     c->launches++;
     k2j_status st = run_scan(c, c->sort_hist.as<uint32_t>(), (uint64_t)tiles * 256, 1, c->sort_base.as<uint64_t>(),
                              c->scan_totals.as<uint64_t>() + 23, &c->launches);
     if (st) return st;
-    launch_behind(k_rs_scatter, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, sort_rounds(n),
+    launch_behind(k_rs_scatter, dim3(tiles), kSortThreads, s, c->sort_keys[cur].as<uint64_t>(), c->sort_vals[cur].as<uint32_t>(), n, sort_rounds(n, c->sms),
                   8 * pass, c->sort_base.as<uint64_t>(), tiles, c->sort_keys[cur ^ 1].as<uint64_t>(), c->sort_vals[cur ^ 1].as<uint32_t>());
     c->launches++;
     cur ^= 1;
@@ -413,7 +414,9 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return K2J_ERR_CUDA; }
     c->own_stream = true;
   }
-  bool ok = cudaMallocHost((void**)&c->h_totals, 32 * sizeof(uint64_t) + kPinnedSpans * sizeof(SpanRec)) == cudaSuccess &&
+  int sms = 0;
+  bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0 &&
+            cudaMallocHost((void**)&c->h_totals, 32 * sizeof(uint64_t) + kPinnedSpans * sizeof(SpanRec)) == cudaSuccess &&
             cudaMallocHost((void**)&c->h_counters, sizeof(Counters)) == cudaSuccess &&
             c->counters.reserve(sizeof(Counters)) == cudaSuccess && c->scan_totals.reserve(32 * 8) == cudaSuccess;
   for (auto& e : c->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
@@ -423,6 +426,7 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
        cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
   if (!ok) { k2j_destroy(c); return K2J_ERR_CUDA; }
   c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
+  c->sms = (uint32_t)sms;
   *out = c;
   return K2J_OK;
 }
@@ -1011,8 +1015,8 @@ constexpr uint64_t kSlabPad = 64;              // bytes in front of a slab's tex
 k2j_status stream_bytes(k2j_ctx* c, const uint8_t* src, int fd, bool positioned, uint64_t file_offset, uint64_t total, cudaStream_t stream);
 
 // Threads of a block of the emit pass: a trace that one wave of the chip holds spreads over all SMs.
-int emit_threads(uint64_t items) {
-  const uint64_t each = (items + 148 * kEmitBlocks - 1) / (148 * kEmitBlocks);
+int emit_threads(uint64_t items, uint32_t sms) {
+  const uint64_t wave = (uint64_t)sms * kEmitBlocks, each = (items + wave - 1) / wave;
   return (int)std::min<uint64_t>(kEmitThreads, std::max<uint64_t>(64, (each + 31) & ~31ull));
 }
 // The emit launches for the events whose text starts in [d.tile_begin, d.tile_end).  `ranges`: per class the work
@@ -1022,7 +1026,7 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     if (end <= begin) return;
     Dev dr = d;
     dr.work_origin = begin; dr.n_work = end;
-    const int threads = emit_threads(end - begin);
+    const int threads = emit_threads(end - begin, c->sms);
     k_events<true><<<(uint32_t)((end - begin + threads - 1) / threads), threads, emit_smem_bytes(threads), s>>>(dr);
     c->launches++;
   };

@@ -11,15 +11,16 @@ namespace k2j {
 constexpr int kSortThreads = 256;
 // Rounds of kSortThreads keys a block (a tile) takes.  The scatter's rounds are a serial chain of barriers, so a sort too
 // short to fill the chip with tiles of eight rounds takes fewer, up to one tile for every block that can be resident
-// (148 SMs x 8): 500 k keys fill 245 blocks at eight rounds and 977 at two.  Size pass and sort of 500 k events: 263 -> 252 us.
-constexpr uint64_t kSortResident = 148 * 8;
+// (8 an SM, 1184 with 148 SMs): 500 k keys fill 245 blocks at eight rounds and 977 at two.  Size pass and sort of 500 k
+// events: 263 -> 252 us.
+constexpr uint64_t kSortBlocks = 8;
 constexpr uint32_t kSortMaxRounds = 8;
-inline uint32_t sort_rounds(uint64_t n) {
-  const uint64_t r = (n + kSortResident * kSortThreads - 1) / (kSortResident * kSortThreads);
+inline uint32_t sort_rounds(uint64_t n, uint32_t sms) {
+  const uint64_t round = sms * kSortBlocks * kSortThreads, r = (n + round - 1) / round;
   return r < 1 ? 1u : r > kSortMaxRounds ? kSortMaxRounds : (uint32_t)r;
 }
-inline uint32_t sort_tiles(uint64_t n) {
-  const uint64_t tile = (uint64_t)sort_rounds(n) * kSortThreads;
+inline uint32_t sort_tiles(uint64_t n, uint32_t sms) {
+  const uint64_t tile = (uint64_t)sort_rounds(n, sms) * kSortThreads;
   return (uint32_t)((n + tile - 1) / tile);
 }
 

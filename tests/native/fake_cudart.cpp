@@ -15,6 +15,7 @@ std::map<const void*, std::string> g_kernels;     // host stub -> name
 std::vector<std::string> g_log;
 size_t g_most = ~(size_t)0;                       // larger allocations fail
 uint64_t g_pool_total = 0;                        // what the segmentation's first launch reports as the pool's size
+uint64_t g_scan_total = 0;                        // what scans report as the (first) column's total, unless 0
 uintptr_t g_handle = 0x1000;
 thread_local struct { dim3 grid, block; size_t smem; void* stream; } g_conf;
 
@@ -24,9 +25,13 @@ void note(const char* what, const void* a, uint64_t b = 0) {
   snprintf(line, sizeof line, "%s %llx %llu", what, (unsigned long long)(uintptr_t)a, (unsigned long long)b);
   g_log.push_back(line);
 }
-cudaError_t launched(const void* f, void** args) {
+cudaError_t launched(const void* f, dim3 grid, dim3 block, void** args) {
   const std::string& name = g_kernels[f];
-  g_log.push_back("launch " + name);
+  g_log.push_back("launch " + name + " " + std::to_string(grid.x) + " " + std::to_string(block.x));
+  if (name.find("k_scan_small") != std::string::npos || name.find("k_scan_apply") != std::string::npos) {
+    uint64_t* totals = *static_cast<uint64_t**>(args[name.find("k_scan_small") != std::string::npos ? 2 : 6]);
+    if (totals && g_scan_total) *totals = g_scan_total;
+  }
   if (name.find("k_seg_chunks") != std::string::npos) {
     const PoolJob* job = static_cast<const PoolJob*>(args[1]);
     if (job->total) *job->total = g_pool_total;
@@ -43,6 +48,7 @@ bool on_device(const void* p) {
 extern "C" {
 void fake_most(size_t bytes) { g_most = bytes; }
 void fake_pool_total(uint64_t bytes) { g_pool_total = bytes; }
+void fake_scan_total(uint64_t total) { g_scan_total = total; }
 int fake_log(char* text, int room) {  // what was noted since the last call, a line each
   std::string all;
   for (const auto& l : g_log) all += l + "\n";
@@ -80,8 +86,8 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   a->type = on_device(p) ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void** args, size_t, cudaStream_t) { return launched(f, args); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void** args) { return launched(f, args); }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3 block, void** args, size_t, cudaStream_t) { return launched(f, grid, block, args); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void** args) { return launched(f, c->gridDim, c->blockDim, args); }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)(g_handle += 16); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }

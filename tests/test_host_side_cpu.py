@@ -18,7 +18,7 @@ import numpy as np
 from kineto_b200 import api
 fake = C.CDLL(os.environ["LD_PRELOAD"])
 fake.fake_most.argtypes = [C.c_size_t]
-fake.fake_pool_total.argtypes = [C.c_uint64]
+fake.fake_pool_total.argtypes = fake.fake_scan_total.argtypes = [C.c_uint64]
 OK, CUDA = 0, 2
 lib = api.load_library()
 ctx = C.c_void_p()
@@ -144,4 +144,21 @@ def test_arrays_in_device_memory_are_read_behind_the_default_stream(fake):
             assert lib.k2j_set_ops(ctx, C.byref(api.Ops(8, *cols, off, md))) == OK and ordered(), trace
             assert lib.k2j_segment(ctx, None) == OK
             log()
+    """)
+
+
+def test_the_emit_pass_spreads_over_the_sms_that_the_gpu_has(fake):
+    """A trace that one wave holds gets the smallest blocks that still make one wave: two an SM of (here) 132."""
+    run(fake, """
+        def threads(n):
+            cols = [np.zeros(n, np.int64) for _ in range(10)]
+            off = np.zeros(n + 1, np.uint32)
+            assert lib.k2j_set_ops(ctx, C.byref(api.Ops(n, *[a.ctypes.data for a in cols], off.ctypes.data, None))) == OK
+            log()
+            fake.fake_scan_total(100 * n)
+            assert lib.k2j_run(ctx, C.byref(api.Result())) == OK
+            (block,) = [int(l[3]) for l in log() if l[0] == "launch" and "k_eventsILb1ELb0E" in l[1]]
+            return block
+
+        assert [threads(132 * 2 * k + more) for k, more in ((1, 0), (64, 0), (64, 1), (96, 0), (96, 1), (320, 0), (320, 1))] == [64, 64, 96, 96, 128, 320, 320]
     """)
