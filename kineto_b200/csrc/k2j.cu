@@ -182,18 +182,18 @@ uint32_t pow2_at_least(uint64_t n) {
 // Exclusive scan of `cols` columns of n u32 each (column stride n) into u64; totals land in
 // totals[0..cols), device or pinned host memory.  One, two or three launches by the column's length.  One column,
 // us per call of k2j_exclusive_scan_u32 with its wait:
-//   elements                   200   4096   8192   12 288   16 384  |  tiles of 2048   4096   4097   6144   8192   16 384
-//   one launch                  16     19     21       25       27  |
-//   two launches                17     18     18       18       18  |                    66     69     93    121      244
-//   three launches                                                  |                    72     72     99    127      237
-//   three launches and a copy   27     27     27       28       31  |                    82     81
-// One launch serves up to 4096 elements, where it meets two (a block's serial rounds of 8192 against a launch); the last
-// two meet between 8192 and 16 384 tiles (sums that every block adds up again against a launch).
-constexpr uint64_t kScanSmallMax = kScanSmallTile / 2;
+//   elements                   200   1000   4096   4097   8192   12 288   16 384  |  tiles of 2048   4096   4097   6144   8192   16 384
+//   one launch                  15     15     17            21       25       27  |
+//   two launches                17            18     19     18       18       18  |                    66     69     93    121      244
+//   three launches                                                                |                    72     72     99    127      237
+//   three launches and a copy   27            27            27       28       31  |                    82     81
+// One launch serves up to 4096 elements, a block of 512 threads and no loop (1024 threads, the upper half idle: 16.5, 16.9,
+// 18.7 us at the first three sizes; beyond it one launch means a block's serial rounds, measured in rounds of 8192 elements);
+// the last two meet between 8192 and 16 384 tiles (sums that every block adds up again against a launch).
 constexpr uint32_t kScanDirectBlocks = 4096;
 k2j_status run_scan(k2j_ctx* c, const uint32_t* in, uint64_t n, uint32_t cols, uint64_t* out, uint64_t* totals, uint32_t* launches,
                     const ScanReport& rep = ScanReport{}) {
-  if (n <= kScanSmallMax) {
+  if (n <= (uint64_t)kScanSmallMax) {
     launch_behind(k_scan_small, dim3(cols), kScanSmallThreads, c->stream, in, n, totals, out, rep);
     *launches += 1;
     K2J_CUDA(c, cudaGetLastError());

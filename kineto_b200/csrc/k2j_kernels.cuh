@@ -836,8 +836,8 @@ __global__ void __launch_bounds__(kClearThreads) k_clear(const __grid_constant__
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr int kScanSmallThreads = 1024;
-constexpr int kScanSmallTile = kScanSmallThreads * kScanItems;
+constexpr int kScanSmallThreads = 512;
+constexpr int kScanSmallMax = kScanSmallThreads * kScanItems;  // elements of a column that one block scans
 
 // What the host wants to know once a scan is done, written straight to its pinned memory by the scan's last kernel: a
 // copy of eight bytes on the stream costs as much as a small kernel.  `at`: element of the (single) column whose offset goes to at_dst.
@@ -890,19 +890,13 @@ __global__ void __launch_bounds__(kScanSmallThreads) k_scan_small(const uint32_t
   let_next_start();
   wait_for_previous();
   const uint32_t* src = in + (uint64_t)blockIdx.x * n;
-  uint64_t* dst = out + (uint64_t)blockIdx.x * n;
-  uint64_t carry = 0;
-  for (uint64_t t0 = 0; t0 < n; t0 += kScanSmallTile) {
-    const uint64_t base = t0 + (uint64_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    const uint64_t s = scan_load(src, base, n, v);
-    uint64_t tot;
-    const uint64_t ex = carry + block_exclusive_scan<kScanSmallThreads>(s, &tot);
-    scan_store(dst, base, n, v, ex, rep);
-    carry += tot;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { totals[blockIdx.x] = carry; scan_report(rep); }
+  const uint64_t base = (uint64_t)threadIdx.x * kScanItems;
+  uint32_t v[kScanItems];
+  const uint64_t s = scan_load(src, base, n, v);
+  uint64_t tot;
+  const uint64_t ex = block_exclusive_scan<kScanSmallThreads>(s, &tot);
+  scan_store(out + (uint64_t)blockIdx.x * n, base, n, v, ex, rep);
+  if (threadIdx.x == 0) { totals[blockIdx.x] = tot; scan_report(rep); }
 }
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* in, uint64_t n, uint64_t col_stride, uint64_t* block_sums, uint32_t n_blocks) {
   let_next_start();

@@ -207,3 +207,11 @@ def test_class_counts_at_the_edge_of_one_launch(n_chunks):
     assert got[:n_ops_text].cpu().numpy().tobytes() == want[:n_ops_text]
     assert got[n_ops_text + times * first:].cpu().numpy().tobytes() == want[n_ops_text + first:]
     ctx.close()
+
+
+# one launch serves a column of up to 4096 elements (the tests it calls have the sizes of an earlier limit, of 16 384)
+@pytest.mark.parametrize("n", [4095, 4096, 4097])
+def test_the_scan_s_one_launch_ends_at_4096_elements(n):
+    test_exclusive_scan_at_the_edges_of_its_shapes(n)
+    test_class_counts_at_the_edge_of_one_launch(n)
+    test_what_the_scan_reports_at_the_edges_of_its_shapes(n)
