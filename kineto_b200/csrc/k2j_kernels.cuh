@@ -232,15 +232,20 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 // Inserts key -> value; among equal keys the largest value stays (values are positions, so that is
 // the last writer in processing order: std::unordered_map::operator[] assignment semantics,
 // libkineto/src/CuptiActivityProfiler.cpp:293-296, GenericActivityProfiler.cpp:262).
-__device__ __forceinline__ bool tab_insert(unsigned long long* tab, uint32_t mask, uint32_t key, uint32_t value) {
+// A new key is swapped in at once: a load in front would be a second trip to the table (join of 500 k launches 68 us with
+// it, 63 without).  Where the key recurs in the warp (recurs) it is likely to be there, and many swaps on one slot cost
+// more than loads: with 450 k memory events, whose ids are all 0, 87 us with the load, 108 without; 500 k records of one
+// correlation id 48 (the last lane of each warp only, with the load), 390 (every lane, with it), 1020 (every lane, without).
+__device__ __forceinline__ bool tab_insert(unsigned long long* tab, uint32_t mask, uint32_t key, uint32_t value, bool recurs) {
   const unsigned long long entry = ((unsigned long long)key << 32) | (unsigned long long)(value + 1u);
   uint32_t i = hash32(key) & mask;
   for (uint32_t probes = 0; probes <= mask; probes++) {
-    // keys are nearly always new: the swap is tried at once, a load in front of it would be a second trip to the table
-    // (join of 1 M launches 107 us with it, 95 without)
-    const unsigned long long old = atomicCAS(&tab[i], 0ull, entry);
-    if (old == 0) return true;
-    if ((uint32_t)(old >> 32) == key) { atomicMax(&tab[i], entry); return true; }
+    unsigned long long old = recurs ? tab[i] : 0ull;
+    if (old == 0) {
+      old = atomicCAS(&tab[i], 0ull, entry);
+      if (old == 0) return true;
+    }
+    if ((uint32_t)(old >> 32) == key) { if (old < entry) atomicMax(&tab[i], entry); return true; }
     i = (i + 1) & mask;
   }
   return false;
@@ -747,7 +752,7 @@ __global__ void k_build_coll(Dev d) {
   if (i >= d.n_ops) return;
   const uint32_t name = d.op_name[i];
   if (name >= d.n_strings || d.str_class[name] != 1u) return;
-  if (!tab_insert(d.coll_tab, d.coll_mask, (uint32_t)d.op_id[i], (uint32_t)i)) atomicAdd(&d.counters->device_check, 1ull);
+  if (!tab_insert(d.coll_tab, d.coll_mask, (uint32_t)d.op_id[i], (uint32_t)i, false)) atomicAdd(&d.counters->device_check, 1ull);
 }
 // CPU-op id -> position (last writer wins): activityMap_[id] = op, GenericActivityProfiler.cpp:262.
 __device__ __forceinline__ void build_ops(const Dev& d, uint64_t i, uint64_t last) {
@@ -758,32 +763,30 @@ __device__ __forceinline__ void build_ops(const Dev& d, uint64_t i, uint64_t las
   // last, which is the one that must win, goes to the table, so a run of equal ids costs one atomic per warp.
   const uint32_t peers = __match_any_sync(0xffffffffu, id) & __ballot_sync(0xffffffffu, valid);
   if (!valid || (threadIdx.x & 31u) != 31u - (uint32_t)__clz((int)peers)) return;
-  if (!tab_insert(d.op_tab, d.op_mask, id, (uint32_t)i)) atomicAdd(&d.counters->device_check, 1ull);
+  if (!tab_insert(d.op_tab, d.op_mask, id, (uint32_t)i, (peers & (peers - 1u)) != 0u)) atomicAdd(&d.counters->device_check, 1ull);
 }
 // correlation id -> index of the winning EXTERNAL_CORRELATION record (handleCorrelationActivity,
 // CuptiActivityProfiler.cpp:290-302).  `count_invalid`: only the shard that owns a record counts it.
 __device__ __forceinline__ void build_corr(const Dev& d, uint64_t i, uint64_t own_begin, uint64_t own_end) {
-  ExtRec e;
-  if (i >= d.n_ext_all || !ext_at(d, i, &e)) return;
-  bool ok = true;
-  if (e.external_kind == 3u) {
-    if (d.need_corr != nullptr) {
-      // this shard's own records are nearly all wanted by its own events: they go in untested
-      if ((i < own_begin || i >= own_end) && !bit_test(d.need_corr, d.need_corr_mask, e.correlation_id)) return;
-      if ((int64_t)e.external_id == (int64_t)(int32_t)e.external_id) bit_set(d.need_op, d.need_op_mask, (uint32_t)e.external_id);
-    }
-    if (e.correlation_id == 0u) atomicMax(&d.corr0[0], (unsigned long long)i + 1ull);
-    else ok = tab_insert(d.corr_tab, d.corr_mask, e.correlation_id, (uint32_t)i);
-  } else if (e.external_kind == 4u) {
-    atomicAdd(&d.counters->n_user, 1ull);
-    // user-annotation spans: the same filter as above when the keys of several shards were gathered
-    if (d.user_tab != nullptr &&
-        (d.need_corr == nullptr || (i >= own_begin && i < own_end) || bit_test(d.need_corr, d.need_corr_mask, e.correlation_id))) {
-      if (d.need_op != nullptr && (int64_t)e.external_id == (int64_t)(int32_t)e.external_id) bit_set(d.need_op, d.need_op_mask, (uint32_t)e.external_id);
-      ok = tab_insert(d.user_tab, d.user_mask, e.correlation_id, (uint32_t)i);
-    }
-  } else if (i >= own_begin && i < own_end) atomicAdd(&d.counters->invalid_external_correlation, 1ull);
-  if (!ok) atomicAdd(&d.counters->device_check, 1ull);
+  ExtRec e{};
+  const bool in = i < d.n_ext_all && ext_at(d, i, &e), own = i >= own_begin && i < own_end;
+  bool corr = in && e.external_kind == 3u, user = in && e.external_kind == 4u;
+  if (in && !corr && !user && own) atomicAdd(&d.counters->invalid_external_correlation, 1ull);
+  if (user) atomicAdd(&d.counters->n_user, 1ull);
+  user = user && d.user_tab != nullptr;
+  if ((corr || user) && d.need_corr != nullptr) {
+    // keys of several shards were gathered: this shard's own records are nearly all wanted by its own events and go in untested
+    if (!own && !bit_test(d.need_corr, d.need_corr_mask, e.correlation_id)) corr = user = false;
+    else if ((int64_t)e.external_id == (int64_t)(int32_t)e.external_id) bit_set(d.need_op, d.need_op_mask, (uint32_t)e.external_id);
+  }
+  if (corr && e.correlation_id == 0u) { atomicMax(&d.corr0[0], (unsigned long long)i + 1ull); corr = false; }
+  const uint32_t same = __match_any_sync(0xffffffffu, e.correlation_id);
+  const uint32_t corrs = __ballot_sync(0xffffffffu, corr), users = __ballot_sync(0xffffffffu, user);
+  if (!corr && !user) return;
+  const uint32_t peers = same & (corr ? corrs : users);
+  if ((threadIdx.x & 31u) != 31u - (uint32_t)__clz((int)peers)) return;
+  if (!tab_insert(corr ? d.corr_tab : d.user_tab, corr ? d.corr_mask : d.user_mask, e.correlation_id, (uint32_t)i, (peers & (peers - 1u)) != 0u))
+    atomicAdd(&d.counters->device_check, 1ull);
 }
 
 // The join tables in one launch: four independent jobs, each with a range of blocks of its own (a job that is not

@@ -215,3 +215,24 @@ def test_the_scan_s_one_launch_ends_at_4096_elements(n):
     test_exclusive_scan_at_the_edges_of_its_shapes(n)
     test_class_counts_at_the_edge_of_one_launch(n)
     test_what_the_scan_reports_at_the_edges_of_its_shapes(n)
+
+
+# of the lanes of a warp that hold one key only the last goes to a join table: keys that recur in a warp, in every warp, hardly ever
+@pytest.mark.parametrize("distinct", [1, 2, 31, 700])
+def test_join_keys_that_recur(distinct):
+    """The last record of a correlation id wins, in each of the two kinds; so does the last op of an id."""
+    rng = np.random.default_rng(distinct)
+    b = synth.TraceBuilder(n_devices=2, flags=tf.FLAG_USER_ANNOTATIONS)
+    for i in range(400):
+        b.op(b.t0 + i, b.t0 + 10_000 + i, int(rng.integers(0, distinct + 1)), "op%d" % i,
+             type=synth.USER_ANNOTATION if i % 5 == 0 else synth.CPU_OP)
+    for i in range(1500):
+        b.extcorr(int(rng.integers(0, distinct + 1)), int(rng.integers(0, distinct + 3)),
+                  ext_kind=tf.EXTERNAL_KIND_CUSTOM1 if rng.random() < 0.3 else tf.EXTERNAL_KIND_CUSTOM0)
+    for i in range(500):
+        b.kernel(b.t0 + 20 * i, b.t0 + 20 * i + 15, int(rng.integers(0, distinct + 2)), "k%d" % (i % 7), stream=7 + i % 3)
+    trace = b.build()
+    from kineto_b200 import api
+    got, _ = api.process(trace, device=0)
+    want, _ = helpers.run_port(trace)
+    assert got == want, helpers.first_diff(want, got)
