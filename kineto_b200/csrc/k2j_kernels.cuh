@@ -1668,7 +1668,8 @@ __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tal
   s32(a, KS_LSMEM, o1.x); s32(a, KS_LWARPS, o1.y); s32(a, KS_LBLOCKS, o1.z); s32(a, KS_LBARR, o1.w);
   s32(a, KS_AREGS, o2.x); s64(a, KS_ASMEM, pack64(o2.z, o2.w));
   s64(a, KS_BPS, packed ? bps10 : (uint64_t)__double_as_longlong((double)bps));
-  s64(a, KS_WPS, packed ? wps10 : (uint64_t)__double_as_longlong((double)wps));
+  // (infinite blocks of no threads: x86 makes a NaN with the sign bit set of that product, the GPU one without, and the sign is printed)
+  s64(a, KS_WPS, packed ? wps10 : sm_count == 0 && block_prod == 0 ? 0xFFF8000000000000ull : (uint64_t)__double_as_longlong((double)wps));
   s64(a, KS_TS, (uint64_t)rel_ts(d, ts)); s64(a, KS_DUR, (uint64_t)(dur < 0 ? 0 : dur));
   s32(a, KS_REGS, regs); s32(a, KS_SMEM, (uint32_t)ssm + (uint32_t)dsm); s32(a, KS_EXT, (uint32_t)ext);
   uint64_t p = ((1ull << K_COUNT) - 1ull) & ~(1ull << K_COLL);  // every field except the optional ones below

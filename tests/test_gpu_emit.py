@@ -119,3 +119,15 @@ def test_inputs_that_the_default_stream_is_still_writing():
         ctx.run()
         assert ctx.copy_output().tobytes() == want
     ctx.close()
+
+
+def test_a_launch_of_no_threads_on_an_unknown_device():
+    """Infinite blocks per SM times no threads: not a number, with the sign that x86 gives it."""
+    b = synth.TraceBuilder(n_devices=1)
+    for i, block in enumerate([(0, 1, 1), (1, 0, 7), (65536, 65536, 1), (32, 1, 1)]):  # (the third product wraps to 0)
+        for device in (0, 77):
+            b.kernel(b.t0 + 10 * i, b.t0 + 10 * i + 5, 0, "none", device=device, block=block)
+    trace = b.build()
+    want, _ = helpers.run_port(trace)
+    assert want.count(b'"warps per SM": "-nan"') == 3
+    check(trace)
