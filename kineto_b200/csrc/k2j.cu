@@ -1094,10 +1094,15 @@ k2j_status emit_core(k2j_ctx* c, k2j_result* res, const TileSink& sink) {
   K2J_CUDA(c, c->ev_off.reserve(std::max<uint64_t>(1, d.n_events) * 8));
   K2J_CUDA(c, c->ev_ext.reserve(std::max<uint64_t>(1, d.n_events) * 4));
   d.ev_size = c->ev_size.as<uint32_t>(); d.ev_off = c->ev_off.as<uint64_t>(); d.ev_ext = c->ev_ext.as<int32_t>();
-  const uint64_t hand_kernels = d.cls_begin[C_MEMCPY] - d.cls_begin[C_KERNEL], hand_items = d.cls_begin[C_OVERHEAD] - d.cls_begin[C_KERNEL];
-  K2J_CUDA(c, c->hand.reserve(std::max<uint64_t>(1, hand_kernels * (3 * sizeof(uint4) + 8) + hand_items * 8)));
-  d.hand_occ = c->hand.as<uint4>(); d.hand_pitch = hand_kernels;
-  d.hand_wps = reinterpret_cast<uint64_t*>(d.hand_occ + 3 * hand_kernels); d.hand_dec = d.hand_wps + hand_kernels;
+  d.hand_occ = nullptr; d.hand_dec = d.hand_wps = nullptr; d.hand_pitch = 0;
+  if (sink.mode == 0) {
+    // (64 bytes to a kernel event's 1 KB of text, which stays as well.  Text that leaves slab by slab is bound by its way out:
+    // 461 MB to pinned host memory 10.59 ms, with a hand-over 10.57)
+    const uint64_t kernels = d.cls_begin[C_MEMCPY] - d.cls_begin[C_KERNEL], items = d.cls_begin[C_OVERHEAD] - d.cls_begin[C_KERNEL];
+    K2J_CUDA(c, c->hand.reserve(std::max<uint64_t>(1, kernels * (3 * sizeof(uint4) + 8) + items * 8)));
+    d.hand_occ = c->hand.as<uint4>(); d.hand_pitch = kernels;
+    d.hand_wps = reinterpret_cast<uint64_t*>(d.hand_occ + 3 * kernels); d.hand_dec = d.hand_wps + kernels;
+  }
   // With gathered keys only those this shard's events can look up enter its tables (see k_mark_corr), so the tables
   // are sized by the shard: its events, plus the share of foreign keys the marking lets through by chance.
   const bool filter = c->have_global_join;

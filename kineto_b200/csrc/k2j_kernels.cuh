@@ -184,7 +184,8 @@ struct Dev {
   int32_t* ev_ext;        // per event: id of the linked CPU op found by the size pass (0 = none)
   // What the size pass has worked out for the emit pass, per work item of the kernel, copy and memset classes (index 0 =
   // the first kernel): doubles as pack_double's words (kernels: blocks per SM; copies and memsets: the bandwidth), and for
-  // kernels warps per SM and the occupancy calculator's results (hand_occ: 3 rows of hand_pitch).
+  // kernels warps per SM and the occupancy calculator's results (hand_occ: 3 rows of hand_pitch).  nullptr: worked out again
+  // (text that leaves slab by slab: no call of that kind is to hold 64 bytes more for every kernel event).
   uint64_t* hand_dec; uint64_t* hand_wps; uint4* hand_occ; uint64_t hand_pitch;
   uint8_t* out; uint64_t out_cap;  // address of output byte 0 (of the whole text), bytes of the whole text
   // Sharded traces: records in front of guest_front (a slot index) and from guest_back on are other shards' records
@@ -1588,7 +1589,7 @@ __device__ __forceinline__ uint64_t gather_api(const Dev& d, uint32_t* a, Tally&
 }
 
 // computeOccupancyMetrics (libkineto/src/DeviceProperties.cpp:176-222) with NVIDIA's occupancy calculator.
-__device__ __forceinline__ void occupancy_metrics(const Dev& d, uint32_t dev, bool have_dev, int sm_count, int32_t grid_prod,
+__device__ __forceinline__ void occupancy_metrics(const DevProps* props, uint32_t dev, bool have_dev, int sm_count, int32_t grid_prod,
                                                int32_t block_prod, uint32_t regs, int32_t ssm, int32_t dsm, cudaOccResult* out,
                                                float* occupancy_out) {
   cudaOccResult occ;
@@ -1597,7 +1598,7 @@ __device__ __forceinline__ void occupancy_metrics(const Dev& d, uint32_t dev, bo
   occ.allocatedSharedMemPerBlock = 0; occ.partitionedGCConfig = PARTITIONED_GC_OFF;
   float occupancy = -1.0f;  // OccupancyMetrics default (DeviceProperties.h:54)
   if (have_dev) {
-    const DevProps& dp = d.props[dev];
+    const DevProps& dp = props[dev];
     const float blocks_per_sm = sm_count != 0 ? __fdiv_rn(__int2float_rn(grid_prod), __int2float_rn(sm_count)) : -1.0f;
     cudaOccFuncAttributes fa;
     fa.maxThreadsPerBlock = INT_MAX; fa.numRegs = (int)regs; fa.sharedSizeBytes = (size_t)(int64_t)ssm;
@@ -1618,6 +1619,27 @@ __device__ __forceinline__ void occupancy_metrics(const Dev& d, uint32_t dev, bo
   }
   *out = occ;
   *occupancy_out = occupancy;
+}
+
+// The calculator's results as the fields of a kernel event take them.
+struct KernelOcc { uint4 o0, o1, o2; };
+__device__ __forceinline__ KernelOcc kernel_occ(const DevProps* props, uint32_t dev, bool have_dev, int sm_count, int32_t grid_prod, int32_t block_prod,
+                                                uint32_t regs, int32_t ssm, int32_t dsm) {
+  cudaOccResult occ;
+  float occupancy;
+  occupancy_metrics(props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm, &occ, &occupancy);
+  const uint64_t asmem = (uint64_t)occ.allocatedSharedMemPerBlock;
+  KernelOcc k;
+  k.o0 = make_uint4((uint32_t)(int32_t)llround(__dmul_rn((double)occupancy, 100.0)), (uint32_t)occ.activeBlocksPerMultiprocessor,
+                    (uint32_t)(CS_LIMIT + (int)(occ.limitingFactors & 31u)), (uint32_t)occ.blockLimitRegs);
+  k.o1 = make_uint4((uint32_t)occ.blockLimitSharedMem, (uint32_t)occ.blockLimitWarps, (uint32_t)occ.blockLimitBlocks, (uint32_t)occ.blockLimitBarriers);
+  k.o2 = make_uint4((uint32_t)occ.allocatedRegistersPerBlock, 0u, (uint32_t)asmem, (uint32_t)(asmem >> 32));
+  return k;
+}
+// out of line: the emit pass without a hand-over
+__device__ __noinline__ KernelOcc kernel_occ_again(const DevProps* props, uint32_t dev, bool have_dev, int sm_count, int32_t grid_prod, int32_t block_prod,
+                                                   uint32_t regs, int32_t ssm, int32_t dsm) {
+  return kernel_occ(props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
 }
 
 // GpuActivity<Kernel> (libkineto/src/CuptiActivity.h:499-576)
@@ -1645,28 +1667,26 @@ __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tal
   // The calculator's results and the digits of both doubles are worked out once, by the size pass: in the emit pass they
   // took 61 of a kernel event's 456 warp instructions; 64 bytes written and read stand for them.
   const uint64_t h = t.work - d.cls_begin[C_KERNEL];
-  uint4 o0, o1, o2;
+  KernelOcc k;
   uint64_t bps10, wps10;
   if (counting) {
-    cudaOccResult occ;
-    float occupancy;
-    occupancy_metrics(d, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm, &occ, &occupancy);
-    const uint64_t asmem = (uint64_t)occ.allocatedSharedMemPerBlock;
-    o0 = make_uint4((uint32_t)(int32_t)llround(__dmul_rn((double)occupancy, 100.0)), (uint32_t)occ.activeBlocksPerMultiprocessor,
-                    (uint32_t)(CS_LIMIT + (int)(occ.limitingFactors & 31u)), (uint32_t)occ.blockLimitRegs);
-    o1 = make_uint4((uint32_t)occ.blockLimitSharedMem, (uint32_t)occ.blockLimitWarps, (uint32_t)occ.blockLimitBlocks, (uint32_t)occ.blockLimitBarriers);
-    o2 = make_uint4((uint32_t)occ.allocatedRegistersPerBlock, 0u, (uint32_t)asmem, (uint32_t)(asmem >> 32));
+    k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
     bps10 = pack_double((double)bps); wps10 = pack_double((double)wps);
-    d.hand_occ[h] = o0; d.hand_occ[d.hand_pitch + h] = o1; d.hand_occ[2 * d.hand_pitch + h] = o2;
-    d.hand_dec[h] = bps10; d.hand_wps[h] = wps10;
-  } else {
-    o0 = d.hand_occ[h]; o1 = d.hand_occ[d.hand_pitch + h]; o2 = d.hand_occ[2 * d.hand_pitch + h];
+    if (d.hand_occ != nullptr) {
+      d.hand_occ[h] = k.o0; d.hand_occ[d.hand_pitch + h] = k.o1; d.hand_occ[2 * d.hand_pitch + h] = k.o2;
+      d.hand_dec[h] = bps10; d.hand_wps[h] = wps10;
+    }
+  } else if (d.hand_occ != nullptr) {
+    k.o0 = d.hand_occ[h]; k.o1 = d.hand_occ[d.hand_pitch + h]; k.o2 = d.hand_occ[2 * d.hand_pitch + h];
     bps10 = d.hand_dec[h]; wps10 = d.hand_wps[h];
+  } else {
+    k = kernel_occ_again(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
+    bps10 = wps10 = 0ull;
   }
   const bool packed = bps10 != 0ull && wps10 != 0ull;
-  s32(a, KS_PCT, o0.x); s32(a, KS_ACTIVE, o0.y); s32(a, KS_LIMIT, o0.z); s32(a, KS_LREGS, o0.w);
-  s32(a, KS_LSMEM, o1.x); s32(a, KS_LWARPS, o1.y); s32(a, KS_LBLOCKS, o1.z); s32(a, KS_LBARR, o1.w);
-  s32(a, KS_AREGS, o2.x); s64(a, KS_ASMEM, pack64(o2.z, o2.w));
+  s32(a, KS_PCT, k.o0.x); s32(a, KS_ACTIVE, k.o0.y); s32(a, KS_LIMIT, k.o0.z); s32(a, KS_LREGS, k.o0.w);
+  s32(a, KS_LSMEM, k.o1.x); s32(a, KS_LWARPS, k.o1.y); s32(a, KS_LBLOCKS, k.o1.z); s32(a, KS_LBARR, k.o1.w);
+  s32(a, KS_AREGS, k.o2.x); s64(a, KS_ASMEM, pack64(k.o2.z, k.o2.w));
   s64(a, KS_BPS, packed ? bps10 : (uint64_t)__double_as_longlong((double)bps));
   // (infinite blocks of no threads: x86 makes a NaN with the sign bit set of that product, the GPU one without, and the sign is printed)
   s64(a, KS_WPS, packed ? wps10 : sm_count == 0 && block_prod == 0 ? 0xFFF8000000000000ull : (uint64_t)__double_as_longlong((double)wps));
@@ -1732,8 +1752,11 @@ __device__ __forceinline__ uint64_t gather_mem(const Dev& d, uint32_t* a, Tally&
   if (dur != 0) {  // addBandwidthTypedMetadata, CuptiActivity.h:460-470
     const uint64_t h = t.work - d.cls_begin[C_KERNEL];
     uint64_t bw10;
-    if (counting) d.hand_dec[h] = bw10 = pack_double(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur)));
-    else bw10 = d.hand_dec[h];
+    if (!counting) bw10 = d.hand_dec != nullptr ? d.hand_dec[h] : 0ull;
+    else {
+      bw10 = pack_double(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur)));
+      if (d.hand_dec != nullptr) d.hand_dec[h] = bw10;
+    }
     on(bw10 != 0ull ? M_BW : M_BWRAW);
     s64(a, MS_BW, bw10 != 0ull ? bw10 : (uint64_t)__double_as_longlong(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur))));
   }

@@ -131,3 +131,33 @@ def test_a_launch_of_no_threads_on_an_unknown_device():
     want, _ = helpers.run_port(trace)
     assert want.count(b'"warps per SM": "-nan"') == 3
     check(trace)
+
+
+def test_slabs_hold_what_the_resident_text_does_for_every_kind_of_kernel_and_copy():
+    """Text that leaves slab by slab works out occupancy and rates again: odd launches, an unknown device, copies of any length."""
+    import torch
+    from kineto_b200 import api
+    rng = np.random.default_rng(71)
+    trace = synth.gen_mixed(1500, seed=72, pool_size=60, n_devices=4)
+    kern, at = kernel_records(trace)
+    for name, of in (("registersPerThread", [0, 1, 32, 255, 256, 65535]), ("staticSharedMemory", [0, 1, 48 << 10, 227 << 10, 1 << 30]),
+                     ("dynamicSharedMemory", [0, 100, 164 << 10, 1 << 28]), ("blockX", [0, 1, 31, 1024, 4096]), ("gridX", [0, 1, 147, 2**31 - 1]),
+                     ("deviceId", [0, 1, 3, 4, 77])):
+        kern[name] = np.where(rng.random(len(kern)) < 0.5, rng.choice(np.array(of), len(kern)).astype(kern[name].dtype), kern[name])
+    cupti = trace.cupti.copy()
+    for a, r in zip(at, kern.view(np.uint8).reshape(len(at), 208)):
+        cupti[a:a + 208] = r
+    trace.cupti = cupti
+    want = helpers.run_port(trace)[0]
+    ctx = api.K2J(0)
+    text = torch.zeros(len(want) + 1000, dtype=torch.uint8)
+    for resident in (False, True, False):
+        ctx.load(trace)
+        if resident:
+            ctx.run()
+            got = ctx.copy_output().tobytes()
+        else:
+            ctx.segment(sync=False)
+            got = text[:ctx.emit_to_host(text)["out_bytes"]].numpy().tobytes()
+        assert got == want, helpers.first_diff(want, got)
+    ctx.close()

@@ -162,3 +162,30 @@ def test_the_emit_pass_spreads_over_the_sms_that_the_gpu_has(fake):
 
         assert [threads(132 * 2 * k + more) for k, more in ((1, 0), (64, 0), (64, 1), (96, 0), (96, 1), (320, 0), (320, 1))] == [64, 64, 96, 96, 128, 320, 320]
     """)
+
+
+def test_text_that_leaves_slab_by_slab_takes_no_hand_over(fake):
+    """What the size pass works out for the emit pass is kept where the text is kept; the calls that bound memory hold a few
+    words an event."""
+    run(fake, """
+        n = 1 << 20
+        columns = np.zeros(13, np.uint64)
+        columns[[1, 12]] = n              # kernel records, records that own an event
+        fake.fake_columns(C.c_void_p(columns.ctypes.data), 13)
+        data, table = np.zeros(4096, np.uint8), np.array([0, 4096], np.uint64)
+        assert lib.k2j_set_cupti(ctx, data.ctypes.data, 4096, table.ctypes.data, 1) == OK
+        fake.fake_scan_total(1 << 20)
+        text, result = np.zeros(1 << 20, np.uint8), api.Result()
+        largest = []
+        for slabs in (True, False):
+            log()
+            assert lib.k2j_segment(ctx, None) == OK
+            if slabs:
+                assert lib.k2j_emit_to_host(ctx, text.ctypes.data, text.nbytes, 0, C.byref(result)) == OK
+            else:
+                assert lib.k2j_emit(ctx, C.byref(result)) == OK
+            lines = log()
+            assert sum("k_events" in l[1] for l in lines if l[0] == "launch") >= 1
+            largest.append(max([int(l[2]) for l in lines if l[0] == "alloc"], default=0))
+        assert largest[0] < 16 * n and largest[1] >= 64 * n
+    """)
