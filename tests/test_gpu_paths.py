@@ -236,3 +236,22 @@ def test_join_keys_that_recur(distinct):
     got, _ = api.process(trace, device=0)
     want, _ = helpers.run_port(trace)
     assert got == want, helpers.first_diff(want, got)
+
+
+# lists of up to 4096 spans are ordered by the GPU, longer ones by the host
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 6001])
+def test_traces_of_many_spans(n):
+    """Three annotations over that many spans of (device, stream) rows, first used in any order."""
+    from kineto_b200 import api
+    rng = np.random.default_rng(n)
+    b = synth.TraceBuilder(n_devices=8, flags=tf.FLAG_USER_ANNOTATIONS)
+    for a in range(3):
+        b.op(b.t0 + a, b.t0 + 1_000_000, 1 + a, "step %d" % a, type=synth.USER_ANNOTATION)
+    for i, k in enumerate(np.concatenate([rng.permutation(n), rng.integers(0, n, 500)]).tolist()):
+        b.extcorr(1 + i, 1 + k % 3, ext_kind=tf.EXTERNAL_KIND_CUSTOM1)
+        b.kernel(b.t0 + 20 * i, b.t0 + 20 * i + 15, 1 + i, "k", device=k // 3 % 8, stream=k // 24)
+    trace = b.build()
+    want, _ = helpers.run_port(trace)
+    assert want.count(b'"cat": "gpu_user_annotation"') == n
+    got, _ = api.process(trace, device=0)
+    assert got == want, helpers.first_diff(want, got)
