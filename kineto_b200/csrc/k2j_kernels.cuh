@@ -2081,9 +2081,7 @@ __device__ __forceinline__ void put_counters(S& s, const Dev& d, uint32_t row, b
 // entries of the op (JsonTypedMetadataVisitor, libkineto/include/TypedMetadataJson.h:72-158): each entry
 // is mapped onto one of the value types, so the kernel holds one copy of every formatter.
 enum : int { T_BOOL = 8, T_MDSTR, T_QMDSTR };
-// ENSURE = false: the caller has asked the sink for room for a number; fields that loop over entries or copy
-// strings still ask for themselves.
-template <class S, bool COLL = true, bool ENSURE = true>
+template <class S, bool COLL = true>
 __device__ __forceinline__ void put_value(S& s, const Dev& d, int type, uint64_t v, unsigned long long* name_bytes) {
   if (type == T_NONE) return;
   if (COLL && (type == T_MDCNT || type == T_HWC)) { put_counters(s, d, (uint32_t)v, type == T_HWC); return; }
@@ -2099,7 +2097,7 @@ __device__ __forceinline__ void put_value(S& s, const Dev& d, int type, uint64_t
   }
   bool more = false, close_quote = false;
   do {
-    if (ENSURE || md_mode) s.ensure(48);  // a number takes at most 24 bytes; quotes and separators around it come out of the sink's slack
+    s.ensure(48);  // a number takes at most 24 bytes; quotes and separators around it come out of the sink's slack
     if (md_mode) {
       if (!coll) {
         close_quote = false;
@@ -2149,7 +2147,7 @@ __device__ __forceinline__ void put_value(S& s, const Dev& d, int type, uint64_t
         if (COLL && coll && !double_is_finite(x)) put_nonfinite(s, x); else put_dbl(s, x);
         break;
       }
-      case T_DEC: put_packed_double(s, v); break;
+      case T_DEC: if constexpr (S::kCounting) put_packed_double(s, v); break;  // (written by run_steps only: app_dec)
       case T_NAME: put_name(s, d, (uint32_t)v, name_bytes); break;
       case T_CSTR: { const FieldDesc cs = g_fields.f[CSTR_BASE + (uint32_t)v]; s.words(g_fields.w + cs.off, cs.len); break; }
       case T_BOOL: if (v) s.put4(0x65757274u); else s.put64(0x65736C6166ull, 5); break;  // true / false
@@ -2516,7 +2514,7 @@ template <int R, bool COLL> __device__ __forceinline__ void put_run(InlineSink& 
       put_pool_name(s, d, a[w]);
       st = sink_state(s);
     } else {  // metadata entries: they ask the sink for room themselves
-      if constexpr (COLL || I::type != T_COLL) put_value<InlineSink, COLL, true>(s, d, I::type, (uint64_t)a[w], name_bytes);
+      if constexpr (COLL || I::type != T_COLL) put_value<InlineSink, COLL>(s, d, I::type, (uint64_t)a[w], name_bytes);
       st = sink_state(s);
     }
     s.pos = (uint32_t)st; s.carry = (uint32_t)(st >> 32);
