@@ -126,10 +126,14 @@ k2j_status fail(k2j_ctx* c, k2j_status st, const char* fmt, ...) {
   if (c) c->err = buf;
   return st;
 }
+// (the runtime keeps the error of a failed call; left there, the next check behind a launch would report it again)
 #define K2J_CUDA(ctx, call)                                                                       \
   do {                                                                                            \
     cudaError_t _e = (call);                                                                      \
-    if (_e != cudaSuccess) return fail(ctx, K2J_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e)); \
+    if (_e != cudaSuccess) {                                                                      \
+      cudaGetLastError();                                                                         \
+      return fail(ctx, K2J_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(_e));                    \
+    }                                                                                             \
   } while (0)
 
 bool is_device_ptr(const void* p) {
@@ -424,7 +428,7 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
   // the emit kernels' shared memory (record areas + output windows) is above the 48 KiB that needs no opt-in
   ok = ok && cudaFuncSetAttribute(k_events<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess &&
        cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
-  if (!ok) { k2j_destroy(c); return K2J_ERR_CUDA; }
+  if (!ok) { k2j_destroy(c); cudaGetLastError(); return K2J_ERR_CUDA; }
   c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
   c->sms = (uint32_t)sms;
   *out = c;

@@ -18,6 +18,7 @@ size_t g_most = ~(size_t)0;                       // larger allocations fail
 uint64_t g_pool_total = 0;                        // what the segmentation's first launch reports as the pool's size
 uint64_t g_scan_total = 0;                        // what scans report as the (first) column's total, unless 0
 std::vector<uint64_t> g_columns;                  // what the scan of the chunks' class counts reports, unless empty
+cudaError_t g_last = cudaSuccess;                 // of a call that failed, until it is asked for
 uintptr_t g_handle = 0x1000;
 thread_local struct { dim3 grid, block; size_t smem; void* stream; } g_conf;
 
@@ -74,7 +75,7 @@ void __cudaRegisterFunction(void**, const char* stub, char*, const char* name, i
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
 
 cudaError_t cudaMalloc(void** p, size_t n) {
-  if (n > g_most) { *p = nullptr; return cudaErrorMemoryAllocation; }
+  if (n > g_most) { *p = nullptr; return g_last = cudaErrorMemoryAllocation; }
   *p = calloc(1, n ? n : 1);
   g_device[(uintptr_t)*p] = n ? n : 1;
   note("alloc", *p, n);
@@ -108,7 +109,7 @@ cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return c
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() { const cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t) { return "out of memory"; }
 cudaError_t cudaGetSymbolAddress(void** p, const void*) { *p = nullptr; return cudaErrorInvalidSymbol; }
 }

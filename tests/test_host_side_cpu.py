@@ -189,3 +189,17 @@ def test_text_that_leaves_slab_by_slab_takes_no_hand_over(fake):
             largest.append(max([int(l[2]) for l in lines if l[0] == "alloc"], default=0))
         assert largest[0] < 16 * n and largest[1] >= 64 * n
     """)
+
+
+def test_a_failed_allocation_is_reported_once(fake):
+    """The runtime holds the error of a failed call until it is asked for; a later run that has its memory is not refused for it."""
+    run(fake, """
+        n = 1 << 16
+        cols, off = [np.zeros(n, np.int64) for _ in range(10)], np.zeros(n + 1, np.uint32)
+        ops = api.Ops(n, *[a.ctypes.data for a in cols], off.ctypes.data, None)
+        for most, want in ((1 << 16, CUDA), (1 << 40, OK)):
+            fake.fake_most(most)
+            assert lib.k2j_set_ops(ctx, C.byref(ops)) == want
+        fake.fake_scan_total(100 * n)
+        assert lib.k2j_run(ctx, C.byref(api.Result())) == OK
+    """)
