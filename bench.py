@@ -51,7 +51,7 @@ FALLBACK_HBM_GBS = 6650.0
 # wrote, from ncu captures of whole launches at size argument 1 000 000 (1.5 and 1.9 GB of text, far beyond the L2;
 # profiles/emit_kernel_dram_traffic.txt).  Traffic grows in proportion to the text, so the line scales it to the
 # launch it timed; workloads without a capture report null.
-EMIT_TRAFFIC_PER_OUT_BYTE = {"mixed": 2254.8 / 1510.1, "kernel_launches": 2637.2 / 1858.1}
+EMIT_TRAFFIC_PER_OUT_BYTE = {"mixed": 2302.2 / 1510.1, "kernel_launches": 2719.7 / 1858.1}
 SLAB_BYTES = 256 << 20
 REF_DRIVER = os.path.join(ROOT, "oracle", "_ref", "ref_driver")
 
