@@ -426,8 +426,8 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
   for (auto& e : c->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&c->default_ev, cudaEventDisableTiming) == cudaSuccess;
   // the emit kernels' shared memory (record areas + output windows) is above the 48 KiB that needs no opt-in
-  ok = ok && cudaFuncSetAttribute(k_events<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess &&
-       cudaFuncSetAttribute(k_events<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
+  for (auto* kernel : {k_events<true, false>, k_events<true, true>, k_events_slab<false>, k_events_slab<true>})
+    ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
   if (!ok) { k2j_destroy(c); cudaGetLastError(); return K2J_ERR_CUDA; }
   c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
   c->sms = (uint32_t)sms;
@@ -1026,12 +1026,14 @@ int emit_threads(uint64_t items, uint32_t sms) {
 // The emit launches for the events whose text starts in [d.tile_begin, d.tile_end).  `ranges`: per class the work
 // items to look at ([begin, end) pairs, C_API .. C_WAIT, then the CPU-side activities); nullptr: everything.
 k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool instant, uint64_t n_coll, cudaStream_t s) {
+  auto* const main = d.hand_occ != nullptr ? k_events<true, false> : k_events_slab<false>;
+  auto* const rare = d.hand_occ != nullptr ? k_events<true, true> : k_events_slab<true>;
   auto launch = [&](uint64_t begin, uint64_t end) {
     if (end <= begin) return;
     Dev dr = d;
     dr.work_origin = begin; dr.n_work = end;
     const int threads = emit_threads(end - begin, c->sms);
-    k_events<true><<<(uint32_t)((end - begin + threads - 1) / threads), threads, emit_smem_bytes(threads), s>>>(dr);
+    main<<<(uint32_t)((end - begin + threads - 1) / threads), threads, emit_smem_bytes(threads), s>>>(dr);
     c->launches++;
   };
   if (!ranges) launch(0, d.n_work);
@@ -1042,7 +1044,7 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     di.work_origin = ranges ? ranges[2 * C_EXT] : d.ops_begin;
     di.n_work = ranges ? ranges[2 * C_EXT + 1] : d.n_work;
     if (di.n_work > di.work_origin) {
-      k_events<true, true><<<(uint32_t)((di.n_work - di.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(di);
+      rare<<<(uint32_t)((di.n_work - di.work_origin + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(di);
       c->launches++;
     }
   }
@@ -1051,7 +1053,7 @@ k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool in
     // listed, so that the launch above holds no code for them
     Dev dk = d;
     dk.work_indirect = d.coll_list; dk.n_indirect = n_coll;
-    k_events<true, true><<<(uint32_t)((dk.n_indirect + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(dk);
+    rare<<<(uint32_t)((dk.n_indirect + kEventThreads - 1) / kEventThreads), kEventThreads, emit_smem_bytes(kEventThreads), s>>>(dk);
     c->launches++;
   }
   K2J_CUDA(c, cudaGetLastError());

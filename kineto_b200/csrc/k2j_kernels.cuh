@@ -185,7 +185,7 @@ struct Dev {
   // What the size pass has worked out for the emit pass, per work item of the kernel, copy and memset classes (index 0 =
   // the first kernel): doubles as pack_double's words (kernels: blocks per SM; copies and memsets: the bandwidth), and for
   // kernels warps per SM and the occupancy calculator's results (hand_occ: 3 rows of hand_pitch).  nullptr: worked out again
-  // (text that leaves slab by slab: no call of that kind is to hold 64 bytes more for every kernel event).
+  // by k_events_slab (text that leaves slab by slab: no call of that kind is to hold 64 bytes more for every kernel event).
   uint64_t* hand_dec; uint64_t* hand_wps; uint4* hand_occ; uint64_t hand_pitch;
   uint8_t* out; uint64_t out_cap;  // address of output byte 0 (of the whole text), bytes of the whole text
   // Sharded traces: records in front of guest_front (a slot index) and from guest_back on are other shards' records
@@ -1636,14 +1636,9 @@ __device__ __forceinline__ KernelOcc kernel_occ(const DevProps* props, uint32_t 
   k.o2 = make_uint4((uint32_t)occ.allocatedRegistersPerBlock, 0u, (uint32_t)asmem, (uint32_t)(asmem >> 32));
   return k;
 }
-// out of line: the emit pass without a hand-over
-__device__ __noinline__ KernelOcc kernel_occ_again(const DevProps* props, uint32_t dev, bool have_dev, int sm_count, int32_t grid_prod, int32_t block_prod,
-                                                   uint32_t regs, int32_t ssm, int32_t dsm) {
-  return kernel_occ(props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
-}
 
 // GpuActivity<Kernel> (libkineto/src/CuptiActivity.h:499-576)
-__device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tally& t, uint32_t* filt, bool counting, int32_t* ext_io) {
+template <bool HAND> __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tally& t, uint32_t* filt, bool counting, int32_t* ext_io) {
   const unsigned long long corr_first = counting ? linked_op_peek(d, a32(a, KR_CORR)) : 0ull;  // issued early
   const uint64_t st = a64(a, 16), en = a64(a, 24);
   const int64_t ts = conv_ts(d, st), dur = conv_dur(d, st, en);
@@ -1670,20 +1665,17 @@ __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tal
   const uint64_t h = t.work - d.cls_begin[C_KERNEL];
   KernelOcc k;
   uint64_t bps10, wps10;
+  if (counting || !HAND) k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
   if (counting) {
-    k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
     bps10 = pack_double((double)bps); wps10 = pack_double((double)wps);
     if (d.hand_occ != nullptr) {
       d.hand_occ[h] = k.o0; d.hand_occ[d.hand_pitch + h] = k.o1; d.hand_occ[2 * d.hand_pitch + h] = k.o2;
       d.hand_dec[h] = bps10; d.hand_wps[h] = wps10;
     }
-  } else if (d.hand_occ != nullptr) {
+  } else if (HAND) {
     k.o0 = d.hand_occ[h]; k.o1 = d.hand_occ[d.hand_pitch + h]; k.o2 = d.hand_occ[2 * d.hand_pitch + h];
     bps10 = d.hand_dec[h]; wps10 = d.hand_wps[h];
-  } else {
-    k = kernel_occ_again(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
-    bps10 = wps10 = 0ull;
-  }
+  } else bps10 = wps10 = 0ull;
   const bool packed = bps10 != 0ull && wps10 != 0ull;
   s32(a, KS_PCT, k.o0.x); s32(a, KS_ACTIVE, k.o0.y); s32(a, KS_LIMIT, k.o0.z); s32(a, KS_LREGS, k.o0.w);
   s32(a, KS_LSMEM, k.o1.x); s32(a, KS_LWARPS, k.o1.y); s32(a, KS_LBLOCKS, k.o1.z); s32(a, KS_LBARR, k.o1.w);
@@ -1715,7 +1707,7 @@ __device__ __forceinline__ uint64_t gather_kernel(const Dev& d, uint32_t* a, Tal
 }
 
 // memcpy / memcpy2 / memset records (libkineto/src/CuptiActivity.h:586-712)
-template <int CLS>
+template <int CLS, bool HAND>
 __device__ __forceinline__ uint64_t gather_mem(const Dev& d, uint32_t* a, Tally& t, uint32_t* filt, bool counting, int32_t* ext_io) {
   const uint64_t st = a64(a, 16), en = a64(a, 24);
   const int64_t ts = conv_ts(d, st), dur = conv_dur(d, st, en);
@@ -1753,7 +1745,7 @@ __device__ __forceinline__ uint64_t gather_mem(const Dev& d, uint32_t* a, Tally&
   if (dur != 0) {  // addBandwidthTypedMetadata, CuptiActivity.h:460-470
     const uint64_t h = t.work - d.cls_begin[C_KERNEL];
     uint64_t bw10;
-    if (!counting) bw10 = d.hand_dec != nullptr ? d.hand_dec[h] : 0ull;
+    if (!counting) bw10 = HAND ? d.hand_dec[h] : 0ull;
     else {
       bw10 = pack_double(__ddiv_rn(__ull2double_rn(bytes), __ll2double_rn(dur)));
       if (d.hand_dec != nullptr) d.hand_dec[h] = bw10;
@@ -2559,18 +2551,18 @@ static_assert(kEmitBlocks * (emit_smem_bytes(kEmitThreads) + 1024) <= 228 * 1024
 
 // COLL (emit pass only): this launch writes the kernel events that carry collective metadata, and only those; the
 // launch without it writes everything else and holds no code for them.  Returns false when the event is left to
-// the other launch.
-template <class S, bool COLL = true>
+// the other launch.  HAND: the size pass has handed values over (Dev::hand_*).
+template <class S, bool COLL = true, bool HAND = true>
 __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32_t* a, uint64_t j, Tally& t, uint32_t* filt, int32_t* ext) {
   unsigned long long* nb = &t.name_bytes;
   if constexpr (S::kCounting) {
     uint64_t p;
     switch (cls) {  // straight-line field code per class
       case C_API: if ((p = gather_api(d, a, t, filt, true, ext))) count_fields<API_BASE, 0, A_COUNT>(s, d, a, p, nb); break;
-      case C_KERNEL: if ((p = gather_kernel(d, a, t, filt, true, ext))) count_fields<KERNEL_BASE, 0, K_COUNT>(s, d, a, p, nb); break;
-      case C_MEMCPY: if ((p = gather_mem<C_MEMCPY>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
-      case C_MEMCPY2: if ((p = gather_mem<C_MEMCPY2>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
-      case C_MEMSET: if ((p = gather_mem<C_MEMSET>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
+      case C_KERNEL: if ((p = gather_kernel<HAND>(d, a, t, filt, true, ext))) count_fields<KERNEL_BASE, 0, K_COUNT>(s, d, a, p, nb); break;
+      case C_MEMCPY: if ((p = gather_mem<C_MEMCPY, HAND>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
+      case C_MEMCPY2: if ((p = gather_mem<C_MEMCPY2, HAND>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
+      case C_MEMSET: if ((p = gather_mem<C_MEMSET, HAND>(d, a, t, filt, true, ext))) count_fields<MEM_BASE, 0, M_COUNT>(s, d, a, p, nb); break;
       case C_OVERHEAD: if ((p = gather_overhead(d, a, t, filt))) count_fields<OP_BASE, 0, O_COUNT>(s, d, a, p, nb); break;
       case C_SYNC: if ((p = gather_sync<C_SYNC>(d, a, t, filt, true, ext))) count_fields<SYNC_BASE, 0, Y_COUNT>(s, d, a, p, nb); break;
       case C_WAIT: if ((p = gather_sync<C_WAIT>(d, a, t, filt, true, ext))) count_fields<SYNC_BASE, 0, Y_COUNT>(s, d, a, p, nb); break;
@@ -2582,10 +2574,10 @@ __device__ __forceinline__ bool format_event(S& s, const Dev& d, int cls, uint32
     int base;
     switch (cls) {
       case C_API: p = gather_api(d, a, t, filt, false, ext); base = API_BASE; break;
-      case C_KERNEL: p = gather_kernel(d, a, t, filt, false, ext); base = KERNEL_BASE; break;
-      case C_MEMCPY: p = gather_mem<C_MEMCPY>(d, a, t, filt, false, ext); base = MEM_BASE; break;
-      case C_MEMCPY2: p = gather_mem<C_MEMCPY2>(d, a, t, filt, false, ext); base = MEM_BASE; break;
-      case C_MEMSET: p = gather_mem<C_MEMSET>(d, a, t, filt, false, ext); base = MEM_BASE; break;
+      case C_KERNEL: p = gather_kernel<HAND>(d, a, t, filt, false, ext); base = KERNEL_BASE; break;
+      case C_MEMCPY: p = gather_mem<C_MEMCPY, HAND>(d, a, t, filt, false, ext); base = MEM_BASE; break;
+      case C_MEMCPY2: p = gather_mem<C_MEMCPY2, HAND>(d, a, t, filt, false, ext); base = MEM_BASE; break;
+      case C_MEMSET: p = gather_mem<C_MEMSET, HAND>(d, a, t, filt, false, ext); base = MEM_BASE; break;
       case C_OVERHEAD: p = gather_overhead(d, a, t, filt); base = OP_BASE; break;
       case C_SYNC: p = gather_sync<C_SYNC>(d, a, t, filt, false, ext); base = SYNC_BASE; break;
       case C_WAIT: p = gather_sync<C_WAIT>(d, a, t, filt, false, ext); base = SYNC_BASE; break;
@@ -2624,8 +2616,7 @@ __device__ __forceinline__ uint32_t class_units(int cls) {
 // the bytes at ev_off[event].  Either pass first copies the 32 records of a warp into shared memory
 // with coalesced loads (lane = 8-byte unit of a record); all later reads of record fields and of the
 // values computed from them are shared-memory reads at table-given offsets.
-template <bool WRITE, bool COLL = false>
-__global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? kEmitBlocks : 8) k_events(Dev d) {
+template <bool WRITE, bool COLL, bool HAND> __device__ __forceinline__ void events(const Dev& d) {
   const uint32_t threads = WRITE ? blockDim.x : (uint32_t)kEventThreads;
   uint64_t* const s_rec = reinterpret_cast<uint64_t*>(s_dyn + (WRITE ? sizeof(Digits3) / 16 : 0));
   uint32_t* const s_win = reinterpret_cast<uint32_t*>(s_rec + threads * kRecStride);
@@ -2714,7 +2705,7 @@ __global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? 
     } else {
       InlineSink s;
       s.init(d.out + off, size, (Win)__cvta_generic_to_shared(s_win + (threadIdx.x >> 5) * (kWinWords * kWinStride) + (threadIdx.x & 31u)));
-      if (format_event<InlineSink, COLL>(s, d, cls, area, j, t, &filt, &ext) && !s.finish(d.out + off, size))
+      if (format_event<InlineSink, COLL, HAND>(s, d, cls, area, j, t, &filt, &ext) && !s.finish(d.out + off, size))
         atomicAdd(&d.counters->device_check, 1ull);
     }
   }
@@ -2742,6 +2733,11 @@ __global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? 
     }
   }
 }
+template <bool WRITE, bool COLL = false>
+__global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? kEmitBlocks : 8) k_events(Dev d) { events<WRITE, COLL, true>(d); }
+// The emit pass without a hand-over from the size pass.  A kernel of its own: the choice inside k_events, with the calculator
+// out of line, cost the emit pass of 100 k launches 1 us of 162.
+template <bool COLL> __global__ void __launch_bounds__(kEmitThreads, kEmitBlocks) k_events_slab(Dev d) { events<true, COLL, false>(d); }
 
 // ---- tiled runs: which events and which work items belong to each slab of the output ----
 // Slab t holds the events whose text starts in [t * slab, (t + 1) * slab).  bounds is a (n_tiles + 1) x
