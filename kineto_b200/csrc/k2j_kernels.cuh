@@ -781,11 +781,15 @@ __device__ __forceinline__ void build_corr(const Dev& d, uint64_t i, uint64_t ow
     else if ((int64_t)e.external_id == (int64_t)(int32_t)e.external_id) bit_set(d.need_op, d.need_op_mask, (uint32_t)e.external_id);
   }
   if (corr && e.correlation_id == 0u) { atomicMax(&d.corr0[0], (unsigned long long)i + 1ull); corr = false; }
-  const uint32_t same = __match_any_sync(0xffffffffu, e.correlation_id);
-  const uint32_t corrs = __ballot_sync(0xffffffffu, corr), users = __ballot_sync(0xffffffffu, user);
-  if (!corr && !user) return;
-  const uint32_t peers = same & (corr ? corrs : users);
-  if ((threadIdx.x & 31u) != 31u - (uint32_t)__clz((int)peers)) return;
+  // As for the ops, of the lanes that hold one id only the last inserts it, in each kind; but ids hardly ever recur here, so
+  // the lanes are matched only where two neighbours agree.
+  const uint32_t lane = threadIdx.x & 31u, left = __shfl_up_sync(0xffffffffu, e.correlation_id, 1);
+  uint32_t peers = 1u << lane;
+  if (__any_sync(0xffffffffu, lane != 0u && left == e.correlation_id)) {
+    const uint32_t corrs = __ballot_sync(0xffffffffu, corr), users = __ballot_sync(0xffffffffu, user);
+    peers = __match_any_sync(0xffffffffu, e.correlation_id) & (corr ? corrs : users);
+  }
+  if ((!corr && !user) || lane != 31u - (uint32_t)__clz((int)peers)) return;
   if (!tab_insert(corr ? d.corr_tab : d.user_tab, corr ? d.corr_mask : d.user_mask, e.correlation_id, (uint32_t)i, (peers & (peers - 1u)) != 0u))
     atomicAdd(&d.counters->device_check, 1ull);
 }
@@ -1665,17 +1669,20 @@ template <bool HAND> __device__ __forceinline__ uint64_t gather_kernel(const Dev
   const uint64_t h = t.work - d.cls_begin[C_KERNEL];
   KernelOcc k;
   uint64_t bps10, wps10;
-  if (counting || !HAND) k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
   if (counting) {
+    k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
     bps10 = pack_double((double)bps); wps10 = pack_double((double)wps);
     if (d.hand_occ != nullptr) {
       d.hand_occ[h] = k.o0; d.hand_occ[d.hand_pitch + h] = k.o1; d.hand_occ[2 * d.hand_pitch + h] = k.o2;
       d.hand_dec[h] = bps10; d.hand_wps[h] = wps10;
     }
-  } else if (HAND) {
+  } else if constexpr (HAND) {
     k.o0 = d.hand_occ[h]; k.o1 = d.hand_occ[d.hand_pitch + h]; k.o2 = d.hand_occ[2 * d.hand_pitch + h];
     bps10 = d.hand_dec[h]; wps10 = d.hand_wps[h];
-  } else bps10 = wps10 = 0ull;
+  } else {
+    k = kernel_occ(d.props, dev, have_dev, sm_count, grid_prod, block_prod, regs, ssm, dsm);
+    bps10 = wps10 = 0ull;
+  }
   const bool packed = bps10 != 0ull && wps10 != 0ull;
   s32(a, KS_PCT, k.o0.x); s32(a, KS_ACTIVE, k.o0.y); s32(a, KS_LIMIT, k.o0.z); s32(a, KS_LREGS, k.o0.w);
   s32(a, KS_LSMEM, k.o1.x); s32(a, KS_LWARPS, k.o1.y); s32(a, KS_LBLOCKS, k.o1.z); s32(a, KS_LBARR, k.o1.w);
