@@ -426,7 +426,7 @@ k2j_status k2j_create(int device, void* stream, k2j_ctx** out) {
   for (auto& e : c->ev) ok = ok && cudaEventCreate(&e) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&c->default_ev, cudaEventDisableTiming) == cudaSuccess;
   // the emit kernels' shared memory (record areas + output windows) is above the 48 KiB that needs no opt-in
-  for (auto* kernel : {k_events<true, false>, k_events<true, true>, k_events_slab<false>, k_events_slab<true>})
+  for (auto* kernel : {k_events<true, false>, k_events<true, true>, k_events<true, false, false>, k_events<true, true, false>})
     ok = ok && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)emit_smem_bytes(kEmitThreads)) == cudaSuccess;
   if (!ok) { k2j_destroy(c); cudaGetLastError(); return K2J_ERR_CUDA; }
   c->h_spans = reinterpret_cast<SpanRec*>(c->h_totals + 32);
@@ -1026,8 +1026,8 @@ int emit_threads(uint64_t items, uint32_t sms) {
 // The emit launches for the events whose text starts in [d.tile_begin, d.tile_end).  `ranges`: per class the work
 // items to look at ([begin, end) pairs, C_API .. C_WAIT, then the CPU-side activities); nullptr: everything.
 k2j_status launch_emit(k2j_ctx* c, const Dev& d, const uint64_t* ranges, bool instant, uint64_t n_coll, cudaStream_t s) {
-  auto* const main = d.hand_occ != nullptr ? k_events<true, false> : k_events_slab<false>;
-  auto* const rare = d.hand_occ != nullptr ? k_events<true, true> : k_events_slab<true>;
+  auto* const main = d.hand_occ != nullptr ? k_events<true, false> : k_events<true, false, false>;
+  auto* const rare = d.hand_occ != nullptr ? k_events<true, true> : k_events<true, true, false>;
   auto launch = [&](uint64_t begin, uint64_t end) {
     if (end <= begin) return;
     Dev dr = d;

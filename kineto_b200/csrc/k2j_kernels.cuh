@@ -185,7 +185,7 @@ struct Dev {
   // What the size pass has worked out for the emit pass, per work item of the kernel, copy and memset classes (index 0 =
   // the first kernel): doubles as pack_double's words (kernels: blocks per SM; copies and memsets: the bandwidth), and for
   // kernels warps per SM and the occupancy calculator's results (hand_occ: 3 rows of hand_pitch).  nullptr: worked out again
-  // by k_events_slab (text that leaves slab by slab: no call of that kind is to hold 64 bytes more for every kernel event).
+  // by k_events without HAND (text that leaves slab by slab: no call of that kind is to hold 64 bytes more for every kernel event).
   uint64_t* hand_dec; uint64_t* hand_wps; uint4* hand_occ; uint64_t hand_pitch;
   uint8_t* out; uint64_t out_cap;  // address of output byte 0 (of the whole text), bytes of the whole text
   // Sharded traces: records in front of guest_front (a slot index) and from guest_back on are other shards' records
@@ -235,8 +235,8 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
 // libkineto/src/CuptiActivityProfiler.cpp:293-296, GenericActivityProfiler.cpp:262).
 // A new key is swapped in at once: a load in front would be a second trip to the table (join of 500 k launches 68 us with
 // it, 63 without).  Where the key recurs in the warp (recurs) it is likely to be there, and many swaps on one slot cost
-// more than loads: with 450 k memory events, whose ids are all 0, 87 us with the load, 108 without; 500 k records of one
-// correlation id 48 (the last lane of each warp only, with the load), 390 (every lane, with it), 1020 (every lane, without).
+// more than loads: with 450 k memory events, whose ids are all 0, 86 us with the load, 108 without; 500 k records of one
+// correlation id 48 (the last lane of each warp only, with the load), 400 (every lane, with it), 1020 (every lane, without).
 __device__ __forceinline__ bool tab_insert(unsigned long long* tab, uint32_t mask, uint32_t key, uint32_t value, bool recurs) {
   const unsigned long long entry = ((unsigned long long)key << 32) | (unsigned long long)(value + 1u);
   uint32_t i = hash32(key) & mask;
@@ -2623,7 +2623,11 @@ __device__ __forceinline__ uint32_t class_units(int cls) {
 // the bytes at ev_off[event].  Either pass first copies the 32 records of a warp into shared memory
 // with coalesced loads (lane = 8-byte unit of a record); all later reads of record fields and of the
 // values computed from them are shared-memory reads at table-given offsets.
-template <bool WRITE, bool COLL, bool HAND> __device__ __forceinline__ void events(const Dev& d) {
+// HAND = false: the emit pass without values handed over by the size pass (the choice at run time, with the calculator out of
+// line, cost the emit pass of 100 k launches 1 us of 162).  The body stands in the kernel: as a function that two kernels share
+// it cost the size pass four more spilled words (1 M launches 256 -> 260 us).
+template <bool WRITE, bool COLL = false, bool HAND = true>
+__global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? kEmitBlocks : 8) k_events(Dev d) {
   const uint32_t threads = WRITE ? blockDim.x : (uint32_t)kEventThreads;
   uint64_t* const s_rec = reinterpret_cast<uint64_t*>(s_dyn + (WRITE ? sizeof(Digits3) / 16 : 0));
   uint32_t* const s_win = reinterpret_cast<uint32_t*>(s_rec + threads * kRecStride);
@@ -2740,11 +2744,6 @@ template <bool WRITE, bool COLL, bool HAND> __device__ __forceinline__ void even
     }
   }
 }
-template <bool WRITE, bool COLL = false>
-__global__ void __launch_bounds__(WRITE ? kEmitThreads : kEventThreads, WRITE ? kEmitBlocks : 8) k_events(Dev d) { events<WRITE, COLL, true>(d); }
-// The emit pass without a hand-over from the size pass.  A kernel of its own: the choice inside k_events, with the calculator
-// out of line, cost the emit pass of 100 k launches 1 us of 162.
-template <bool COLL> __global__ void __launch_bounds__(kEmitThreads, kEmitBlocks) k_events_slab(Dev d) { events<true, COLL, false>(d); }
 
 // ---- tiled runs: which events and which work items belong to each slab of the output ----
 // Slab t holds the events whose text starts in [t * slab, (t + 1) * slab).  bounds is a (n_tiles + 1) x
